@@ -134,7 +134,7 @@ sk_status sk_batch_create(sk_ctx *ctx, const sk_job *jobs, int32_t n_jobs, int32
       st = make_plan(ctx, jp, *c, plan);
       if (st != SK_OK) continue;
       LaunchBuffers buf;
-      st = upload_plan(ctx, jp, plan, buf, false);
+      st = upload_plan(ctx, plan, buf, false);
       if (st != SK_OK) return st;
       float ms = 0.0f;
       st = time_plan(ctx, plan, buf, 2, &ms);
@@ -159,7 +159,7 @@ sk_status sk_batch_create(sk_ctx *ctx, const sk_job *jobs, int32_t n_jobs, int32
   b->ctx = ctx;
   st = build_jobs(ctx, jobs, n_jobs, *cfg, b->jobs, &b->pairs);
   if (st == SK_OK) st = make_plan(ctx, b->jobs, *cfg, b->plan);
-  if (st == SK_OK) st = upload_plan(ctx, b->jobs, b->plan, b->buf, true);
+  if (st == SK_OK) st = upload_plan(ctx, b->plan, b->buf, true);
   if (st == SK_OK) {
     cudaError_t e = cudaStreamSynchronize(ctx->stream);
     if (e == cudaSuccess)
@@ -212,7 +212,7 @@ sk_status sk_batch_info(const sk_batch *b, int32_t *tile_config_id, int32_t *gri
                         int64_t *n_items, int64_t *n_pairs_out) {
   if (!b) return SK_EINVAL;
   if (tile_config_id) *tile_config_id = b->plan.cfg->id;
-  if (grid) *grid = b->plan.grid;
+  if (grid) *grid = static_cast<int32_t>(std::min<int64_t>(b->plan.grid, b->plan.items.size()));
   if (n_items) *n_items = static_cast<int64_t>(b->plan.items.size());
   if (n_pairs_out) *n_pairs_out = b->pairs;
   return SK_OK;
@@ -257,7 +257,7 @@ sk_status sk_autotune(sk_ctx *ctx, const sk_db *ref, const sk_db *query, const s
     Plan plan;
     if (make_plan(ctx, jp, *c, plan) != SK_OK) continue;
     LaunchBuffers buf;
-    st = upload_plan(ctx, jp, plan, buf, false);
+    st = upload_plan(ctx, plan, buf, false);
     if (st != SK_OK) return st;
     float ms = 0.0f;
     st = time_plan(ctx, plan, buf, std::max(1, repeats), &ms);

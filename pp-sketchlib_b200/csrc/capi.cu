@@ -206,6 +206,16 @@ void plan_tiles(JobParams &jp, const TileConfig &cfg) {
   }
 }
 
+// Pairs a job's tiles compute, padding included (n_query 0: all-vs-all).
+double padded_pairs(const TileConfig &cfg, int64_t n_ref, int64_t n_query) {
+  JobParams jp;
+  jp.self = n_query == 0;
+  jp.n_rows = n_query == 0 ? n_ref : n_query;
+  jp.n_cols = n_ref;
+  plan_tiles(jp, cfg);
+  return static_cast<double>(jp.n_tiles) * cfg.tile_rows * cfg.tile_cols;
+}
+
 // The reference GPU path's equal-base chances: csrs(k, use_rc, l0, l0) with l0
 // the first sample's length, narrowed to float (flattened_random,
 // src/random/random_match.cpp:278-310; csrs :318-336).
@@ -272,14 +282,18 @@ sk_status build_job(sk_ctx *ctx, const sk_db *ref, const sk_db *query, const sk_
   if (random && random->kmers != ref->kmers)
     return fail(ctx, SK_EMISMATCH, "Random match table k-mer lengths differ from the sketches");
   const TileConfig *cfg = choose_config(ctx, ref->K, ref->s64);
-  // A query batch of at most 64 samples fills one 64-row tile: with the
-  // default 128-row tile more than half of every tile's work would be padding
-  // (serving slices of a few queries), so use the 64 x 64 shape unless a shape
-  // was forced or tuned for this (K, sketchsize64).
-  if (query && query->n <= 64 && cfg && cfg->tile_rows > 64 && ctx->tile_cfg == 0 &&
+  // The 64 x 64 shape where 128 x 128 tiles would spend more on padding (rows
+  // and columns past the samples, the lower half of diagonal tiles) than the
+  // 5% it is slower by per pair, unless a shape was forced or tuned for this
+  // (K, sketchsize64): 64 samples fill a quarter of a 128 x 128 tile, 150
+  // queries 150 of 256 rows.
+  if (cfg && cfg->id == 1 && ctx->tile_cfg == 0 &&
       ctx->tuning.find({ref->K, ref->s64}) == ctx->tuning.end()) {
-    const TileConfig *small = tile_config(kSmallQueryConfig);
-    if (small && small->tile_rows == 64 && small->max_kmers >= ref->K) cfg = small;
+    const TileConfig *small = tile_config(kSmallTileConfig);
+    if (small && small->max_kmers >= ref->K &&
+        1.05 * padded_pairs(*small, ref->n, query ? query->n : 0) <
+            padded_pairs(*cfg, ref->n, query ? query->n : 0))
+      cfg = small;
   }
   if (!cfg || cfg->max_kmers < ref->K)
     return fail(ctx, SK_ENOTSUP, "No tile configuration holds %d k-mer lengths (at most %d)",
@@ -358,134 +372,138 @@ sk_status build_job(sk_ctx *ctx, const sk_db *ref, const sk_db *query, const sk_
   return SK_OK;
 }
 
-// Work list for one launch.  Jobs are visited in decreasing cost per tile
-// (K x blocks, longest first) so the dynamic queue ends on the cheapest items.
-// The tiles of the last, partial wave are cut into p parts along k (p chosen to
-// minimise ceil(r p / W) * ceil(K / p), r tail tiles on W resident CTAs); the
-// per-k counts are independent, so the parts need no reduction, only a shared
-// count slot and an arrival counter.  When every part holds one k, narrow
-// jobs' parts are cut further into block ranges (about 32 parts per tile), so
-// the launch ends within a small fraction of a tile on every SM; the partial
-// counts of one k's ranges are summed by the tile's finishing thread.
-void plan_items(const std::vector<JobParams> &jobs, int grid, Plan &plan) {
-  plan.items.clear();
-  plan.n_splits = 0;
-  plan.k_slots = 1;
-  std::vector<int> order(jobs.size());
-  for (size_t j = 0; j < jobs.size(); ++j) order[j] = static_cast<int>(j);
-  std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
-    return static_cast<int64_t>(jobs[a].n_kmers) * jobs[a].nb >
-           static_cast<int64_t>(jobs[b].n_kmers) * jobs[b].nb;
-  });
-  for (int j : order) {
-    plan.k_slots = std::max(plan.k_slots, job_slots(jobs[j]));
-    for (int64_t t = 0; t < jobs[j].n_tiles; ++t)
-      plan.items.push_back(WorkItem{t, j, 0, static_cast<int16_t>(jobs[j].n_kmers), -1, 1});
+// Block ranges each k of a narrow job's tail tile is cut into when r tail
+// tiles share `grid` resident CTAs: about 32 parts per tile with the k parts,
+// of at least 16 32-bin blocks each, so the dynamic queue ends the launch
+// within a small fraction of a tile on every SM; and, for a tail of few tiles,
+// two parts per CTA, of at least four blocks (two pipeline steps), so that a
+// job of one tile fills the device (64 samples: 405 us in 32 parts, 17 us in
+// 624, K = 8 and 312 blocks).
+int32_t tail_block_parts(const JobParams &jp, int64_t r, int grid) {
+  auto per_k = [&](int64_t parts) { return (parts + jp.n_kmers - 1) / jp.n_kmers; };
+  const int64_t even = std::min<int64_t>(per_k(32), jp.nb / 16);
+  const int64_t fill = std::min<int64_t>(per_k((2 * static_cast<int64_t>(grid) + r - 1) / r), jp.nb / 4);
+  return static_cast<int32_t>(std::max<int64_t>({1, even, fill}));
+}
+
+// Largest split scratch (count slots over all split tiles) and work list a
+// tail of up to grid - 1 tiles of this job can need.
+void tail_bounds(const JobParams &jp, int grid, int64_t *slots, int64_t *items) {
+  *slots = *items = 0;
+  for (int64_t r = 1; r < grid; ++r) {
+    const int64_t per = needs_wide(jp) ? job_slots(jp)
+                                       : static_cast<int64_t>(jp.n_kmers) * tail_block_parts(jp, r, grid);
+    *slots = std::max(*slots, r * per);
+    *items = std::max(*items, r * per);
   }
-  split_tail(plan.items, 0, grid, &plan.n_splits, &jobs);
-  plan.k_slots = items_slots(plan.items, plan.k_slots);
 }
 
-// Block ranges each k of a narrow job's tail tile is cut into: about 32 parts
-// per tile with the k parts, each range a whole number of 2-block steps.
-int32_t tail_block_parts(const JobParams &jp) {
-  if (needs_wide(jp)) return 1;
-  return std::max(1, std::min(32 / jp.n_kmers, jp.nb / 2));
-}
-
-// Count slots the items of a work list need: base (the jobs' K x nchunk), or
-// K x block ranges for tail tiles cut into block ranges.
-int32_t items_slots(const std::vector<WorkItem> &items, int32_t base) {
-  for (const WorkItem &it : items)
-    if (it.nbpart > 1) base = std::max<int32_t>(base, it.k1 * it.nbpart);
-  return base;
-}
-
-// Splits the last partial wave of items[begin..end) (whole tiles, k range
-// [0, K)) along k; split slots are numbered from 0 for this range.
-void split_tail(std::vector<WorkItem> &items, size_t begin, int grid, int32_t *n_splits,
-                const std::vector<JobParams> *jobs) {
-  *n_splits = 0;
+// Cuts the tiles of the last, partial wave of items[begin..end) (whole tiles)
+// into parts.  Narrow launches: every k and, within it, block ranges
+// (tail_block_parts); each range has its own count slot, summed by the split
+// kernel.  Wide launches: along k only, into the number of parts p that
+// minimises ceil(r p / W) * ceil(K / p), r tiles on W resident CTAs.
+void Plan::split_tail(size_t begin, Sub &sub) {
   const int64_t T = static_cast<int64_t>(items.size() - begin);
-  if (T == 0 || grid <= 0) return;
-  const int64_t r = T % grid == 0 ? 0 : T % grid;
+  const int64_t r = T % grid;
   if (r == 0) return;
-  // tail tiles: the last r items; k is split by the smallest K among them
-  int kmin = kMaxKmers;
-  for (size_t i = items.size() - r; i < items.size(); ++i) kmin = std::min<int>(kmin, items[i].k1);
-  int best_p = 1;
-  int64_t best = -1;
-  for (int p = 1; p <= kmin; ++p) {
-    const int64_t rounds = (r * p + grid - 1) / grid;
-    const int64_t cost = rounds * ((kmin + p - 1) / p);
-    if (best < 0 || cost < best) {
-      best = cost;
-      best_p = p;
+  int best_p = kMaxKmers;
+  if (wide) {
+    int kmin = kMaxKmers;
+    for (size_t i = items.size() - r; i < items.size(); ++i) kmin = std::min<int>(kmin, items[i].k1);
+    int64_t best = -1;
+    for (int p = 1; p <= kmin; ++p) {
+      const int64_t cost = ((r * p + grid - 1) / grid) * ((kmin + p - 1) / p);
+      if (best < 0 || cost < best) {
+        best = cost;
+        best_p = p;
+      }
     }
+    if (best_p == 1) return;
   }
-  if (best_p == 1) return;
-  std::vector<WorkItem> tail(items.end() - r, items.end());
+  const std::vector<WorkItem> tail(items.end() - r, items.end());
   items.resize(items.size() - r);
-  int32_t slot = 0;
   for (const WorkItem &it : tail) {
+    const JobParams &jp = jobs[it.job];
     const int K = it.k1;
     const int parts = std::min(best_p, K);
-    // narrow jobs cut each k further into block ranges when the tile is
-    // already cut into single k: about 32 parts per tile
-    int q = 1, nb = 0;
-    if (jobs && parts == K) {
-      const JobParams &jp = (*jobs)[it.job];
-      q = tail_block_parts(jp);
-      nb = jp.nb;
-    }
+    const int q = wide ? 1 : tail_block_parts(jp, r, grid);
+    const int steps = jp.nb / 2;
     for (int p = 0; p < parts; ++p) {
       const int k0 = K * p / parts, k1 = K * (p + 1) / parts;
       for (int b = 0; b < q; ++b) {
-        WorkItem w{it.tile, it.job, static_cast<int16_t>(k0), static_cast<int16_t>(k1), slot,
-                   parts * q};
+        WorkItem w{it.tile, it.job, static_cast<int16_t>(k0), static_cast<int16_t>(k1),
+                   sub.n_splits};
         if (q > 1) {
-          const int steps = nb / 2;
-          w.b0 = 2 * (steps * b / q);
-          w.b1 = 2 * (steps * (b + 1) / q);
+          w.b0 = static_cast<int32_t>(2 * (static_cast<int64_t>(steps) * b / q));
+          w.b1 = static_cast<int32_t>(2 * (static_cast<int64_t>(steps) * (b + 1) / q));
           w.bpart = static_cast<int16_t>(b);
           w.nbpart = static_cast<int16_t>(q);
         }
         items.push_back(w);
       }
     }
-    ++slot;
+    splits.push_back(SplitTile{it.tile, it.job, q});
+    sub.split_slots = std::max(sub.split_slots, wide ? job_slots(jp) : K * q);
+    ++sub.n_splits;
   }
-  *n_splits = slot;
 }
 
-// Device buffers for a plan: job table, work list, control block (queue
-// counter + split arrival counters, zeroed per launch) and count scratch.
-MetaLayout meta_layout(size_t n_jobs, size_t n_items, int32_t n_splits, int threads) {
+void Plan::add_tile(int job, int64_t tile) {
+  items.push_back(WorkItem{tile, job, 0, static_cast<int16_t>(jobs[job].n_kmers), -1});
+}
+
+// Ends the current launch: the tiles added since the last one.
+void Plan::close_launch() {
+  Sub sub;
+  sub.item0 = subs.empty() ? 0 : subs.back().item0 + subs.back().n_items;
+  sub.split0 = splits.size();
+  split_tail(sub.item0, sub);
+  sub.n_items = items.size() - sub.item0;
+  subs.push_back(sub);
+}
+
+sk_status Plan::start(sk_ctx *ctx, const std::vector<JobParams> &j, const TileConfig &c) {
+  cfg = &c;
+  jobs = j;
+  grid = resident_grid(ctx, c);
+  if (grid < 1) return fail(ctx, SK_ECUDA, "Tile configuration %d does not fit the device", c.id);
+  for (const JobParams &jp : jobs) {
+    k_slots = std::max(k_slots, job_slots(jp));
+    wide |= needs_wide(jp);
+  }
+  return SK_OK;
+}
+
+size_t Plan::split_bytes() const {
+  size_t b = 16;
+  for (const Sub &s : subs) b = std::max(b, s.n_splits * count_slot_bytes(*cfg, s.split_slots));
+  return b;
+}
+
+// Byte layout of a plan's meta buffer: job table, work list, split tiles and
+// the launches' queue counters (zeroed before every run), 256-aligned.
+MetaLayout meta_layout(size_t n_jobs, size_t n_items, size_t n_splits, size_t n_subs) {
+  auto up = [](size_t x) { return (x + 255) & ~static_cast<size_t>(255); };
   MetaLayout m;
-  m.items_off = (n_jobs * sizeof(JobParams) + 255) & ~static_cast<size_t>(255);
-  m.ctrl_off = (m.items_off + n_items * sizeof(WorkItem) + 255) & ~static_cast<size_t>(255);
-  m.ctrl_bytes = 8 + static_cast<size_t>(n_splits) * threads * 4;
+  m.items_off = up(n_jobs * sizeof(JobParams));
+  m.splits_off = up(m.items_off + n_items * sizeof(WorkItem));
+  m.ctrl_off = up(m.splits_off + n_splits * sizeof(SplitTile));
+  m.ctrl_bytes = n_subs * 8;
   m.bytes = m.ctrl_off + m.ctrl_bytes;
   return m;
 }
 
-sk_status upload_plan(sk_ctx *ctx, const std::vector<JobParams> &jobs, Plan &plan,
-                      LaunchBuffers &buf, bool owned) {
-  const TileConfig &cfg = *plan.cfg;
-  const size_t jobs_bytes = jobs.size() * sizeof(JobParams);
-  const size_t items_bytes = plan.items.size() * sizeof(WorkItem);
-  const MetaLayout ml = meta_layout(jobs.size(), plan.items.size(), plan.n_splits, cfg.threads);
-  const size_t ctrl_bytes = ml.ctrl_bytes;
-  const size_t jobs_off = 0;
-  const size_t items_off = ml.items_off;
-  const size_t ctrl_off = ml.ctrl_off;
-  const size_t meta_bytes = ml.bytes;
-  const size_t slot = count_slot_bytes(cfg, plan.k_slots);
-  const size_t cta_bytes = static_cast<size_t>(plan.grid) * slot;
-  const size_t split_bytes = std::max<size_t>(static_cast<size_t>(plan.n_splits) * slot, 16);
+// Device buffers for a plan: the meta buffer (uploaded here) and the count
+// scratch, from the context's scratch slots or (owned) allocated for the plan.
+sk_status upload_plan(sk_ctx *ctx, const Plan &plan, LaunchBuffers &buf, bool owned) {
+  const MetaLayout ml =
+      meta_layout(plan.jobs.size(), plan.items.size(), plan.splits.size(), plan.subs.size());
+  const size_t cta_bytes = static_cast<size_t>(plan.grid) * count_slot_bytes(*plan.cfg, plan.k_slots);
+  const size_t split_bytes = plan.split_bytes();
   void *meta = nullptr, *cta = nullptr, *split = nullptr;
   if (owned) {
-    cudaError_t e = cudaMalloc(&meta, meta_bytes);
+    cudaError_t e = cudaMalloc(&meta, ml.bytes);
     if (e == cudaSuccess) e = cudaMalloc(&cta, cta_bytes);
     if (e == cudaSuccess) e = cudaMalloc(&split, split_bytes);
     if (e != cudaSuccess) {
@@ -495,45 +513,70 @@ sk_status upload_plan(sk_ctx *ctx, const std::vector<JobParams> &jobs, Plan &pla
       return cuda_fail(ctx, e, "batch buffers");
     }
   } else {
-    sk_status st = scratch(ctx, kSlotLaunchMeta, meta_bytes, &meta);
+    sk_status st = scratch(ctx, kSlotLaunchMeta, ml.bytes, &meta);
     if (st == SK_OK) st = scratch(ctx, kSlotCounts, cta_bytes, &cta);
     if (st == SK_OK) st = scratch(ctx, kSlotSplitCounts, split_bytes, &split);
     if (st != SK_OK) return st;
   }
+  // one upload: the parts are laid out in a host image first
+  std::vector<char> image(ml.ctrl_off);
+  std::memcpy(image.data(), plan.jobs.data(), plan.jobs.size() * sizeof(JobParams));
+  if (!plan.items.empty())
+    std::memcpy(image.data() + ml.items_off, plan.items.data(), plan.items.size() * sizeof(WorkItem));
+  if (!plan.splits.empty())
+    std::memcpy(image.data() + ml.splits_off, plan.splits.data(),
+                plan.splits.size() * sizeof(SplitTile));
   char *m = static_cast<char *>(meta);
-  cudaError_t e = cudaMemcpyAsync(m + jobs_off, jobs.data(), jobs_bytes, cudaMemcpyHostToDevice,
-                                  ctx->stream);
-  if (e == cudaSuccess && items_bytes)
-    e = cudaMemcpyAsync(m + items_off, plan.items.data(), items_bytes, cudaMemcpyHostToDevice,
-                        ctx->stream);
-  if (e != cudaSuccess) return cuda_fail(ctx, e, "work list upload");
   buf.meta = meta;
   buf.cta = cta;
   buf.split = split;
-  buf.ctrl = m + ctrl_off;
-  buf.ctrl_bytes = ctrl_bytes;
+  cudaError_t e = cudaMemcpyAsync(m, image.data(), image.size(), cudaMemcpyHostToDevice, ctx->stream);
+  if (e != cudaSuccess) return cuda_fail(ctx, e, "work list upload");
+  buf.ctrl = m + ml.ctrl_off;
+  buf.ctrl_bytes = ml.ctrl_bytes;
   LaunchParams &lp = buf.lp;
-  lp.jobs = reinterpret_cast<const JobParams *>(m + jobs_off);
-  lp.items = reinterpret_cast<const WorkItem *>(m + items_off);
-  lp.n_items = static_cast<int64_t>(plan.items.size());
-  lp.item_counter = reinterpret_cast<unsigned long long *>(m + ctrl_off);
-  lp.split_done = reinterpret_cast<unsigned int *>(m + ctrl_off + 8);
+  lp = LaunchParams{};
+  lp.jobs = reinterpret_cast<const JobParams *>(m);
+  lp.items = reinterpret_cast<const WorkItem *>(m + ml.items_off);
+  lp.splits = reinterpret_cast<const SplitTile *>(m + ml.splits_off);
+  lp.item_counter = reinterpret_cast<unsigned long long *>(m + ml.ctrl_off);
   lp.cta_scratch = static_cast<uint16_t *>(cta);
   lp.split_scratch = static_cast<uint16_t *>(split);
   lp.k_slots = plan.k_slots;
-  lp.wide = 0;
-  for (const JobParams &jp : jobs) lp.wide |= needs_wide(jp) ? 1 : 0;
+  lp.wide = plan.wide ? 1 : 0;
   lp.status = ctx->status_dev;
   lp.cancel = ctx->cancel_dev;
   return SK_OK;
 }
 
-sk_status enqueue_plan(sk_ctx *ctx, const Plan &plan, const LaunchBuffers &buf) {
-  if (buf.lp.n_items == 0) return SK_OK;
+// Zeroes the queue counters of every launch of the plan.
+sk_status reset_plan(sk_ctx *ctx, const LaunchBuffers &buf) {
   cudaError_t e = cudaMemsetAsync(buf.ctrl, 0, buf.ctrl_bytes, ctx->stream);
-  if (e == cudaSuccess) e = plan.cfg->launch(buf.lp, plan.grid, ctx->stream);
-  if (e != cudaSuccess) return cuda_fail(ctx, e, "distance kernel launch");
-  return SK_OK;
+  return e == cudaSuccess ? SK_OK : cuda_fail(ctx, e, "work queue reset");
+}
+
+// Queues launch i of the plan on `stream`.
+sk_status enqueue_launch(sk_ctx *ctx, const Plan &plan, const LaunchBuffers &buf, size_t i,
+                         cudaStream_t stream) {
+  const Plan::Sub &sub = plan.subs[i];
+  if (sub.n_items == 0) return SK_OK;
+  LaunchParams lp = buf.lp;
+  lp.items += sub.item0;
+  lp.n_items = static_cast<int64_t>(sub.n_items);
+  lp.splits += sub.split0;
+  lp.n_splits = sub.n_splits;
+  lp.split_slots = sub.split_slots;
+  lp.item_counter += i;
+  const int g = static_cast<int>(std::min<int64_t>(plan.grid, lp.n_items));
+  cudaError_t e = plan.cfg->launch(lp, g, stream);
+  return e == cudaSuccess ? SK_OK : cuda_fail(ctx, e, "distance kernel launch");
+}
+
+sk_status enqueue_plan(sk_ctx *ctx, const Plan &plan, const LaunchBuffers &buf) {
+  sk_status st = reset_plan(ctx, buf);
+  for (size_t i = 0; st == SK_OK && i < plan.subs.size(); ++i)
+    st = enqueue_launch(ctx, plan, buf, i, ctx->stream);
+  return st;
 }
 
 int resident_grid(sk_ctx *ctx, const TileConfig &cfg) {
@@ -541,28 +584,31 @@ int resident_grid(sk_ctx *ctx, const TileConfig &cfg) {
   return per_sm < 1 ? 0 : per_sm * ctx->sm_count;
 }
 
+// One launch over every tile of the jobs, the jobs in decreasing cost per tile
+// (K x blocks, longest first) so the dynamic queue ends on the cheapest items.
 sk_status make_plan(sk_ctx *ctx, const std::vector<JobParams> &jobs, const TileConfig &cfg,
                     Plan &plan) {
-  plan.cfg = &cfg;
-  const int resident = resident_grid(ctx, cfg);
-  if (resident < 1) return fail(ctx, SK_ECUDA, "Tile configuration %d does not fit the device", cfg.id);
-  int64_t tiles = 0;
-  for (const JobParams &j : jobs) tiles += j.n_tiles;
-  plan.grid = resident;
-  plan_items(jobs, resident, plan);
-  if (static_cast<int64_t>(plan.items.size()) < plan.grid)
-    plan.grid = static_cast<int>(std::max<int64_t>(1, plan.items.size()));
+  sk_status st = plan.start(ctx, jobs, cfg);
+  if (st != SK_OK) return st;
+  std::vector<int> order(jobs.size());
+  for (size_t j = 0; j < jobs.size(); ++j) order[j] = static_cast<int>(j);
+  std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
+    return static_cast<int64_t>(jobs[a].n_kmers) * jobs[a].nb >
+           static_cast<int64_t>(jobs[b].n_kmers) * jobs[b].nb;
+  });
+  for (int j : order)
+    for (int64_t t = 0; t < jobs[j].n_tiles; ++t) plan.add_tile(j, t);
+  plan.close_launch();
   return SK_OK;
 }
 
 sk_status launch_job(sk_ctx *ctx, const JobParams &jp, const TileConfig &cfg) {
   if (jp.n_tiles == 0) return SK_OK;
-  std::vector<JobParams> jobs{jp};
   Plan plan;
-  sk_status st = make_plan(ctx, jobs, cfg, plan);
+  sk_status st = make_plan(ctx, {jp}, cfg, plan);
   if (st != SK_OK) return st;
   LaunchBuffers buf;
-  st = upload_plan(ctx, jobs, plan, buf, false);
+  st = upload_plan(ctx, plan, buf, false);
   if (st != SK_OK) return st;
   return enqueue_plan(ctx, plan, buf);
 }
@@ -633,8 +679,6 @@ sk_status dense_blocked_to_host(sk_ctx *ctx, const sk_db *ref, const sk_db *quer
   if (st != SK_OK) return st;
   st = ensure_copy_stream(ctx);
   if (st != SK_OK) return st;
-  const int grid = resident_grid(ctx, *cfg);
-  if (grid < 1) return fail(ctx, SK_ECUDA, "Tile configuration %d does not fit the device", cfg->id);
   const size_t elem = out_bytes(out_mode, 1, base.n_kmers);
   const int64_t nrt = base.n_row_tiles;
   const int64_t m = base.tile_rows / base.tile_cols;
@@ -661,53 +705,23 @@ sk_status dense_blocked_to_host(sk_ctx *ctx, const sk_db *ref, const sk_db *quer
   }
   const int nblk = static_cast<int>(cut.size() - 1);
   std::vector<JobParams> jobs(nblk, base);
-  std::vector<WorkItem> items;
-  std::vector<size_t> start(nblk), count(nblk);
-  std::vector<int32_t> splits(nblk);
-  for (int c = 0; c < nblk; ++c) {
-    jobs[c].out_row0 = first_row(cut[c]);
-    start[c] = items.size();
-    for (int64_t t = first_tile(cut[c]); t < first_tile(cut[c + 1]); ++t)
-      items.push_back(WorkItem{t, c, 0, static_cast<int16_t>(base.n_kmers), -1, 1});
-    split_tail(items, start[c], grid, &splits[c], &jobs);
-    count[c] = items.size() - start[c];
-  }
-  int32_t max_splits = *std::max_element(splits.begin(), splits.end());
-  const int32_t k_slots = items_slots(items, job_slots(base));
-  const size_t items_off = (jobs.size() * sizeof(JobParams) + 255) & ~static_cast<size_t>(255);
-  const size_t ctrl_off = (items_off + items.size() * sizeof(WorkItem) + 255) & ~static_cast<size_t>(255);
-  std::vector<size_t> ctrl_at(nblk);
-  size_t meta_bytes = ctrl_off;
-  for (int c = 0; c < nblk; ++c) {
-    ctrl_at[c] = meta_bytes;
-    meta_bytes += (8 + static_cast<size_t>(splits[c]) * cfg->threads * 4 + 255) & ~static_cast<size_t>(255);
-  }
-  const size_t slot = count_slot_bytes(*cfg, k_slots);
-  void *meta = nullptr, *cta = nullptr, *split = nullptr, *obuf = nullptr;
-  st = scratch(ctx, kSlotLaunchMeta, meta_bytes, &meta);
-  if (st == SK_OK) st = scratch(ctx, kSlotCounts, static_cast<size_t>(grid) * slot, &cta);
-  if (st == SK_OK)
-    st = scratch(ctx, kSlotSplitCounts, std::max<size_t>(static_cast<size_t>(max_splits) * slot, 16), &split);
-  if (st == SK_OK) st = scratch(ctx, kSlotOut, 2 * static_cast<size_t>(max_rows) * elem, &obuf);
+  for (int c = 0; c < nblk; ++c) jobs[c].out_row0 = first_row(cut[c]);
+  void *obuf = nullptr;
+  st = scratch(ctx, kSlotOut, 2 * static_cast<size_t>(max_rows) * elem, &obuf);
   if (st != SK_OK) return st;
   char *buf[2] = {static_cast<char *>(obuf), static_cast<char *>(obuf) + max_rows * elem};
   for (int c = 0; c < nblk; ++c) jobs[c].out = buf[c & 1];
-  char *mt = static_cast<char *>(meta);
-  cudaError_t e = cudaMemcpyAsync(mt, jobs.data(), jobs.size() * sizeof(JobParams),
-                                  cudaMemcpyHostToDevice, ctx->stream);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(mt + items_off, items.data(), items.size() * sizeof(WorkItem),
-                        cudaMemcpyHostToDevice, ctx->stream);
-  if (e == cudaSuccess) e = cudaMemsetAsync(mt + ctrl_off, 0, meta_bytes - ctrl_off, ctx->stream);
-  if (e != cudaSuccess) return cuda_fail(ctx, e, "work list upload");
-  LaunchParams lp{};
-  lp.jobs = reinterpret_cast<const JobParams *>(mt);
-  lp.cta_scratch = static_cast<uint16_t *>(cta);
-  lp.split_scratch = static_cast<uint16_t *>(split);
-  lp.k_slots = k_slots;
-  lp.wide = needs_wide(base) ? 1 : 0;
-  lp.status = ctx->status_dev;
-  lp.cancel = ctx->cancel_dev;
+  Plan plan;
+  LaunchBuffers lb;
+  st = plan.start(ctx, jobs, *cfg);
+  for (int c = 0; st == SK_OK && c < nblk; ++c) {
+    for (int64_t t = first_tile(cut[c]); t < first_tile(cut[c + 1]); ++t) plan.add_tile(c, t);
+    plan.close_launch();
+  }
+  if (st == SK_OK) st = upload_plan(ctx, plan, lb, false);
+  if (st == SK_OK) st = reset_plan(ctx, lb);
+  if (st != SK_OK) return st;
+  cudaError_t e = cudaSuccess;
   // block c computes into buf[c & 1] once the copy of block c - 2 has left it;
   // its copy is queued after block c + 1's launch, so a pageable destination
   // (whose copy returns only when done) still overlaps the next block
@@ -725,13 +739,9 @@ sk_status dense_blocked_to_host(sk_ctx *ctx, const sk_db *ref, const sk_db *quer
     if (c < nblk) {
       const int b = c & 1;
       if (c >= 2) e = cudaStreamWaitEvent(ctx->stream, ctx->ev_free[b], 0);
-      if (e == cudaSuccess && count[c] > 0) {
-        LaunchParams l = lp;
-        l.items = reinterpret_cast<const WorkItem *>(mt + items_off) + start[c];
-        l.n_items = static_cast<int64_t>(count[c]);
-        l.item_counter = reinterpret_cast<unsigned long long *>(mt + ctrl_at[c]);
-        l.split_done = reinterpret_cast<unsigned int *>(mt + ctrl_at[c] + 8);
-        e = cfg->launch(l, static_cast<int>(std::min<int64_t>(grid, l.n_items)), ctx->stream);
+      if (e == cudaSuccess) {
+        st = enqueue_launch(ctx, plan, lb, c, ctx->stream);
+        if (st != SK_OK) return st;
       }
       if (e == cudaSuccess) e = cudaEventRecord(ctx->ev_ready[b], ctx->stream);
     }

@@ -41,8 +41,6 @@ struct StepMeta {
   int32_t kidx;       // count slot of this step: k-mer index x nchunk + chunk
   int32_t flags;      // kStepEnd / kStepLastOfK (last step of a count slot) / kStepLastOfItem
   int32_t split;      // split slot of the item, -1 for whole tiles
-  int32_t nparts;
-  int32_t nbpart;     // block ranges per k of the item's tile (count slots per k)
 };
 constexpr int32_t kStepEnd = 1, kStepLastOfK = 2, kStepLastOfItem = 4;
 
@@ -130,8 +128,9 @@ __global__ void __launch_bounds__((QT / TQ) * (RT / TR), MINB)
   const int row0 = tq * TQ;   // first tile row of this thread
   const int col0 = tr * TR;   // first tile column of this thread
   const int64_t slot_k_stride = static_cast<int64_t>(NT) * PT;      // uint16 between k slots
-  const int64_t slot_size = slot_k_stride * lp.k_slots;
-  uint16_t *my_counts = lp.cta_scratch + blockIdx.x * slot_size + static_cast<int64_t>(tid) * PT;
+  const int64_t split_size = slot_k_stride * lp.split_slots;
+  uint16_t *my_counts = lp.cta_scratch + blockIdx.x * slot_k_stride * lp.k_slots +
+                        static_cast<int64_t>(tid) * PT;
 
   if (tid == 0) {
     for (int s = 0; s < STAGES; ++s) mbar_init(&full_bar[s], 1);
@@ -145,7 +144,7 @@ __global__ void __launch_bounds__((QT / TQ) * (RT / TR), MINB)
   // keeps its registers for the pair block.
   struct Producer {
     const uint32_t *rows, *cols;
-    int32_t done, have, job, ti, tj, k, k1, split, nparts, b0, nb, ngr, ngc;
+    int32_t done, have, job, ti, tj, k, k1, split, b0, nb, ngr, ngc;
     int32_t slot, slot_end, chunk_nb;   // count slot of the step, its last block + 1
     int32_t bstart, bend, bpart, nbpart;  // the item's block range of each k
   };
@@ -165,8 +164,7 @@ __global__ void __launch_bounds__((QT / TQ) * (RT / TR), MINB)
       return;
     }
     if (!ps.have) {
-      const bool cancelled = lp.cancel != nullptr && *lp.cancel != 0;
-      if (cancelled) atomicOr(&lp.status->error, 2u);
+      const bool cancelled = poll_cancelled(lp.status, lp.cancel);
       const unsigned long long idx = cancelled ? ~0ull : atomicAdd(lp.item_counter, 1ull);
       if (idx >= static_cast<unsigned long long>(lp.n_items)) {
         meta[s].flags = kStepEnd;
@@ -184,7 +182,6 @@ __global__ void __launch_bounds__((QT / TQ) * (RT / TR), MINB)
       ps.k = it.k0;
       ps.k1 = it.k1;
       ps.split = it.split;
-      ps.nparts = it.nparts;
       ps.nb = jp.nb;
       ps.bstart = it.b1 ? it.b0 : 0;
       ps.bend = it.b1 ? it.b1 : jp.nb;
@@ -213,10 +210,8 @@ __global__ void __launch_bounds__((QT / TQ) * (RT / TR), MINB)
     m.ti = ps.ti;
     m.tj = ps.tj;
     m.kidx = WIDE ? ps.slot : ps.k * ps.nbpart + ps.bpart;
-    m.nbpart = WIDE ? 1 : ps.nbpart;
     m.flags = (last_of_slot ? kStepLastOfK : 0) | (last_of_item ? kStepLastOfItem : 0);
     m.split = ps.split;
-    m.nparts = ps.nparts;
     mbar_arrive_expect_tx(&full_bar[s], S::kStageBytes);
 #pragma unroll
     for (int b = 0; b < kBlocksPerStage; ++b) {
@@ -342,7 +337,7 @@ __global__ void __launch_bounds__((QT / TQ) * (RT / TR), MINB)
     if (m.flags & kStepLastOfK) {
       // counts of count slot m.kidx done: park them (own slot or split slot)
       uint16_t *base = m.split >= 0
-                           ? lp.split_scratch + m.split * slot_size + static_cast<int64_t>(tid) * PT
+                           ? lp.split_scratch + m.split * split_size + static_cast<int64_t>(tid) * PT
                            : my_counts;
       // pair q = i * TR + j is uint16 q of the slot: word q / 2 = cnt[i][j / 2]
       uint4 *dst = reinterpret_cast<uint4 *>(base + m.kidx * slot_k_stride);
@@ -358,60 +353,78 @@ __global__ void __launch_bounds__((QT / TQ) * (RT / TR), MINB)
         for (int j = 0; j < TR / 2; ++j) cnt[i][j] = 0;
     }
 
-    if (m.flags & kStepLastOfItem) {
+    if ((m.flags & kStepLastOfItem) && m.split < 0) {
       const JobParams &jp = lp.jobs[m.job];
-      bool finish = true;
-      if (m.split >= 0) {
-        // Split tile: every thread owns its pairs' counts, so each thread
-        // counts its own arrivals; the thread of the last part to arrive
-        // gathers all k from the split slot and finishes those pairs.  No
-        // CTA-wide barrier, so a stage that timed out cannot strand a warp.
-        __threadfence();
-        const unsigned int prev =
-            atomicAdd(&lp.split_done[static_cast<int64_t>(m.split) * NT + tid], 1u);
-        finish = prev + 1 == static_cast<unsigned int>(m.nparts);
-        if (finish) {
-          __threadfence();
-          const uint4 *src = reinterpret_cast<const uint4 *>(
-              lp.split_scratch + m.split * slot_size + static_cast<int64_t>(tid) * PT);
-          if (WIDE || m.nbpart == 1) {
-            const int slots = WIDE ? job_slots(jp) : jp.n_kmers;
-            for (int k = 0; k < slots; ++k)
-#pragma unroll
-              for (int w = 0; w < PT / 8; ++w)
-                reinterpret_cast<uint4 *>(my_counts + k * slot_k_stride)[w] =
-                    __ldcg(src + k * (slot_k_stride / 8) + w);
-          } else {
-            // block ranges of one k: partial counts add up (two 16-bit
-            // counts per word never carry: their sums fit 16 bits)
-            for (int k = 0; k < jp.n_kmers; ++k)
-#pragma unroll
-              for (int w = 0; w < PT / 8; ++w) {
-                uint4 acc = __ldcg(src + (k * m.nbpart) * (slot_k_stride / 8) + w);
-                for (int p = 1; p < m.nbpart; ++p) {
-                  const uint4 v = __ldcg(src + (k * m.nbpart + p) * (slot_k_stride / 8) + w);
-                  acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
-                }
-                reinterpret_cast<uint4 *>(my_counts + k * slot_k_stride)[w] = acc;
-              }
-          }
-        }
-      }
-      if (finish) {
-        const int64_t gi0 = static_cast<int64_t>(m.ti) * QT + row0;
-        const int64_t gj0 = static_cast<int64_t>(m.tj) * RT + col0;
+      const int64_t gi0 = static_cast<int64_t>(m.ti) * QT + row0;
+      const int64_t gj0 = static_cast<int64_t>(m.tj) * RT + col0;
 #pragma unroll 1
-        for (int q = 0; q < PT; ++q) {
-          const int64_t gi = gi0 + q / TR;
-          const int64_t gj = gj0 + q % TR;
-          const bool valid =
-              jp.self ? (gj > gi && gj < jp.n_cols) : (gi < jp.n_rows && gj < jp.n_cols);
-          if (valid)
-            finish_pair_any<WIDE>(jp, gi, gj, my_counts + q, static_cast<int>(slot_k_stride));
-        }
+      for (int q = 0; q < PT; ++q) {
+        const int64_t gi = gi0 + q / TR;
+        const int64_t gj = gj0 + q % TR;
+        if (pair_valid(jp, gi, gj))
+          finish_pair_any<WIDE>(jp, gi, gj, my_counts + q, static_cast<int>(slot_k_stride));
       }
     }
   }
+}
+
+// The epilogue of the split tiles, one thread per pair over every SM.
+//
+// A split tile's counts lie in its slot by block range.  A CTA first adds up
+// the ranges of its 128 pairs: a thread owns 8 neighbouring pairs (one 128-bit
+// load per range; two 16-bit counts per word never carry, their sums fit 16
+// bits) at every eighth k, so a tile cut into hundreds of ranges keeps enough
+// loads in flight.  The sums go to shared memory, where finish_pair_any reads
+// them.  A pair's arithmetic is a chain of about 575 FP64 instructions: finished
+// inside the distance kernel by the last part's CTA, 32 pairs per thread one
+// after another, it held a single CTA for about 300 us at the end of a launch.
+// Wide jobs (one slot per chunk, no block ranges) are read where they lie.
+constexpr int kFinishPairs = 128;   // threads = pairs per CTA
+
+template <int QT, int RT, int TQ, int TR, bool WIDE>
+__global__ void __launch_bounds__(kFinishPairs) finish_splits_kernel(const LaunchParams lp) {
+  constexpr int PT = TQ * TR;
+  constexpr int TCOLS = RT / TR;
+  constexpr int kStride = QT * RT;   // uint16 between count slots
+  constexpr int kGroups = kStride / kFinishPairs;
+  __shared__ __align__(16) uint16_t sums[WIDE ? 8 : kNarrowKmers * kFinishPairs];
+  __shared__ int32_t s_ti, s_tj;
+  // an item that was cancelled or timed out parked nothing: its slot holds
+  // another launch's counts
+  if (*reinterpret_cast<const volatile unsigned int *>(&lp.status->error) != 0) return;
+  const int split = blockIdx.x / kGroups;
+  const int p0 = (blockIdx.x % kGroups) * kFinishPairs;   // first pair within the tile
+  const SplitTile st = lp.splits[split];
+  const JobParams &jp = lp.jobs[st.job];
+  if (threadIdx.x == 0) {
+    int32_t ti, tj;
+    tile_coords(jp, st.tile, ti, tj);
+    s_ti = ti;
+    s_tj = tj;
+  }
+  const uint16_t *src =
+      lp.split_scratch + static_cast<int64_t>(split) * lp.split_slots * kStride + p0;
+  if constexpr (!WIDE) {
+    const int g = threadIdx.x % (kFinishPairs / 8);
+    for (int k = threadIdx.x / (kFinishPairs / 8); k < jp.n_kmers; k += 8) {
+      const uint16_t *s = src + static_cast<int64_t>(k) * st.nbpart * kStride + 8 * g;
+      uint4 c = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll 8
+      for (int b = 0; b < st.nbpart; ++b) {
+        const uint4 v = *reinterpret_cast<const uint4 *>(s + static_cast<int64_t>(b) * kStride);
+        c.x += v.x; c.y += v.y; c.z += v.z; c.w += v.w;
+      }
+      *reinterpret_cast<uint4 *>(sums + k * kFinishPairs + 8 * g) = c;
+    }
+  }
+  __syncthreads();
+  const int p = p0 + threadIdx.x;
+  const int owner = p / PT, q = p % PT;
+  const int64_t gi = static_cast<int64_t>(s_ti) * QT + owner / TCOLS * TQ + q / TR;
+  const int64_t gj = static_cast<int64_t>(s_tj) * RT + owner % TCOLS * TR + q % TR;
+  if (!pair_valid(jp, gi, gj)) return;
+  if constexpr (WIDE) finish_pair_any<true>(jp, gi, gj, src + threadIdx.x, kStride);
+  else finish_pair_any<false>(jp, gi, gj, sums + threadIdx.x, kFinishPairs);
 }
 
 // ------------------------------------------------------------ config registry
@@ -437,11 +450,17 @@ cudaError_t launch_cfg(const LaunchParams &lp, int grid, cudaStream_t stream) {
     if (e != cudaSuccess) return e;
     dist_items_kernel<QT, RT, TQ, TR, STAGES, MINB, ROT, true>
         <<<grid, S::kThreads, S::kSmemBytes, stream>>>(lp);
+    if (lp.n_splits > 0)
+      finish_splits_kernel<QT, RT, TQ, TR, true>
+          <<<lp.n_splits * (QT * RT / kFinishPairs), kFinishPairs, 0, stream>>>(lp);
   } else {
     cudaError_t e = ensure_smem_attr<QT, RT, TQ, TR, STAGES, MINB, ROT, false>();
     if (e != cudaSuccess) return e;
     dist_items_kernel<QT, RT, TQ, TR, STAGES, MINB, ROT, false>
         <<<grid, S::kThreads, S::kSmemBytes, stream>>>(lp);
+    if (lp.n_splits > 0)
+      finish_splits_kernel<QT, RT, TQ, TR, false>
+          <<<lp.n_splits * (QT * RT / kFinishPairs), kFinishPairs, 0, stream>>>(lp);
   }
   return cudaGetLastError();
 }

@@ -89,7 +89,7 @@ extern "C" sk_status sk_dists_dense_noalloc(sk_ctx *ctx, const sk_db *ref, const
   if (grid > jp.n_tiles) grid = static_cast<int>(jp.n_tiles);
   std::vector<WorkItem> items(static_cast<size_t>(jp.n_tiles));
   for (int64_t t = 0; t < jp.n_tiles; ++t)
-    items[t] = WorkItem{t, 0, 0, static_cast<int16_t>(jp.n_kmers), -1, 1};
+    items[t] = WorkItem{t, 0, 0, static_cast<int16_t>(jp.n_kmers), -1};   // no tile is split
   const size_t off_job = 0;
   const size_t off_items = align256(off_job + sizeof(JobParams));
   const size_t off_ctrl = align256(off_items + items.size() * sizeof(WorkItem));
@@ -157,7 +157,6 @@ extern "C" sk_status sk_dists_dense_noalloc(sk_ctx *ctx, const sk_db *ref, const
   lp.items = reinterpret_cast<const WorkItem *>(base + off_items);
   lp.n_items = static_cast<int64_t>(items.size());
   lp.item_counter = reinterpret_cast<unsigned long long *>(base + off_ctrl);
-  lp.split_done = nullptr;       // no tile is split here
   lp.cta_scratch = reinterpret_cast<uint16_t *>(base + off_counts);
   lp.split_scratch = nullptr;
   lp.k_slots = job_slots(jp);

@@ -147,8 +147,6 @@ extern "C" sk_status sk_query_db_ready(sk_ctx *ctx, const sk_host_sketches *ref,
   st = build_job(ctx, dbs.ref, dbs.query, random, out_mode, 0, d_out, &cfg, &jp);
   if (st == SK_OK) st = attach_count_tables(ctx, &jp);
   if (st != SK_OK) return st;
-  const int grid = resident_grid(ctx, *cfg);
-  if (grid < 1) return fail(ctx, SK_ECUDA, "Tile configuration %d does not fit the device", cfg->id);
 
   // ---- work lists, one per reference chunk
   const int64_t n_ref = dbs.ref->n;
@@ -175,58 +173,33 @@ extern "C" sk_status sk_query_db_ready(sk_ctx *ctx, const sk_host_sketches *ref,
       }
     }
   }
-  std::vector<WorkItem> items;
-  const std::vector<JobParams> job_list{jp};
-  std::vector<size_t> start(n_chunks), count(n_chunks);
-  std::vector<int32_t> splits(n_chunks);
-  int32_t max_splits = 0;
+  Plan plan;
+  st = plan.start(ctx, {jp}, *cfg);
+  if (st != SK_OK) return st;
   for (int c = 0; c < n_chunks; ++c) {
-    start[c] = items.size();
-    for (int64_t t : bucket[c])
-      items.push_back(WorkItem{t, 0, 0, static_cast<int16_t>(jp.n_kmers), -1, 1});
-    split_tail(items, start[c], grid, &splits[c], &job_list);
-    count[c] = items.size() - start[c];
-    max_splits = std::max(max_splits, splits[c]);
+    for (int64_t t : bucket[c]) plan.add_tile(0, t);
+    plan.close_launch();
   }
 
-  // ---- device buffers: job, all items, one control block per chunk
-  const size_t items_off = (sizeof(JobParams) + 255) & ~static_cast<size_t>(255);
-  const size_t ctrl_off = (items_off + items.size() * sizeof(WorkItem) + 255) & ~static_cast<size_t>(255);
-  std::vector<size_t> ctrl_at(n_chunks);
-  size_t meta_bytes = ctrl_off;
-  for (int c = 0; c < n_chunks; ++c) {
-    ctrl_at[c] = meta_bytes;
-    meta_bytes += (8 + static_cast<size_t>(splits[c]) * cfg->threads * 4 + 255) & ~static_cast<size_t>(255);
-  }
-  const int32_t k_slots = items_slots(items, job_slots(jp));
-  const size_t slot = count_slot_bytes(*cfg, k_slots);
+  // ---- device buffers: the plan, count scratch for the second stream, staging
   const int64_t wps = static_cast<int64_t>(n_kmers) * sketchsize64 * bbits;   // words per sample
-  void *meta = nullptr, *staging = nullptr, *cta[2] = {}, *split[2] = {};
-  const size_t split_bytes = std::max<size_t>(static_cast<size_t>(max_splits) * slot, 16);
-  st = scratch(ctx, kSlotLaunchMeta, meta_bytes, &meta);
-  if (st == SK_OK) st = scratch(ctx, kSlotCounts, static_cast<size_t>(grid) * slot, &cta[0]);
-  if (st == SK_OK) st = scratch(ctx, kSlotCountsB, static_cast<size_t>(grid) * slot, &cta[1]);
-  if (st == SK_OK) st = scratch(ctx, kSlotSplitCounts, split_bytes, &split[0]);
-  if (st == SK_OK) st = scratch(ctx, kSlotSplitCountsB, split_bytes, &split[1]);
+  LaunchBuffers lb[2];
+  void *staging = nullptr, *cta_b = nullptr, *split_b = nullptr;
+  st = upload_plan(ctx, plan, lb[0], false);
+  if (st == SK_OK)
+    st = scratch(ctx, kSlotCountsB,
+                 static_cast<size_t>(plan.grid) * count_slot_bytes(*cfg, plan.k_slots), &cta_b);
+  if (st == SK_OK) st = scratch(ctx, kSlotSplitCountsB, plan.split_bytes(), &split_b);
   if (st == SK_OK) st = scratch(ctx, kSlotStaging, static_cast<size_t>(2 * cs * wps) * 8, &staging);
+  if (st == SK_OK) st = reset_plan(ctx, lb[0]);
   if (st != SK_OK) return st;
-  char *m = static_cast<char *>(meta);
-  cudaError_t e = cudaMemcpyAsync(m, &jp, sizeof(jp), cudaMemcpyHostToDevice, ctx->stream);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(m + items_off, items.data(), items.size() * sizeof(WorkItem),
-                        cudaMemcpyHostToDevice, ctx->stream);
-  if (e == cudaSuccess) e = cudaMemsetAsync(m + ctrl_off, 0, meta_bytes - ctrl_off, ctx->stream);
+  lb[1] = lb[0];
+  lb[1].lp.cta_scratch = static_cast<uint16_t *>(cta_b);
+  lb[1].lp.split_scratch = static_cast<uint16_t *>(split_b);
   // the second compute stream starts after the status reset and the work list
-  if (e == cudaSuccess) e = cudaEventRecord(ctx->ev_join, ctx->stream);
+  cudaError_t e = cudaEventRecord(ctx->ev_join, ctx->stream);
   if (e == cudaSuccess) e = cudaStreamWaitEvent(ctx->stream_b, ctx->ev_join, 0);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "work list upload");
-  LaunchParams base{};
-  base.jobs = reinterpret_cast<const JobParams *>(m);
-  base.k_slots = k_slots;
-  base.wide = needs_wide(jp) ? 1 : 0;
-  base.status = ctx->status_dev;
-  base.cancel = ctx->cancel_dev;
-  const WorkItem *d_items = reinterpret_cast<const WorkItem *>(m + items_off);
 
   // ---- upload units: the query side whole (in chunk-sized pieces), then the
   // reference chunk by chunk
@@ -283,19 +256,12 @@ extern "C" sk_status sk_query_db_ready(sk_ctx *ctx, const sk_host_sketches *ref,
     if (e == cudaSuccess) e = cudaEventRecord(ctx->ev_free[b], ctx->pack_stream);
     if (e == cudaSuccess) e = cudaEventRecord(ctx->ev_chunk[i], ctx->pack_stream);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "sketch upload");
-    if (!blocked && u.chunk >= 0 && count[u.chunk] > 0) {
+    if (!blocked && u.chunk >= 0 && plan.subs[u.chunk].n_items > 0) {
       const int w = launches++ & 1;
-      LaunchParams lp = base;
-      lp.cta_scratch = static_cast<uint16_t *>(cta[w]);
-      lp.split_scratch = static_cast<uint16_t *>(split[w]);
-      lp.items = d_items + start[u.chunk];
-      lp.n_items = static_cast<int64_t>(count[u.chunk]);
-      lp.item_counter = reinterpret_cast<unsigned long long *>(m + ctrl_at[u.chunk]);
-      lp.split_done = reinterpret_cast<unsigned int *>(m + ctrl_at[u.chunk] + 8);
-      const int g = static_cast<int>(std::min<int64_t>(grid, lp.n_items));
       e = cudaStreamWaitEvent(compute[w], ctx->ev_chunk[i], 0);   // packs complete in unit order
-      if (e == cudaSuccess) e = cfg->launch(lp, g, compute[w]);
       if (e != cudaSuccess) return cuda_fail(ctx, e, "distance kernel launch");
+      st = enqueue_launch(ctx, plan, lb[w], u.chunk, compute[w]);
+      if (st != SK_OK) return st;
       if (stream_out) {   // this chunk's rows are final: copy them back now
         const int64_t i0 = u.chunk * cs, i1 = std::min<int64_t>((u.chunk + 1) * cs, n_ref - 1);
         if (i1 > i0) {

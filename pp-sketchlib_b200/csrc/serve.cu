@@ -198,20 +198,19 @@ sk_status reserve_slice_scratch(sk_server *sv, Slot &s, int64_t *bytes) {
   if (st == SK_OK) st = attach_count_tables(ctx, &jp);
   if (st != SK_OK) return st;
   size_t meta = 0, cta = 16, split = 16;
-  for (const TileConfig *c : {choose_config(ctx, ref->K, ref->s64), tile_config(kSmallQueryConfig)}) {
+  for (const TileConfig *c : {choose_config(ctx, ref->K, ref->s64), tile_config(kSmallTileConfig)}) {
     if (!c || c->max_kmers < ref->K) continue;
     const int grid = resident_grid(ctx, *c);
     if (grid < 1) continue;
     const int64_t tiles = ((sq + c->tile_rows - 1) / c->tile_rows) *
                           ((ref->n + c->tile_cols - 1) / c->tile_cols);
-    // the tail tiles (fewer than the grid) may each be cut into K parts and
-    // each part into block ranges, every range its own count slot
-    const int32_t q = tail_block_parts(jp);
-    const int64_t items = tiles + static_cast<int64_t>(grid) * ref->K * q;
-    meta = std::max(meta, meta_layout(1, static_cast<size_t>(items), grid, c->threads).bytes);
-    const size_t slot = count_slot_bytes(*c, std::max(job_slots(jp), ref->K * q));
-    cta = std::max(cta, static_cast<size_t>(grid) * slot);
-    split = std::max(split, static_cast<size_t>(grid) * slot);
+    // the tail tiles (fewer than the grid) are cut into parts, every part
+    // with its own count slot
+    int64_t slots = 0, parts = 0;
+    tail_bounds(jp, grid, &slots, &parts);
+    meta = std::max(meta, meta_layout(1, static_cast<size_t>(tiles + parts), grid, 1).bytes);
+    cta = std::max(cta, static_cast<size_t>(grid) * count_slot_bytes(*c, job_slots(jp)));
+    split = std::max(split, static_cast<size_t>(slots) * count_slot_bytes(*c, 1));
   }
   void *p = nullptr;
   st = scratch(ctx, kSlotLaunchMeta, meta, &p);
@@ -360,9 +359,12 @@ int64_t take(Slot &s, const std::shared_ptr<Request> &r, int64_t room) {
   return nq;
 }
 
-// Rows of the query tile(s) a slice of nq queries occupies: the 64-row tile
-// of at most 64 queries, else 128-row tiles (build_job's choice).
-int64_t tile_rows_for(int64_t nq) { return nq <= 64 ? 64 : ((nq + 127) / 128) * 128; }
+// Rows of the query tiles a slice of nq queries occupies: 64-row tiles where
+// 128-row ones would be mostly padding (build_job's choice).
+int64_t tile_rows_for(int64_t nq) {
+  const int64_t r64 = (nq + 63) / 64 * 64, r128 = (nq + 127) / 128 * 128;
+  return 1.05 * static_cast<double>(r64) < static_cast<double>(r128) ? r64 : r128;
+}
 
 // Fills a free slot with the next slice, or leaves it empty when nothing may
 // start now.  `order` is the pending requests in admission order.

@@ -45,6 +45,7 @@ struct DevStatus {
   unsigned int error;      // bit 0: bounded wait timed out, bit 1: cancelled
   unsigned int where;      // last site that raised an error
   unsigned long long tiles_done;
+  unsigned long long next_poll;   // %globaltimer before which nobody reads the host's cancel word
 };
 
 // Everything one distance launch (one job) needs.  Rows are the "this"/query
@@ -105,18 +106,23 @@ __host__ __device__
 inline bool needs_wide(const JobParams &jp) { return jp.n_kmers > kNarrowKmers || jp.nchunk > 1; }
 
 // One unit of work of the persistent distance kernel: k-mer indices
-// [k0, k1) of one tile of one job.  A tile whose k range is cut into several
-// items (the last wave's tiles, to even out the tail) shares a split slot; the
-// item that finishes last runs the tile's epilogue.
+// [k0, k1) of one tile of one job.  A tile cut into several items (the last
+// wave's tiles, to even out the tail) shares a split slot: its items only park
+// their counts there, and the split kernel that follows finishes its pairs.
 struct WorkItem {
   int64_t tile;     // tile index within the job
   int32_t job;
   int16_t k0, k1;
   int32_t split;    // split slot, -1 for a whole tile
-  int32_t nparts;   // items sharing the split slot
   int32_t b0, b1;   // 32-bin blocks [b0, b1) of each k; b1 == 0: all of them
   int16_t bpart, nbpart;  // block range index, ranges per k (0: one)
-  int32_t pad;
+};
+
+// A tile cut into items: what the split kernel needs to finish it.
+struct SplitTile {
+  int64_t tile;
+  int32_t job;
+  int32_t nbpart;   // count slots per k (block ranges), 1 for wide jobs' chunks
 };
 
 // Everything one launch needs: the job table, the work list and the scratch.
@@ -125,10 +131,12 @@ struct LaunchParams {
   const WorkItem *items;
   int64_t n_items;
   unsigned long long *item_counter;   // zeroed before each launch
-  unsigned int *split_done;           // [n_splits][threads], zeroed before each launch
+  const SplitTile *splits;            // [n_splits]
+  int32_t n_splits;
   uint16_t *cta_scratch;              // [grid][k_slots][threads][pairs per thread]
-  uint16_t *split_scratch;            // [n_splits][k_slots][threads][pairs per thread]
+  uint16_t *split_scratch;            // [n_splits][split_slots][threads][pairs per thread]
   int32_t k_slots;                    // largest K x nchunk over the jobs
+  int32_t split_slots;                // largest count-slot need of a split tile
   int32_t wide;                       // 1: some job needs the wide kernel instance
   DevStatus *status;
   const volatile int *cancel;

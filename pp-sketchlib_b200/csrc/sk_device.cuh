@@ -73,6 +73,25 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity
   }
 }
 
+// Whether the call was cancelled, asked before every work item.  The host sets
+// a page-locked word; reading it crosses PCIe (about 1 us, one read at a time,
+// and in the way of uploads), so one thread per kPollNs reads it and everyone
+// else reads the error bit that thread sets in device memory.  With a read per
+// item, launches of many small items ran at the rate of those reads: 64
+// samples in 624 items took 938 us, and 3,001 samples from host memory in
+// 2,000 items slowed their own upload from 8 to 31 ms.
+constexpr unsigned long long kPollNs = 100000;
+__device__ __forceinline__ bool poll_cancelled(DevStatus *status, const volatile int *cancel) {
+  if (cancel == nullptr) return false;
+  const volatile DevStatus *st = status;
+  if (st->error & 2u) return true;
+  const unsigned long long due = st->next_poll, now = global_ns();
+  if (now < due || atomicCAS(&status->next_poll, due, now + kPollNs) != due) return false;
+  if (*cancel == 0) return false;
+  atomicOr(&status->error, 2u);
+  return true;
+}
+
 // acc & ~(a ^ b): one 3-input LOP3 per 32 bins per bit plane.
 __device__ __forceinline__ uint32_t lop_eq_and(uint32_t acc, uint32_t a, uint32_t b) {
   uint32_t d;
@@ -120,6 +139,12 @@ __device__ __forceinline__ void tile_coords(const JobParams &p, int64_t tile, in
 }
 
 // -------------------------------------------------------------- pair epilogue
+
+// Whether (gi, gj) is a pair of the job: padded rows and columns, and for
+// all-vs-all the lower triangle, are not.
+__device__ __forceinline__ bool pair_valid(const JobParams &p, int64_t gi, int64_t gj) {
+  return p.self ? (gj > gi && gj < p.n_cols) : (gi < p.n_rows && gj < p.n_cols);
+}
 
 // Intersection count of k-mer index k: its count slot, or (CHUNKED) the sum
 // of its chunks' slots when the sketch is wider than one uint16 counter holds

@@ -112,21 +112,36 @@ struct sk_sparse {
 
 namespace sk {
 
-// A launch of the persistent distance kernel: tile shape, grid and work list.
+// Launches of the persistent distance kernel that share a tile shape and one
+// meta buffer: the job table, and per launch its work list and split tiles.
 struct Plan {
+  struct Sub {
+    size_t item0 = 0, n_items = 0, split0 = 0;
+    int32_t n_splits = 0;
+    int32_t split_slots = 0;   // largest count-slot need of its split tiles
+  };
   const TileConfig *cfg = nullptr;
-  int grid = 0;
-  std::vector<WorkItem> items;
-  int32_t n_splits = 0;
+  int grid = 0;                // resident CTAs
+  bool wide = false;           // some job needs the wide kernel instance
   int32_t k_slots = 1;
+  std::vector<JobParams> jobs;
+  std::vector<WorkItem> items;
+  std::vector<SplitTile> splits;
+  std::vector<Sub> subs;
+
+  sk_status start(sk_ctx *ctx, const std::vector<JobParams> &j, const TileConfig &c);
+  void add_tile(int job, int64_t tile);
+  void close_launch();
+  size_t split_bytes() const;
+
+ private:
+  void split_tail(size_t begin, Sub &sub);
 };
 
-// Byte layout of a launch's meta buffer: job table at 0, then the work list
-// and the control block (queue counter, split arrival counters), 256-aligned.
 struct MetaLayout {
-  size_t items_off = 0, ctrl_off = 0, ctrl_bytes = 0, bytes = 0;
+  size_t items_off = 0, splits_off = 0, ctrl_off = 0, ctrl_bytes = 0, bytes = 0;
 };
-MetaLayout meta_layout(size_t n_jobs, size_t n_items, int32_t n_splits, int threads);
+MetaLayout meta_layout(size_t n_jobs, size_t n_items, size_t n_splits, size_t n_subs);
 
 struct LaunchBuffers {
   void *meta = nullptr, *cta = nullptr, *split = nullptr;
@@ -168,18 +183,18 @@ sk_status launch_job(sk_ctx *ctx, const JobParams &jp, const TileConfig &cfg);
 // a Monte Carlo table measured no faster (20.69 against 20.71 ms at 4,096
 // samples).
 sk_status attach_count_tables(sk_ctx *ctx, JobParams *jp, bool alloc = true);
-void plan_items(const std::vector<JobParams> &jobs, int grid, Plan &plan);
-void split_tail(std::vector<WorkItem> &items, size_t begin, int grid, int32_t *n_splits,
-                const std::vector<JobParams> *jobs = nullptr);
-int32_t items_slots(const std::vector<WorkItem> &items, int32_t base);
-int32_t tail_block_parts(const JobParams &jp);
+int32_t tail_block_parts(const JobParams &jp, int64_t r, int grid);
+void tail_bounds(const JobParams &jp, int grid, int64_t *slots, int64_t *items);
+double padded_pairs(const TileConfig &cfg, int64_t n_ref, int64_t n_query);
 sk_status db_alloc(sk_ctx *ctx, int64_t n, const int32_t *kmers, int32_t K, int32_t s64,
                    int32_t bbits, sk_db **out, int packed_slot = -1);
 void db_free(sk_db *db);
 sk_status make_plan(sk_ctx *ctx, const std::vector<JobParams> &jobs, const TileConfig &cfg,
                     Plan &plan);
-sk_status upload_plan(sk_ctx *ctx, const std::vector<JobParams> &jobs, Plan &plan,
-                      LaunchBuffers &buf, bool owned);
+sk_status upload_plan(sk_ctx *ctx, const Plan &plan, LaunchBuffers &buf, bool owned);
+sk_status reset_plan(sk_ctx *ctx, const LaunchBuffers &buf);
+sk_status enqueue_launch(sk_ctx *ctx, const Plan &plan, const LaunchBuffers &buf, size_t i,
+                         cudaStream_t stream);
 sk_status enqueue_plan(sk_ctx *ctx, const Plan &plan, const LaunchBuffers &buf);
 int resident_grid(sk_ctx *ctx, const TileConfig &cfg);
 sk_status dense_to_device(sk_ctx *ctx, const sk_db *ref, const sk_db *query,
