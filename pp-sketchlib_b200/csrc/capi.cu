@@ -17,6 +17,7 @@
 #include <fstream>
 #include <map>
 #include <mutex>
+#include <queue>
 #include <sstream>
 #include <string>
 #include <thread>
@@ -398,14 +399,48 @@ void tail_bounds(const JobParams &jp, int grid, int64_t *slots, int64_t *items) 
   }
 }
 
-// Cuts the tiles of the last, partial wave of items[begin..end) (whole tiles)
-// into parts.  Narrow launches: every k and, within it, block ranges
-// (tail_block_parts); each range has its own count slot, summed by the split
-// kernel.  Wide launches: along k only, into the number of parts p that
-// minimises ceil(r p / W) * ceil(K / p), r tiles on W resident CTAs.
-void Plan::split_tail(size_t begin, Sub &sub) {
+// Moves the tiles of items[begin..end) (whole tiles, costliest first) that are
+// to be cut to the end of the list and returns their number.  Whole tiles are
+// dealt to the least loaded of the resident CTAs while they end within the
+// mean load M = total / CTAs; the others are cut.  Tiles of one cost: the
+// last, partial wave.  Tiles of different costs (a batch): also those that
+// would outlast M, e.g. a few wide sketches among many narrow ones, which
+// alone held their CTAs for 10.6 of 13.0 ms in a batch of 12 databases.
+int64_t Plan::choose_splits(size_t begin) {
   const int64_t T = static_cast<int64_t>(items.size() - begin);
-  const int64_t r = T % grid;
+  if (T == 0) return 0;
+  auto cost = [&](const WorkItem &it) {
+    return static_cast<int64_t>(jobs[it.job].n_kmers) * jobs[it.job].nb;
+  };
+  int64_t total = 0;
+  for (size_t i = begin; i < items.size(); ++i) total += cost(items[i]);
+  if (total == T * cost(items[begin])) return T % grid;
+  std::priority_queue<int64_t, std::vector<int64_t>, std::greater<int64_t>> load(
+      std::greater<int64_t>(), std::vector<int64_t>(grid, 0));
+  std::vector<WorkItem> cut;
+  size_t keep = begin;
+  for (size_t i = begin; i < items.size(); ++i) {
+    const int64_t c = cost(items[i]);
+    if ((load.top() + c) * grid <= total) {
+      const int64_t l = load.top();
+      load.pop();
+      load.push(l + c);
+      items[keep++] = items[i];
+    } else {
+      cut.push_back(items[i]);
+    }
+  }
+  std::copy(cut.begin(), cut.end(), items.begin() + keep);
+  return static_cast<int64_t>(cut.size());
+}
+
+// Cuts the tiles choose_splits picks into parts.  Narrow launches: every k
+// and, within it, block ranges (tail_block_parts); each range has its own
+// count slot, summed by the split kernel.  Wide launches: along k only, into
+// the number of parts p that minimises ceil(r p / W) * ceil(K / p), r tiles on
+// W resident CTAs.
+void Plan::split_tail(size_t begin, Sub &sub) {
+  const int64_t r = choose_splits(begin);
   if (r == 0) return;
   int best_p = kMaxKmers;
   if (wide) {

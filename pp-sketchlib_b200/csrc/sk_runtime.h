@@ -135,6 +135,7 @@ struct Plan {
   size_t split_bytes() const;
 
  private:
+  int64_t choose_splits(size_t begin);
   void split_tail(size_t begin, Sub &sub);
 };
 
