@@ -33,6 +33,7 @@ void free_buffers(LaunchBuffers &b) {
   if (b.meta) cudaFree(b.meta);
   if (b.cta) cudaFree(b.cta);
   if (b.split) cudaFree(b.split);
+  if (b.codes) cudaFree(b.codes);
   b = LaunchBuffers{};
 }
 
@@ -78,6 +79,16 @@ sk_status build_jobs(sk_ctx *ctx, const sk_job *in, int n, const TileConfig &cfg
     *pairs += n_pairs(in[j].ref, in[j].query);
   }
   return SK_OK;
+}
+
+// Code bytes of a batch's launches beside its column values: at most 8 GiB,
+// and values and codes within a quarter of the free memory.
+size_t batch_code_budget(const std::vector<JobParams> &jobs, const TileConfig &cfg) {
+  size_t values = 0, codes = 0, free_b = 0, total_b = 0;
+  code_wants(jobs, cfg, &values, &codes);
+  if (codes == 0 || cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || free_b / 4 <= values)
+    return 0;
+  return std::min({codes, size_t(8) << 30, free_b / 4 - values});
 }
 
 // Times `repeats` launches of the plan (after one warm-up), in milliseconds.
@@ -131,7 +142,7 @@ sk_status sk_batch_create(sk_ctx *ctx, const sk_job *jobs, int32_t n_jobs, int32
       st = build_jobs(ctx, jobs, n_jobs, *c, jp, &pairs);
       if (st != SK_OK) return st;
       Plan plan;
-      st = make_plan(ctx, jp, *c, plan);
+      st = make_plan(ctx, jp, *c, code_budget_for(ctx, jp, *c), plan);
       if (st != SK_OK) continue;
       LaunchBuffers buf;
       st = upload_plan(ctx, plan, buf, false);
@@ -158,8 +169,19 @@ sk_status sk_batch_create(sk_ctx *ctx, const sk_job *jobs, int32_t n_jobs, int32
   sk_batch *b = new sk_batch();
   b->ctx = ctx;
   st = build_jobs(ctx, jobs, n_jobs, *cfg, b->jobs, &b->pairs);
-  if (st == SK_OK) st = make_plan(ctx, b->jobs, *cfg, b->plan);
-  if (st == SK_OK) st = upload_plan(ctx, b->plan, b->buf, true);
+  if (st == SK_OK) {
+    // the batch owns its code buffer, sized as the context's would be; where
+    // that cannot be had, its jobs run on their 14 planes
+    st = make_plan(ctx, b->jobs, *cfg, batch_code_budget(b->jobs, *cfg), b->plan);
+    if (st == SK_OK) st = upload_plan(ctx, b->plan, b->buf, true);
+    if (st == SK_ENOMEM) {
+      cudaGetLastError();
+      free_buffers(b->buf);
+      b->plan = Plan{};
+      st = make_plan(ctx, b->jobs, *cfg, 0, b->plan);
+      if (st == SK_OK) st = upload_plan(ctx, b->plan, b->buf, true);
+    }
+  }
   if (st == SK_OK) {
     cudaError_t e = cudaStreamSynchronize(ctx->stream);
     if (e == cudaSuccess)
@@ -255,7 +277,7 @@ sk_status sk_autotune(sk_ctx *ctx, const sk_db *ref, const sk_db *query, const s
     st = build_jobs(ctx, &job, 1, *c, jp, &p);
     if (st != SK_OK) return st;
     Plan plan;
-    if (make_plan(ctx, jp, *c, plan) != SK_OK) continue;
+    if (make_plan(ctx, jp, *c, code_budget_for(ctx, jp, *c), plan) != SK_OK) continue;
     LaunchBuffers buf;
     st = upload_plan(ctx, plan, buf, false);
     if (st != SK_OK) return st;

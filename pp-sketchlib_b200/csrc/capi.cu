@@ -12,6 +12,7 @@
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <limits>
 #include <fstream>
@@ -287,8 +288,10 @@ sk_status build_job(sk_ctx *ctx, const sk_db *ref, const sk_db *query, const sk_
   // and columns past the samples, the lower half of diagonal tiles) than the
   // 5% it is slower by per pair, unless a shape was forced or tuned for this
   // (K, sketchsize64): 64 samples fill a quarter of a 128 x 128 tile, 150
-  // queries 150 of 256 rows.
+  // queries 150 of 256 rows.  Jobs large enough to be coded stay on the shape
+  // that has a coded instance.
   if (cfg && cfg->id == 1 && ctx->tile_cfg == 0 &&
+      !use_codes(query ? query->n : ref->n, ref->n, ref->K, 2 * ref->s64, !query) &&
       ctx->tuning.find({ref->K, ref->s64}) == ctx->tuning.end()) {
     const TileConfig *small = tile_config(kSmallTileConfig);
     if (small && small->max_kmers >= ref->K &&
@@ -442,6 +445,7 @@ int64_t Plan::choose_splits(size_t begin) {
 void Plan::split_tail(size_t begin, Sub &sub) {
   const int64_t r = choose_splits(begin);
   if (r == 0) return;
+  const bool wide = sub.wide;
   int best_p = kMaxKmers;
   if (wide) {
     int kmin = kMaxKmers;
@@ -484,30 +488,211 @@ void Plan::split_tail(size_t begin, Sub &sub) {
   }
 }
 
+int Plan::add_job(const JobParams &jp) {
+  jobs.push_back(jp);
+  k_slots = std::max(k_slots, job_slots(jp));
+  return static_cast<int>(jobs.size()) - 1;
+}
+
 void Plan::add_tile(int job, int64_t tile) {
+  open_.wide |= needs_wide(jobs[job]);
   items.push_back(WorkItem{tile, job, 0, static_cast<int16_t>(jobs[job].n_kmers), -1});
+}
+
+namespace {
+
+size_t up256(size_t x) { return (x + 255) & ~static_cast<size_t>(255); }
+
+// Bytes of a column database's bin values.
+size_t value_bytes(int64_t KB, int64_t ng) {
+  return static_cast<size_t>(KB) * ng * kValueStripeWords * 4;
+}
+
+// Code bytes of one row block over `groups` column groups, KB blocks.
+size_t row_block_bytes(int64_t KB, int64_t groups) {
+  return static_cast<size_t>(KB) * ((1 + groups) * kCodeStripeWords * 4 + kCodeListWords * 2 + 1) + 768;
+}
+
+}  // namespace
+
+// One range of row blocks over column groups: its job (a copy of jp with the
+// range's layout), encoding task and tiles, in the open launch.
+void Plan::add_piece(const JobParams &jp, int32_t rb0, int32_t rb1, int32_t cg0, int32_t cg1,
+                     bool self, int code_buf) {
+  Code c{};
+  JobParams j = jp;
+  j.code = CodeLayout{self ? 1 : 0, rb0, cg0, cg1};
+  c.job = add_job(j);
+  CodeTask &t = c.task;
+  t.row_words = jp.row_words;
+  t.ng_rows = jp.ng_rows;
+  t.ng_cols = jp.ng_cols;
+  t.n_rows = jp.n_rows;
+  t.kb = jp.n_kmers * jp.nb;
+  t.n_rb = rb1 - rb0;
+  t.layout = j.code;
+  c.chunk0 = chunks.size();
+  for (int32_t rb = rb0; rb < rb1; ++rb) {
+    const int32_t g0 = code_first_group(j.code, rb), n = cg1 - g0;
+    // two row blocks at a time, over ranges of at most kCodeChunkGroups column
+    // groups (one per warp), of even size
+    const int32_t parts = (rb - rb0) % 2 ? 0 : (n + kCodeChunkGroups - 1) / kCodeChunkGroups;
+    for (int32_t p = 0; p < parts; ++p)
+      chunks.push_back(make_int4(rb - rb0, g0 + static_cast<int32_t>(int64_t(n) * p / parts),
+                                 g0 + static_cast<int32_t>(int64_t(n) * (p + 1) / parts), 0));
+    for (int32_t tj = g0; tj < cg1; ++tj)
+      add_tile(c.job, jp.self ? static_cast<int64_t>(rb) * jp.n_col_tiles -
+                                    static_cast<int64_t>(rb) * (rb - 1) / 2 + (tj - rb)
+                              : static_cast<int64_t>(rb) * jp.n_col_tiles + tj);
+  }
+  t.n_chunks = static_cast<int32_t>(chunks.size() - c.chunk0);
+  c.words_off = open_.code_bytes;
+  c.lists_off = up256(c.words_off +
+                      static_cast<size_t>(code_groups_before(j.code, rb1)) * t.kb * kCodeStripeWords * 4);
+  c.planes_off = up256(c.lists_off + static_cast<size_t>(t.n_rb) * t.kb * kCodeListWords * 2);
+  open_.code_bytes = up256(c.planes_off + static_cast<size_t>(t.n_rb) * t.kb);
+  open_.code_buf = code_buf;
+  // the columns' values: one task per packed array of the plan
+  size_t v = 0;
+  while (v < values.size() && values[v].packed != jp.col_words) ++v;
+  if (v == values.size()) {
+    values.push_back(Values{jp.col_words, t.kb, jp.ng_cols, value_bytes_});
+    value_bytes_ += up256(value_bytes(t.kb, jp.ng_cols));
+  }
+  c.values = v;
+  open_.codes.push_back(c);
+}
+
+void Plan::add_coded(const JobParams &jp, int32_t rt0, int32_t rt1, int32_t ct0, int32_t ct1,
+                     int code_buf) {
+  const int64_t KB = static_cast<int64_t>(jp.n_kmers) * jp.nb;
+  auto first = [&](int32_t rb) { return jp.self ? std::max(rb, ct0) : ct0; };
+  for (int32_t rb = rt0; rb < rt1;) {
+    // row blocks that fit the open launch
+    size_t bytes = open_.code_bytes;
+    int32_t end = rb;
+    // a range with its own first column per row block needs the columns to
+    // start at the diagonal
+    const bool diag = jp.self && first(rb) == rb;
+    while (end < rt1 && (!jp.self || diag || end == rb)) {
+      const size_t b = row_block_bytes(KB, ct1 - first(end));
+      if (bytes + b > code_budget) break;
+      bytes += b;
+      ++end;
+    }
+    if (end > rb) {
+      add_piece(jp, rb, end, first(rb), ct1, diag, code_buf);
+      rb = end;
+    } else if (!open_empty()) {
+      close_launch();
+    } else {   // one row block alone is over the budget: its columns in even parts
+      const int32_t c0 = first(rb), n = ct1 - c0;
+      int32_t parts = 2;
+      while (parts < n && row_block_bytes(KB, (n + parts - 1) / parts) > code_budget) ++parts;
+      for (int32_t p = 0; p < parts; ++p) {
+        add_piece(jp, rb, rb + 1, c0 + static_cast<int32_t>(int64_t(n) * p / parts),
+                  c0 + static_cast<int32_t>(int64_t(n) * (p + 1) / parts), false, code_buf);
+        close_launch();
+      }
+      ++rb;
+    }
+  }
 }
 
 // Ends the current launch: the tiles added since the last one.
 void Plan::close_launch() {
-  Sub sub;
-  sub.item0 = subs.empty() ? 0 : subs.back().item0 + subs.back().n_items;
-  sub.split0 = splits.size();
-  split_tail(sub.item0, sub);
-  sub.n_items = items.size() - sub.item0;
-  subs.push_back(sub);
+  open_.item0 = closed_items_;
+  open_.split0 = splits.size();
+  split_tail(open_.item0, open_);
+  open_.n_items = items.size() - open_.item0;
+  closed_items_ = items.size();
+  open_.values0 = closed_values_;
+  open_.n_values = values.size() - closed_values_;
+  closed_values_ = values.size();
+  subs.push_back(std::move(open_));
+  open_ = Sub{};
 }
 
-sk_status Plan::start(sk_ctx *ctx, const std::vector<JobParams> &j, const TileConfig &c) {
+sk_status Plan::start(sk_ctx *ctx, const TileConfig &c, size_t budget) {
   cfg = &c;
-  jobs = j;
+  code_budget = budget;
+  sm_count = ctx->sm_count;
   grid = resident_grid(ctx, c);
   if (grid < 1) return fail(ctx, SK_ECUDA, "Tile configuration %d does not fit the device", c.id);
-  for (const JobParams &jp : jobs) {
-    k_slots = std::max(k_slots, job_slots(jp));
-    wide |= needs_wide(jp);
+  if (code_budget > 0) {   // before any stream capture
+    const cudaError_t e = prepare_code_kernels();
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "encoder setup");
   }
   return SK_OK;
+}
+
+size_t Plan::code_stride() const {
+  size_t one = 0;
+  for (const Sub &s : subs) one = std::max(one, s.code_bytes);
+  return up256(one);
+}
+
+size_t Plan::code_bytes() const {
+  int bufs = 0;
+  for (const Sub &s : subs)
+    if (!s.codes.empty()) bufs = std::max(bufs, s.code_buf + 1);
+  return code_stride() * bufs + value_bytes_;
+}
+
+// Whether a job's tiles are worth encoding first (128 x 128 tiles of narrow
+// jobs).  The encoder costs about as much per row block and column as the
+// planes it saves in one tile, so it pays where a row block meets many columns
+// and, since it serves two row blocks per lookup, where there are two: an
+// all-vs-all at K = 8, 156 words on a random tree took 2.85 ms plain and 2.88
+// coded at 1,500 samples, 4.99 and 4.64 at 2,000, 11.5 and 9.5 at 3,000 (in
+// clades 2.86 and 2.72, 4.99 and 4.33, 11.0 and 9.1); 100 queries against
+// 20,000 samples 5.70 and 6.07, 300 queries 15.1 and 13.8, 300 against 2,000
+// 1.60 and 1.53.  Narrower sketches and fewer k cross at the same sizes.
+bool use_codes(int64_t n_rows, int64_t n_cols, int32_t n_kmers, int32_t nb, bool self) {
+  if (n_kmers > kNarrowKmers || nb > kMaxChunkBlocks) return false;
+  return self ? n_cols >= 1700 : n_rows > kCodeGroup && n_cols >= 1000;
+}
+
+// Bytes of a job's column values.
+size_t job_value_bytes(const JobParams &jp) {
+  return up256(value_bytes(static_cast<int64_t>(jp.n_kmers) * jp.nb, jp.ng_cols));
+}
+
+// Code bytes of a job in one launch.
+size_t code_bytes_wanted(const JobParams &jp) {
+  const int64_t KB = static_cast<int64_t>(jp.n_kmers) * jp.nb;
+  size_t b = 0;
+  for (int64_t rb = 0; rb < jp.n_row_tiles; ++rb)
+    b += row_block_bytes(KB, jp.n_col_tiles - (jp.self ? rb : 0));
+  return b;
+}
+
+// Grows the context's code buffer to `values` bytes and towards `codes` more
+// (at most 8 GiB), within a quarter of the memory that is free or held by the
+// buffer, or the limit a server set for its slots.  Returns the code bytes
+// granted, 0 for none: a job that cannot be encoded runs on its 14 planes.
+size_t code_reserve(sk_ctx *ctx, size_t values, size_t codes) {
+  if (ctx->code_limit < 0) return 0;
+  Scratch &s = ctx->scratch[kSlotCodes];
+  codes = std::min(codes, size_t(8) << 30);
+  if (s.bytes < values + codes) {
+    size_t cap = static_cast<size_t>(ctx->code_limit);
+    if (cap == 0) {
+      size_t free_b = 0, total_b = 0;
+      if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return 0;
+      cap = (free_b + s.bytes) / 4;
+    }
+    const size_t want = std::min(values + codes, std::max(cap, s.bytes));
+    if (want <= values) return 0;
+    void *p = nullptr;
+    if (scratch(ctx, kSlotCodes, want, &p) != SK_OK) {
+      cudaGetLastError();
+      ctx->err.clear();
+      return 0;
+    }
+    codes = want - values;
+  }
+  return codes;
 }
 
 size_t Plan::split_bytes() const {
@@ -516,55 +701,69 @@ size_t Plan::split_bytes() const {
   return b;
 }
 
-// Byte layout of a plan's meta buffer: job table, work list, split tiles and
-// the launches' queue counters (zeroed before every run), 256-aligned.
-MetaLayout meta_layout(size_t n_jobs, size_t n_items, size_t n_splits, size_t n_subs) {
-  auto up = [](size_t x) { return (x + 255) & ~static_cast<size_t>(255); };
+// Byte layout of a plan's meta buffer: job table, work list, split tiles,
+// column ranges to encode and the launches' queue counters (zeroed before
+// every run), 256-aligned.
+MetaLayout meta_layout(size_t n_jobs, size_t n_items, size_t n_splits, size_t n_chunks,
+                       size_t n_subs) {
   MetaLayout m;
-  m.items_off = up(n_jobs * sizeof(JobParams));
-  m.splits_off = up(m.items_off + n_items * sizeof(WorkItem));
-  m.ctrl_off = up(m.splits_off + n_splits * sizeof(SplitTile));
+  m.items_off = up256(n_jobs * sizeof(JobParams));
+  m.splits_off = up256(m.items_off + n_items * sizeof(WorkItem));
+  m.chunks_off = up256(m.splits_off + n_splits * sizeof(SplitTile));
+  m.ctrl_off = up256(m.chunks_off + n_chunks * sizeof(int4));
   m.ctrl_bytes = n_subs * 8;
   m.bytes = m.ctrl_off + m.ctrl_bytes;
   return m;
 }
 
 // Device buffers for a plan: the meta buffer (uploaded here) and the count
-// scratch, from the context's scratch slots or (owned) allocated for the plan.
-sk_status upload_plan(sk_ctx *ctx, const Plan &plan, LaunchBuffers &buf, bool owned) {
-  const MetaLayout ml =
-      meta_layout(plan.jobs.size(), plan.items.size(), plan.splits.size(), plan.subs.size());
-  const size_t cta_bytes = static_cast<size_t>(plan.grid) * count_slot_bytes(*plan.cfg, plan.k_slots);
-  const size_t split_bytes = plan.split_bytes();
-  void *meta = nullptr, *cta = nullptr, *split = nullptr;
-  if (owned) {
-    cudaError_t e = cudaMalloc(&meta, ml.bytes);
-    if (e == cudaSuccess) e = cudaMalloc(&cta, cta_bytes);
-    if (e == cudaSuccess) e = cudaMalloc(&split, split_bytes);
-    if (e != cudaSuccess) {
-      if (meta) cudaFree(meta);
-      if (cta) cudaFree(cta);
-      if (split) cudaFree(split);
-      return cuda_fail(ctx, e, "batch buffers");
+// and code scratch, from the context's scratch slots or (owned) allocated for
+// the plan.
+sk_status upload_plan(sk_ctx *ctx, Plan &plan, LaunchBuffers &buf, bool owned) {
+  const MetaLayout ml = meta_layout(plan.jobs.size(), plan.items.size(), plan.splits.size(),
+                                    plan.chunks.size(), plan.subs.size());
+  const size_t sizes[4] = {ml.bytes,
+                           static_cast<size_t>(plan.grid) * count_slot_bytes(*plan.cfg, plan.k_slots),
+                           plan.split_bytes(), plan.code_bytes()};
+  const int slots[4] = {kSlotLaunchMeta, kSlotCounts, kSlotSplitCounts, kSlotCodes};
+  void **ptrs[4] = {&buf.meta, &buf.cta, &buf.split, &buf.codes};
+  for (int i = 0; i < 4; ++i) {
+    *ptrs[i] = nullptr;
+    if (sizes[i] == 0) continue;
+    if (owned) {
+      const cudaError_t e = cudaMalloc(ptrs[i], sizes[i]);
+      if (e != cudaSuccess) return cuda_fail(ctx, e, "batch buffers");
+    } else {
+      const sk_status st = scratch(ctx, slots[i], sizes[i], ptrs[i]);
+      if (st != SK_OK) return st;
     }
-  } else {
-    sk_status st = scratch(ctx, kSlotLaunchMeta, ml.bytes, &meta);
-    if (st == SK_OK) st = scratch(ctx, kSlotCounts, cta_bytes, &cta);
-    if (st == SK_OK) st = scratch(ctx, kSlotSplitCounts, split_bytes, &split);
-    if (st != SK_OK) return st;
+  }
+  char *m = static_cast<char *>(buf.meta);
+  // the code pointers of tasks and jobs, now that the buffer is known
+  const size_t stride = plan.code_stride();
+  buf.values = static_cast<char *>(buf.codes) + plan.code_bytes() - plan.value_bytes_total();
+  for (Plan::Sub &s : plan.subs) {
+    char *base = static_cast<char *>(buf.codes) + s.code_buf * stride;
+    for (Plan::Code &c : s.codes) {
+      c.task.words = reinterpret_cast<uint32_t *>(base + c.words_off);
+      c.task.lists = reinterpret_cast<uint16_t *>(base + c.lists_off);
+      c.task.planes = reinterpret_cast<uint8_t *>(base + c.planes_off);
+      c.task.chunks = reinterpret_cast<const int4 *>(m + ml.chunks_off) + c.chunk0;
+      c.task.status = ctx->status_dev;
+      c.task.col_values = reinterpret_cast<const uint32_t *>(buf.values + plan.values[c.values].off);
+      plan.jobs[c.job].code_words = c.task.words;
+      plan.jobs[c.job].code_planes = c.task.planes;
+    }
   }
   // one upload: the parts are laid out in a host image first
   std::vector<char> image(ml.ctrl_off);
-  std::memcpy(image.data(), plan.jobs.data(), plan.jobs.size() * sizeof(JobParams));
-  if (!plan.items.empty())
-    std::memcpy(image.data() + ml.items_off, plan.items.data(), plan.items.size() * sizeof(WorkItem));
-  if (!plan.splits.empty())
-    std::memcpy(image.data() + ml.splits_off, plan.splits.data(),
-                plan.splits.size() * sizeof(SplitTile));
-  char *m = static_cast<char *>(meta);
-  buf.meta = meta;
-  buf.cta = cta;
-  buf.split = split;
+  auto place = [&](size_t at, const void *src, size_t bytes) {
+    if (bytes) std::memcpy(image.data() + at, src, bytes);
+  };
+  place(0, plan.jobs.data(), plan.jobs.size() * sizeof(JobParams));
+  place(ml.items_off, plan.items.data(), plan.items.size() * sizeof(WorkItem));
+  place(ml.splits_off, plan.splits.data(), plan.splits.size() * sizeof(SplitTile));
+  place(ml.chunks_off, plan.chunks.data(), plan.chunks.size() * sizeof(int4));
   cudaError_t e = cudaMemcpyAsync(m, image.data(), image.size(), cudaMemcpyHostToDevice, ctx->stream);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "work list upload");
   buf.ctrl = m + ml.ctrl_off;
@@ -575,10 +774,9 @@ sk_status upload_plan(sk_ctx *ctx, const Plan &plan, LaunchBuffers &buf, bool ow
   lp.items = reinterpret_cast<const WorkItem *>(m + ml.items_off);
   lp.splits = reinterpret_cast<const SplitTile *>(m + ml.splits_off);
   lp.item_counter = reinterpret_cast<unsigned long long *>(m + ml.ctrl_off);
-  lp.cta_scratch = static_cast<uint16_t *>(cta);
-  lp.split_scratch = static_cast<uint16_t *>(split);
+  lp.cta_scratch = static_cast<uint16_t *>(buf.cta);
+  lp.split_scratch = static_cast<uint16_t *>(buf.split);
   lp.k_slots = plan.k_slots;
-  lp.wide = plan.wide ? 1 : 0;
   lp.status = ctx->status_dev;
   lp.cancel = ctx->cancel_dev;
   return SK_OK;
@@ -602,8 +800,19 @@ sk_status enqueue_launch(sk_ctx *ctx, const Plan &plan, const LaunchBuffers &buf
   lp.n_splits = sub.n_splits;
   lp.split_slots = sub.split_slots;
   lp.item_counter += i;
+  lp.wide = sub.wide ? 1 : 0;
+  lp.coded = sub.codes.empty() ? 0 : 1;
   const int g = static_cast<int>(std::min<int64_t>(plan.grid, lp.n_items));
-  cudaError_t e = plan.cfg->launch(lp, g, stream);
+  cudaError_t e = cudaSuccess;
+  if (!plan.values_by_caller)
+    for (size_t v = sub.values0; v < sub.values0 + sub.n_values && e == cudaSuccess; ++v)
+      e = launch_code_values(plan.values[v].packed, plan.values[v].kb, plan.values[v].ng, 0,
+                             plan.values[v].ng,
+                             reinterpret_cast<uint32_t *>(buf.values + plan.values[v].off),
+                             plan.sm_count, stream);
+  for (const Plan::Code &c : sub.codes)
+    if (e == cudaSuccess) e = launch_codes(c.task, plan.sm_count, stream);
+  if (e == cudaSuccess) e = plan.cfg->launch(lp, g, stream);
   return e == cudaSuccess ? SK_OK : cuda_fail(ctx, e, "distance kernel launch");
 }
 
@@ -619,11 +828,45 @@ int resident_grid(sk_ctx *ctx, const TileConfig &cfg) {
   return per_sm < 1 ? 0 : per_sm * ctx->sm_count;
 }
 
-// One launch over every tile of the jobs, the jobs in decreasing cost per tile
-// (K x blocks, longest first) so the dynamic queue ends on the cheapest items.
+// Whether this plan codes a job: a shape with a coded instance, a job worth
+// it, and a budget that holds a row block over one column group.
+bool Plan::can_code(const JobParams &jp) const {
+  return code_budget > 0 && cfg->id == kCodedConfig && jp.n_tiles > 0 &&
+         use_codes(jp.n_rows, jp.n_cols, jp.n_kmers, jp.nb, jp.self != 0) &&
+         row_block_bytes(static_cast<int64_t>(jp.n_kmers) * jp.nb, 1) <= code_budget;
+}
+
+// Value and code bytes of the jobs that are worth coding.
+void code_wants(const std::vector<JobParams> &jobs, const TileConfig &cfg, size_t *values,
+                size_t *codes) {
+  *values = *codes = 0;
+  std::vector<const uint32_t *> seen;
+  for (const JobParams &jp : jobs) {
+    if (cfg.id != kCodedConfig || jp.n_tiles == 0 ||
+        !use_codes(jp.n_rows, jp.n_cols, jp.n_kmers, jp.nb, jp.self != 0))
+      continue;
+    *codes += code_bytes_wanted(jp);
+    if (std::find(seen.begin(), seen.end(), jp.col_words) != seen.end()) continue;
+    seen.push_back(jp.col_words);
+    *values += job_value_bytes(jp);
+  }
+}
+
+// Code bytes the context grants to a launch of these jobs, 0 when none of
+// them is to be coded.
+size_t code_budget_for(sk_ctx *ctx, const std::vector<JobParams> &jobs, const TileConfig &cfg) {
+  size_t values = 0, codes = 0;
+  code_wants(jobs, cfg, &values, &codes);
+  return codes ? code_reserve(ctx, values, codes) : 0;
+}
+
+// Every tile of the jobs, the jobs in decreasing cost per tile (K x blocks,
+// longest first) so the dynamic queue ends on the cheapest items: the coded
+// jobs in launches of up to `code_budget` bytes of codes (0: none are coded),
+// the others in one launch.
 sk_status make_plan(sk_ctx *ctx, const std::vector<JobParams> &jobs, const TileConfig &cfg,
-                    Plan &plan) {
-  sk_status st = plan.start(ctx, jobs, cfg);
+                    size_t code_budget, Plan &plan) {
+  sk_status st = plan.start(ctx, cfg, code_budget);
   if (st != SK_OK) return st;
   std::vector<int> order(jobs.size());
   for (size_t j = 0; j < jobs.size(); ++j) order[j] = static_cast<int>(j);
@@ -632,15 +875,21 @@ sk_status make_plan(sk_ctx *ctx, const std::vector<JobParams> &jobs, const TileC
            static_cast<int64_t>(jobs[b].n_kmers) * jobs[b].nb;
   });
   for (int j : order)
-    for (int64_t t = 0; t < jobs[j].n_tiles; ++t) plan.add_tile(j, t);
-  plan.close_launch();
+    if (plan.can_code(jobs[j])) plan.add_coded(jobs[j], 0, jobs[j].n_row_tiles, 0, jobs[j].n_col_tiles, 0);
+  if (!plan.open_empty()) plan.close_launch();
+  for (int j : order)
+    if (!plan.can_code(jobs[j])) {
+      const int at = plan.add_job(jobs[j]);
+      for (int64_t t = 0; t < jobs[j].n_tiles; ++t) plan.add_tile(at, t);
+    }
+  if (!plan.open_empty()) plan.close_launch();
   return SK_OK;
 }
 
 sk_status launch_job(sk_ctx *ctx, const JobParams &jp, const TileConfig &cfg) {
   if (jp.n_tiles == 0) return SK_OK;
   Plan plan;
-  sk_status st = make_plan(ctx, {jp}, cfg, plan);
+  sk_status st = make_plan(ctx, {jp}, cfg, code_budget_for(ctx, {jp}, cfg), plan);
   if (st != SK_OK) return st;
   LaunchBuffers buf;
   st = upload_plan(ctx, plan, buf, false);
@@ -748,10 +997,19 @@ sk_status dense_blocked_to_host(sk_ctx *ctx, const sk_db *ref, const sk_db *quer
   for (int c = 0; c < nblk; ++c) jobs[c].out = buf[c & 1];
   Plan plan;
   LaunchBuffers lb;
-  st = plan.start(ctx, jobs, *cfg);
+  st = plan.start(ctx, *cfg, code_budget_for(ctx, {base}, *cfg));
+  const bool coded = plan.can_code(base);
+  std::vector<size_t> sub_end(nblk);   // launches of blocks 0 .. c
   for (int c = 0; st == SK_OK && c < nblk; ++c) {
-    for (int64_t t = first_tile(cut[c]); t < first_tile(cut[c + 1]); ++t) plan.add_tile(c, t);
-    plan.close_launch();
+    if (coded) {
+      plan.add_coded(jobs[c], static_cast<int32_t>(cut[c]), static_cast<int32_t>(cut[c + 1]), 0,
+                     base.n_col_tiles, 0);
+    } else {
+      const int at = plan.add_job(jobs[c]);
+      for (int64_t t = first_tile(cut[c]); t < first_tile(cut[c + 1]); ++t) plan.add_tile(at, t);
+    }
+    if (!plan.open_empty()) plan.close_launch();
+    sub_end[c] = plan.subs.size();
   }
   if (st == SK_OK) st = upload_plan(ctx, plan, lb, false);
   if (st == SK_OK) st = reset_plan(ctx, lb);
@@ -774,8 +1032,8 @@ sk_status dense_blocked_to_host(sk_ctx *ctx, const sk_db *ref, const sk_db *quer
     if (c < nblk) {
       const int b = c & 1;
       if (c >= 2) e = cudaStreamWaitEvent(ctx->stream, ctx->ev_free[b], 0);
-      if (e == cudaSuccess) {
-        st = enqueue_launch(ctx, plan, lb, c, ctx->stream);
+      for (size_t i = c == 0 ? 0 : sub_end[c - 1]; e == cudaSuccess && i < sub_end[c]; ++i) {
+        st = enqueue_launch(ctx, plan, lb, i, ctx->stream);
         if (st != SK_OK) return st;
       }
       if (e == cudaSuccess) e = cudaEventRecord(ctx->ev_ready[b], ctx->stream);

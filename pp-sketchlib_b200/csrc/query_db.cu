@@ -173,12 +173,38 @@ extern "C" sk_status sk_query_db_ready(sk_ctx *ctx, const sk_host_sketches *ref,
       }
     }
   }
+  // the two compute streams alternate between the halves of the code buffer
   Plan plan;
-  st = plan.start(ctx, {jp}, *cfg);
+  st = plan.start(ctx, *cfg, code_budget_for(ctx, {jp}, *cfg) / 2);
   if (st != SK_OK) return st;
-  for (int c = 0; c < n_chunks; ++c) {
-    for (int64_t t : bucket[c]) plan.add_tile(0, t);
-    plan.close_launch();
+  plan.values_by_caller = true;   // chunk by chunk, behind each pack
+  const bool coded = plan.can_code(jp) && !blocked;
+  const int whole = coded ? -1 : plan.add_job(jp);
+  std::vector<size_t> sub0(n_chunks), sub1(n_chunks);   // launches of each chunk
+  std::vector<int> side(n_chunks);                      // compute stream of each chunk
+  for (int k = 0, launches = 0; k < n_chunks; ++k) {
+    const int c = reverse ? n_chunks - 1 - k : k;       // in upload order
+    sub0[c] = plan.subs.size();
+    side[c] = launches & 1;
+    if (coded) {
+      // self: the row tiles that start in the chunk, over every column from
+      // the diagonal on; query: every row tile over the chunk's columns
+      const auto tile_at = [&](int64_t s, int32_t n) {
+        return static_cast<int32_t>(std::min<int64_t>(s / kCodeGroup, n));
+      };
+      if (jp.self)
+        plan.add_coded(jp, tile_at(c * cs, jp.n_row_tiles), tile_at((c + 1) * cs, jp.n_row_tiles),
+                       0, jp.n_col_tiles, side[c]);
+      else
+        plan.add_coded(jp, 0, jp.n_row_tiles, tile_at(c * cs, jp.n_col_tiles),
+                       c + 1 == n_chunks ? jp.n_col_tiles
+                                         : tile_at((c + 1) * cs, jp.n_col_tiles), side[c]);
+    } else if (!blocked) {
+      for (int64_t t : bucket[c]) plan.add_tile(whole, t);
+    }
+    if (!plan.open_empty()) plan.close_launch();
+    sub1[c] = plan.subs.size();
+    if (sub1[c] > sub0[c]) ++launches;
   }
 
   // ---- device buffers: the plan, count scratch for the second stream, staging
@@ -234,7 +260,6 @@ extern "C" sk_status sk_query_db_ready(sk_ctx *ctx, const sk_host_sketches *ref,
   // scratch and every launch its own control block.
   uint64_t *stage[2] = {static_cast<uint64_t *>(staging), static_cast<uint64_t *>(staging) + cs * wps};
   cudaStream_t compute[2] = {ctx->stream, ctx->stream_b};
-  int launches = 0;
   for (size_t i = 0; i < units.size() && e == cudaSuccess; ++i) {
     const Unit &u = units[i];
     const int b = static_cast<int>(i & 1);
@@ -254,14 +279,20 @@ extern "C" sk_status sk_query_db_ready(sk_ctx *ctx, const sk_host_sketches *ref,
       e = launch_pack_range(stage[b], u.n, n_kmers, sketchsize64, ng, g0, u.db->ng, u.db->packed,
                             ctx->pack_stream);
     if (e == cudaSuccess) e = cudaEventRecord(ctx->ev_free[b], ctx->pack_stream);
+    if (e == cudaSuccess && coded && u.db == dbs.ref)
+      e = launch_code_values(u.db->packed, n_kmers * jp.nb, u.db->ng, g0, ng,
+                             reinterpret_cast<uint32_t *>(lb[0].values), plan.sm_count,
+                             ctx->pack_stream);
     if (e == cudaSuccess) e = cudaEventRecord(ctx->ev_chunk[i], ctx->pack_stream);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "sketch upload");
-    if (!blocked && u.chunk >= 0 && plan.subs[u.chunk].n_items > 0) {
-      const int w = launches++ & 1;
+    if (u.chunk >= 0 && sub1[u.chunk] > sub0[u.chunk]) {
+      const int w = side[u.chunk];
       e = cudaStreamWaitEvent(compute[w], ctx->ev_chunk[i], 0);   // packs complete in unit order
       if (e != cudaSuccess) return cuda_fail(ctx, e, "distance kernel launch");
-      st = enqueue_launch(ctx, plan, lb[w], u.chunk, compute[w]);
-      if (st != SK_OK) return st;
+      for (size_t j = sub0[u.chunk]; j < sub1[u.chunk]; ++j) {
+        st = enqueue_launch(ctx, plan, lb[w], j, compute[w]);
+        if (st != SK_OK) return st;
+      }
       if (stream_out) {   // this chunk's rows are final: copy them back now
         const int64_t i0 = u.chunk * cs, i1 = std::min<int64_t>((u.chunk + 1) * cs, n_ref - 1);
         if (i1 > i0) {

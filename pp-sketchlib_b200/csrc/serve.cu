@@ -114,6 +114,10 @@ struct Slot {
   bool high = false;                 // the running slice is on hi_stream
 };
 
+// Coded tiles a slot keeps at most: about 160 column tiles of 100 queries at
+// K = 10 and 312 blocks, a little over one wave.
+constexpr size_t kSlotCodeBytes = size_t(2) << 30;
+
 // A request waiting longer than this goes ahead of every younger request.
 constexpr double kStarveSeconds = 2.0;
 
@@ -208,7 +212,7 @@ sk_status reserve_slice_scratch(sk_server *sv, Slot &s, int64_t *bytes) {
     // with its own count slot
     int64_t slots = 0, parts = 0;
     tail_bounds(jp, grid, &slots, &parts);
-    meta = std::max(meta, meta_layout(1, static_cast<size_t>(tiles + parts), grid, 1).bytes);
+    meta = std::max(meta, meta_layout(1, static_cast<size_t>(tiles + parts), grid, 0, 1).bytes);
     cta = std::max(cta, static_cast<size_t>(grid) * count_slot_bytes(*c, job_slots(jp)));
     split = std::max(split, static_cast<size_t>(slots) * count_slot_bytes(*c, 1));
   }
@@ -217,7 +221,22 @@ sk_status reserve_slice_scratch(sk_server *sv, Slot &s, int64_t *bytes) {
   if (st == SK_OK) st = scratch(ctx, kSlotCounts, cta, &p);
   if (st == SK_OK) st = scratch(ctx, kSlotSplitCounts, split, &p);
   *bytes += static_cast<int64_t>(meta + cta + split);
-  return st;
+  if (st != SK_OK) return st;
+  // coded tiles of the largest slice (in several launches above kSlotCodeBytes),
+  // where the server's budget has room for them in every slot; a slot without
+  // the buffer compares the 14 planes
+  size_t values = 0, codes = 0;
+  code_wants({jp}, *cfg, &values, &codes);
+  codes = std::min(codes, kSlotCodeBytes);
+  const int64_t budget = sv->params.device_bytes;
+  ctx->code_limit = -1;
+  if (codes > 0 && (budget == 0 || (*bytes + static_cast<int64_t>(values + codes)) *
+                                           sv->params.slots <= budget)) {
+    ctx->code_limit = static_cast<int64_t>(values + codes);
+    if (code_reserve(ctx, values, codes) == codes) *bytes += static_cast<int64_t>(values + codes);
+    else ctx->code_limit = -1;
+  }
+  return SK_OK;
 }
 
 // Queues one slice on its slot's stream.  Called by the scheduler thread only.

@@ -11,8 +11,16 @@
 // 256-byte row read with 128-bit shared-memory loads.
 #pragma once
 
+#include <vector_types.h>
+
 #include <cstddef>
 #include <cstdint>
+
+#if defined(__CUDACC__)
+#define SK_HD __host__ __device__
+#else
+#define SK_HD
+#endif
 
 namespace sk {
 
@@ -29,6 +37,17 @@ constexpr int kMaxSketch64 = 1 << 16;   // sketchsize64 accepted (4.2 M bins per
 // (2046 * 32 = 65,472): a k with more blocks is counted in chunks of this
 // many blocks, each in its own count slot, summed by the epilogue.
 constexpr int kMaxChunkBlocks = 2046;
+
+// Coded tiles (code_kernels.cu): bins as codes of a dictionary per block of
+// kCodeGroup rows, stored as bit planes of 128-sample groups.
+constexpr int kCodeGroup = 128;         // rows per dictionary, samples per group
+constexpr int kCodeMaxPlanes = 8;       // codes 0 .. 128
+constexpr int kCodeMinPlanes = 4;       // the fewest the distance kernel compares
+constexpr int kCodeStripeWords = kCodeMaxPlanes * kCodeGroup;   // uint32 per (kb, group): 4 KB
+constexpr int kCodeListWords = 32 * kCodeGroup;                 // uint16 per (row block, kb)
+constexpr uint16_t kCodeNoValue = 0xFFFF;                       // unused dictionary entry
+constexpr int kCodeChunkGroups = 16;    // column groups one CTA of the encoder takes at a time
+constexpr int kValueStripeWords = 16 * kGranule;   // uint32 per (kb, granule) of bin values
 
 // Output modes (public values in sketchlib_b200.h) plus internal single-column modes.
 enum OutMode : int {
@@ -47,6 +66,32 @@ struct DevStatus {
   unsigned long long tiles_done;
   unsigned long long next_poll;   // %globaltimer before which nobody reads the host's cancel word
 };
+
+// Where the coded groups of a range of row blocks lie.  Row block rb holds its
+// own rows as group 0, then column groups first .. cg1 - 1 (first = rb for an
+// all-vs-all range, cg0 otherwise), for each of the KB = n_kmers * nb blocks.
+struct CodeLayout {
+  int32_t self;       // 1: columns from the row block on
+  int32_t rb0;        // first row block of the range
+  int32_t cg0, cg1;   // column groups
+};
+SK_HD inline int32_t code_first_group(const CodeLayout &l, int32_t rb) {
+  return l.self ? rb : l.cg0;
+}
+SK_HD inline int32_t code_groups(const CodeLayout &l, int32_t rb) {
+  return 1 + l.cg1 - code_first_group(l, rb);
+}
+SK_HD inline int64_t code_groups_before(const CodeLayout &l, int32_t rb) {
+  const int64_t n = rb - l.rb0;
+  if (!l.self) return n * (1 + l.cg1 - l.cg0);
+  return n * (1 + l.cg1) - n * (static_cast<int64_t>(l.rb0) + rb - 1) / 2;
+}
+// First word of group g of row block rb at block kb of KB.
+SK_HD inline int64_t code_stripe(const CodeLayout &l, int32_t KB, int32_t rb, int32_t kb,
+                                 int32_t g) {
+  return (code_groups_before(l, rb) * KB + static_cast<int64_t>(kb) * code_groups(l, rb) + g) *
+         kCodeStripeWords;
+}
 
 // Everything one distance launch (one job) needs.  Rows are the "this"/query
 // side of a pair, columns the reference side; for all-vs-all both are the
@@ -90,20 +135,35 @@ struct JobParams {
   // clusters by sample index as the all-vs-all path does.
   int32_t self_view;
   int64_t row_base;
+  // Coded launches: the tiles' codes instead of row_words / col_words.
+  CodeLayout code;
+  const uint32_t *code_words;
+  const uint8_t *code_planes;   // [row blocks][n_kmers * nb] planes per block
+};
+
+// One range of row blocks to encode (code_kernels.cu).
+struct CodeTask {
+  const uint32_t *row_words;   // packed stripes of the rows
+  const uint32_t *col_values;  // bin values of the columns (code_values_kernel)
+  int32_t ng_rows, ng_cols;
+  int64_t n_rows;
+  int32_t kb;            // n_kmers * nb
+  int32_t n_rb;          // row blocks
+  CodeLayout layout;
+  uint32_t *words;
+  uint8_t *planes;
+  uint16_t *lists;       // [n_rb][kb][32 bins][kCodeGroup] dictionary values
+  const int4 *chunks;    // (first of two row blocks of the range, first and end column group)
+  int32_t n_chunks;
+  DevStatus *status;
 };
 
 // Count slots one job's tile needs: one per (k, chunk of blocks).
-#if defined(__CUDACC__)
-__host__ __device__
-#endif
-inline int32_t job_slots(const JobParams &jp) { return jp.n_kmers * jp.nchunk; }
+SK_HD inline int32_t job_slots(const JobParams &jp) { return jp.n_kmers * jp.nchunk; }
 
 // Jobs the wide kernel instance must run: more k-mer lengths than the narrow
 // instance finishes, or sketches counted in chunks.
-#if defined(__CUDACC__)
-__host__ __device__
-#endif
-inline bool needs_wide(const JobParams &jp) { return jp.n_kmers > kNarrowKmers || jp.nchunk > 1; }
+SK_HD inline bool needs_wide(const JobParams &jp) { return jp.n_kmers > kNarrowKmers || jp.nchunk > 1; }
 
 // One unit of work of the persistent distance kernel: k-mer indices
 // [k0, k1) of one tile of one job.  A tile cut into several items (the last
@@ -138,16 +198,14 @@ struct LaunchParams {
   int32_t k_slots;                    // largest K x nchunk over the jobs
   int32_t split_slots;                // largest count-slot need of a split tile
   int32_t wide;                       // 1: some job needs the wide kernel instance
+  int32_t coded;                      // 1: the coded instance, over the jobs' codes
   DevStatus *status;
   const volatile int *cancel;
 };
 
 // splitmix64 finaliser: the counter-based hash of the synthetic generator.
 // Identical on host and device (pure integer arithmetic).
-#if defined(__CUDACC__)
-__host__ __device__
-#endif
-inline uint64_t synth_mix(uint64_t x) {
+SK_HD inline uint64_t synth_mix(uint64_t x) {
   x ^= x >> 30;
   x *= 0xBF58476D1CE4E5B9ULL;
   x ^= x >> 27;
@@ -161,10 +219,7 @@ inline uint64_t synth_mix(uint64_t x) {
 // (probability 1-(1-c)^k(1-a) for its branch), in which case it draws a fresh
 // uniform value; roots always draw.  Walking up the lineage makes every bin
 // independent of the order samples are generated in.
-#if defined(__CUDACC__)
-__host__ __device__
-#endif
-inline uint32_t synth_bin(const int32_t *parent, const uint32_t *thresh,
+SK_HD inline uint32_t synth_bin(const int32_t *parent, const uint32_t *thresh,
                           int32_t n_kmers, int64_t s, int32_t k, uint32_t bin,
                           uint64_t seed) {
   int64_t node = s;

@@ -27,11 +27,20 @@ const TileConfig *tile_config(int id);
 // The 64 x 64 shape (8 x 4 pairs per thread, three CTAs per SM) used where
 // 128 x 128 tiles would be mostly padding.
 constexpr int kSmallTileConfig = 6;
+// The shape with a coded instance.
+constexpr int kCodedConfig = 1;
 // Bytes of count scratch per slot (one per CTA, one per split tile).
 inline size_t count_slot_bytes(const TileConfig &cfg, int k_slots) {
   return static_cast<size_t>(k_slots) * cfg.tile_rows * cfg.tile_cols * 2;
 }
 
+
+// code_kernels.cu: bin values of granules g0 .. g0 + n_g - 1 of a packed array
+// of ng granules; the row and column encoders of one task.
+cudaError_t prepare_code_kernels();
+cudaError_t launch_code_values(const uint32_t *packed, int32_t kb, int32_t ng, int32_t g0,
+                               int32_t n_g, uint32_t *values, int sm_count, cudaStream_t stream);
+cudaError_t launch_codes(const CodeTask &t, int sm_count, cudaStream_t stream);
 
 // aux_kernels.cu
 cudaError_t launch_pack(const uint64_t *words, int64_t n, int32_t n_kmers, int32_t s64,

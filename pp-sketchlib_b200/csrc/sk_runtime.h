@@ -39,7 +39,8 @@ enum ScratchSlot : int {
   kSlotSketchBins = 15,   // bin minima per (sample, k)
   kSlotSketchWords = 16,  // finished sketches, inverse minhashes, densify flags
   kSlotSketchTable = 17,  // k-mer count table of read sets
-  kSlotCount = 18
+  kSlotCodes = 18,        // coded tiles (code_kernels.cu)
+  kSlotCount = 19
 };
 
 struct sk_ctx {
@@ -55,6 +56,7 @@ struct sk_ctx {
   cudaStream_t d2h_stream = nullptr;    // result rows copied back while later chunks compute
   std::vector<cudaEvent_t> ev_out;      // chunk c's output rows written
   cudaEvent_t ev_join = nullptr;        // second compute stream done
+  int64_t code_limit = 0;               // bytes of coded tiles (0: automatic, -1: none)
   int64_t mem_limit = 0;                // bytes a dense call may stage output in (0 = free memory)
   int sm_count = 0;
   std::string err;
@@ -113,39 +115,77 @@ struct sk_sparse {
 namespace sk {
 
 // Launches of the persistent distance kernel that share a tile shape and one
-// meta buffer: the job table, and per launch its work list and split tiles.
+// meta buffer: the job table, and per launch its work list, split tiles and
+// (coded launches) the row blocks to encode first.
 struct Plan {
+  struct Code {                // one range of row blocks of one job
+    int job;
+    CodeTask task;             // pointers are filled in when the buffers are known
+    size_t words_off, lists_off, planes_off;   // in the launch's code buffer
+    size_t chunk0;             // first entry in chunks
+    size_t values;             // entry in values
+  };
+  struct Values {              // bin values of one column database
+    const uint32_t *packed;
+    int32_t kb, ng;
+    size_t off;                // in the value area, after the code buffers
+  };
   struct Sub {
     size_t item0 = 0, n_items = 0, split0 = 0;
     int32_t n_splits = 0;
     int32_t split_slots = 0;   // largest count-slot need of its split tiles
+    bool wide = false;         // some job needs the wide kernel instance
+    int code_buf = 0;          // which of the plan's two code buffers it uses
+    size_t code_bytes = 0;
+    std::vector<Code> codes;   // empty: a plain launch
+    size_t values0 = 0, n_values = 0;   // value tasks to run first
   };
   const TileConfig *cfg = nullptr;
   int grid = 0;                // resident CTAs
-  bool wide = false;           // some job needs the wide kernel instance
+  int sm_count = 0;
   int32_t k_slots = 1;
+  size_t code_budget = 0;      // bytes of one launch's codes
   std::vector<JobParams> jobs;
   std::vector<WorkItem> items;
   std::vector<SplitTile> splits;
+  std::vector<int4> chunks;
+  std::vector<Values> values;
+  bool values_by_caller = false;   // the caller queues the value tasks itself
   std::vector<Sub> subs;
 
-  sk_status start(sk_ctx *ctx, const std::vector<JobParams> &j, const TileConfig &c);
+  sk_status start(sk_ctx *ctx, const TileConfig &c, size_t budget);
+  int add_job(const JobParams &jp);
   void add_tile(int job, int64_t tile);
-  void close_launch();
+  // The tiles of row tiles [rt0, rt1) and column tiles [ct0, ct1), coded, in
+  // as many launches as the budget asks for.
+  void add_coded(const JobParams &jp, int32_t rt0, int32_t rt1, int32_t ct0, int32_t ct1,
+                 int code_buf);
+  bool can_code(const JobParams &jp) const;
+  void close_launch();         // ends the current launch
+  bool open_empty() const { return items.size() == closed_items_; }
   size_t split_bytes() const;
+  size_t code_stride() const;  // bytes of one code buffer
+  size_t code_bytes() const;   // of the whole plan: code buffers and values
+  size_t value_bytes_total() const { return value_bytes_; }
 
  private:
   int64_t choose_splits(size_t begin);
   void split_tail(size_t begin, Sub &sub);
+  void add_piece(const JobParams &jp, int32_t rb0, int32_t rb1, int32_t cg0, int32_t cg1,
+                 bool self, int code_buf);
+  size_t closed_items_ = 0, closed_values_ = 0, value_bytes_ = 0;
+  Sub open_;
 };
 
 struct MetaLayout {
-  size_t items_off = 0, splits_off = 0, ctrl_off = 0, ctrl_bytes = 0, bytes = 0;
+  size_t items_off = 0, splits_off = 0, chunks_off = 0, ctrl_off = 0, ctrl_bytes = 0, bytes = 0;
 };
-MetaLayout meta_layout(size_t n_jobs, size_t n_items, size_t n_splits, size_t n_subs);
+MetaLayout meta_layout(size_t n_jobs, size_t n_items, size_t n_splits, size_t n_chunks,
+                       size_t n_subs);
 
 struct LaunchBuffers {
-  void *meta = nullptr, *cta = nullptr, *split = nullptr;
+  void *meta = nullptr, *cta = nullptr, *split = nullptr, *codes = nullptr;
+  char *values = nullptr;      // the value area of `codes`
   void *ctrl = nullptr;
   size_t ctrl_bytes = 0;
   LaunchParams lp{};
@@ -186,13 +226,20 @@ sk_status launch_job(sk_ctx *ctx, const JobParams &jp, const TileConfig &cfg);
 sk_status attach_count_tables(sk_ctx *ctx, JobParams *jp, bool alloc = true);
 int32_t tail_block_parts(const JobParams &jp, int64_t r, int grid);
 void tail_bounds(const JobParams &jp, int grid, int64_t *slots, int64_t *items);
+bool use_codes(int64_t n_rows, int64_t n_cols, int32_t n_kmers, int32_t nb, bool self);
+size_t code_bytes_wanted(const JobParams &jp);
+size_t job_value_bytes(const JobParams &jp);
+size_t code_reserve(sk_ctx *ctx, size_t values, size_t codes);
+void code_wants(const std::vector<JobParams> &jobs, const TileConfig &cfg, size_t *values,
+                size_t *codes);
+size_t code_budget_for(sk_ctx *ctx, const std::vector<JobParams> &jobs, const TileConfig &cfg);
 double padded_pairs(const TileConfig &cfg, int64_t n_ref, int64_t n_query);
 sk_status db_alloc(sk_ctx *ctx, int64_t n, const int32_t *kmers, int32_t K, int32_t s64,
                    int32_t bbits, sk_db **out, int packed_slot = -1);
 void db_free(sk_db *db);
 sk_status make_plan(sk_ctx *ctx, const std::vector<JobParams> &jobs, const TileConfig &cfg,
-                    Plan &plan);
-sk_status upload_plan(sk_ctx *ctx, const Plan &plan, LaunchBuffers &buf, bool owned);
+                    size_t code_budget, Plan &plan);
+sk_status upload_plan(sk_ctx *ctx, Plan &plan, LaunchBuffers &buf, bool owned);
 sk_status reset_plan(sk_ctx *ctx, const LaunchBuffers &buf);
 sk_status enqueue_launch(sk_ctx *ctx, const Plan &plan, const LaunchBuffers &buf, size_t i,
                          cudaStream_t stream);
