@@ -23,7 +23,7 @@ LIB = PKG / "sketchlib_b200" / "libsketchlib_b200.so"
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 
-CUDA_SOURCES = ["dist_kernel.cu", "code_kernels.cu", "aux_kernels.cu", "probe_kernels.cu", "capi.cu", "batch.cu",
+CUDA_SOURCES = ["dist_kernel.cu", "code_kernels.cu", "query_kernel.cu", "aux_kernels.cu", "probe_kernels.cu", "capi.cu", "batch.cu",
                 "serve.cu", "noalloc.cu", "query_db.cu", "sketch.cu"]
 
 

@@ -886,8 +886,33 @@ sk_status make_plan(sk_ctx *ctx, const std::vector<JobParams> &jobs, const TileC
   return SK_OK;
 }
 
+// Whether a query job goes to the few-queries kernel: no tile shape forced or
+// tuned, narrow, and few rows.  Both kernels run at the same LOP3 rate, so the
+// line is the padding: groups of 1 .. 16 rows there, tiles of 64 or 128 rows
+// here.  Against 30,011 references (K = 10, 156 words), tiles and groups: 1
+// query 5.9 and 0.8 ms, 32 queries 6.0 and 2.8, 64 queries 6.0 and 5.5, 70
+// queries 10.5 and 7.1, 100 queries 10.5 and 10.3, 128 queries 10.6 and 10.8.
+// Against few references a tile's parts fill the device better: 300 references,
+// 32 queries 130 and 100 us, 48 queries 114 and 120, 100 queries 189 and 242.
+bool few_queries(const sk_ctx *ctx, const JobParams &jp) {
+  if (jp.self || jp.n_rows > kFewQueries || needs_wide(jp) || ctx->tile_cfg != 0 ||
+      ctx->tuning.find({jp.n_kmers, jp.nb / 2}) != ctx->tuning.end())
+    return false;
+  if (jp.n_rows <= 32) return true;
+  return jp.n_cols >= 1000 &&
+         1.05 * static_cast<double>(few_queries_rows(jp.n_rows)) <= (jp.n_rows <= 64 ? 64 : 128);
+}
+
 sk_status launch_job(sk_ctx *ctx, const JobParams &jp, const TileConfig &cfg) {
   if (jp.n_tiles == 0) return SK_OK;
+  if (few_queries(ctx, jp)) {
+    void *parts = nullptr;
+    sk_status st = scratch(ctx, kSlotSplitCounts, few_queries_bytes(jp, ctx->sm_count), &parts);
+    if (st != SK_OK) return st;
+    const cudaError_t e = launch_few_queries(jp, static_cast<uint16_t *>(parts), ctx->status_dev,
+                                             ctx->cancel_dev, ctx->sm_count, ctx->stream);
+    return e == cudaSuccess ? SK_OK : cuda_fail(ctx, e, "query kernel launch");
+  }
   Plan plan;
   sk_status st = make_plan(ctx, {jp}, cfg, code_budget_for(ctx, {jp}, cfg), plan);
   if (st != SK_OK) return st;

@@ -216,6 +216,11 @@ sk_status reserve_slice_scratch(sk_server *sv, Slot &s, int64_t *bytes) {
     cta = std::max(cta, static_cast<size_t>(grid) * count_slot_bytes(*c, job_slots(jp)));
     split = std::max(split, static_cast<size_t>(slots) * count_slot_bytes(*c, 1));
   }
+  for (int64_t nq = 1; nq <= std::min<int64_t>(sq, kFewQueries); ++nq) {
+    JobParams few = jp;
+    few.n_rows = nq;
+    if (few_queries(ctx, few)) split = std::max(split, few_queries_bytes(few, ctx->sm_count));
+  }
   void *p = nullptr;
   st = scratch(ctx, kSlotLaunchMeta, meta, &p);
   if (st == SK_OK) st = scratch(ctx, kSlotCounts, cta, &p);

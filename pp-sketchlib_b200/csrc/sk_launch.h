@@ -42,6 +42,14 @@ cudaError_t launch_code_values(const uint32_t *packed, int32_t kb, int32_t ng, i
                                int32_t n_g, uint32_t *values, int sm_count, cudaStream_t stream);
 cudaError_t launch_codes(const CodeTask &t, int sm_count, cudaStream_t stream);
 
+// query_kernel.cu: a narrow query job of at most kFewQueries rows; `parts` holds
+// few_queries_bytes(jp).
+constexpr int kFewQueries = 128;
+int64_t few_queries_rows(int64_t n);   // rows computed for n queries, padding included
+size_t few_queries_bytes(const JobParams &jp, int sm_count);
+cudaError_t launch_few_queries(const JobParams &jp, uint16_t *parts, DevStatus *status,
+                               const volatile int *cancel, int sm_count, cudaStream_t stream);
+
 // aux_kernels.cu
 cudaError_t launch_pack(const uint64_t *words, int64_t n, int32_t n_kmers, int32_t s64,
                         int32_t ng, uint32_t *packed, cudaStream_t stream);

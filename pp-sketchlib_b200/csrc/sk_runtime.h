@@ -214,6 +214,7 @@ void plan_tiles(JobParams &jp, const TileConfig &cfg);
 sk_status build_job(sk_ctx *ctx, const sk_db *ref, const sk_db *query, const sk_random *random,
                     int out_mode, int out_col, void *d_out, const TileConfig **cfg_out,
                     JobParams *jp);
+bool few_queries(const sk_ctx *ctx, const JobParams &jp);
 sk_status launch_job(sk_ctx *ctx, const JobParams &jp, const TileConfig &cfg);
 // Points a job without random-match correction at the context's Jaccard /
 // log-Jaccard tables by count for its union size, built on first use (one
