@@ -160,114 +160,103 @@ __global__ void synth_kernel(const int32_t *__restrict__ parent, const uint32_t 
 
 // ----------------------------------------------------------------------- kNN
 
-// Self kNN over a condensed single column: lane = row i of a 32-row block.
-// Each lane keeps its kNN best (key, j) in shared memory, sorted ascending;
-// j is visited in increasing order, so equal keys keep the smaller j first.
-// Keys are the distances, or 1 - J for Jaccard (src/api.cpp:370-371).
-__global__ void knn_self_kernel(const float *__restrict__ vals, int64_t n, int knn, int jaccard,
-                                int64_t *__restrict__ j_out, float *__restrict__ d_out) {
-  extern __shared__ unsigned char smem[];
-  float *key = reinterpret_cast<float *>(smem);
-  int32_t *idx = reinterpret_cast<int32_t *>(key + 32 * knn);
-  const int lane = threadIdx.x;
-  const int64_t i = static_cast<int64_t>(blockIdx.x) * 32 + lane;
-  const bool active = i < n;
-  int count = 0;
-  float worst = FLT_MAX;
-  for (int64_t j = 0; j < n; ++j) {
-    if (!active) break;
-    float d;
-    if (j == i) {
-      d = INFINITY;  // the diagonal (src/api.cpp:365)
-    } else {
-      const int64_t a = j < i ? j : i, b = j < i ? i : j;
-      d = vals[condensed(a, b, n)];
-      if (jaccard) d = 1.0f - d;
-    }
-    if (count < knn || d < worst) {
-      int pos = count < knn ? count++ : knn - 1;
-      while (pos > 0 && key[(pos - 1) * 32 + lane] > d) {
-        key[pos * 32 + lane] = key[(pos - 1) * 32 + lane];
-        idx[pos * 32 + lane] = idx[(pos - 1) * 32 + lane];
-        --pos;
-      }
-      key[pos * 32 + lane] = d;
-      idx[pos * 32 + lane] = static_cast<int32_t>(j);
-      worst = key[(count - 1) * 32 + lane];
-    }
-  }
-  if (active) {
-    for (int e = 0; e < knn; ++e) {
-      const float k = key[e * 32 + lane];
-      j_out[i * knn + e] = idx[e * 32 + lane];
-      d_out[i * knn + e] = jaccard ? 1.0f - k : k;
-    }
-  }
+// Order-preserving 32-bit image of a key; -0 reads as +0.
+__device__ __forceinline__ uint32_t key_image(float f) {
+  if (f == 0.0f) f = 0.0f;
+  const uint32_t b = __float_as_uint(f);
+  return b ^ ((b >> 31) ? 0xFFFFFFFFu : 0x80000000u);
 }
 
-// Row kNN over a dense (n_rows, n_cols) column: one warp per row, lanes take
-// every 32nd column, then lane 0 merges the 32 sorted lists by (key, col).
-// diag0 >= 0: row r is sample diag0 + r of the column set, whose own column
-// counts as +inf (as in knn_self_kernel); jaccard: keys are 1 - J.
-__global__ void knn_rows_kernel(const float *__restrict__ vals, int64_t n_rows, int64_t n_cols,
-                                int knn, int64_t diag0, int jaccard, int64_t *__restrict__ j_out,
-                                float *__restrict__ d_out) {
-  extern __shared__ unsigned char smem[];
-  float *key = reinterpret_cast<float *>(smem);
-  int32_t *idx = reinterpret_cast<int32_t *>(key + 32 * knn);
-  __shared__ int counts[32];
-  const int lane = threadIdx.x;
+__device__ __forceinline__ float image_key(uint32_t u) {
+  return __uint_as_float(u ^ ((u >> 31) ? 0x80000000u : 0xFFFFFFFFu));
+}
+
+// kNN lists of at most kKnnListMax entries, one CTA per row: SELF, row i of a
+// condensed single column (its own column is +inf, src/api.cpp:365), else a row
+// of a dense (n_rows, n_cols) column; diag0 >= 0: row r is sample diag0 + r of
+// the column set, whose own column counts as +inf.  Keys are the distances, or
+// 1 - J for Jaccard (src/api.cpp:370-371), as 64-bit words (key image, column):
+// unique, and in the order of (key, column).  Each thread keeps the kNN best of
+// every blockDim-th column, sorted, in shared memory; then the CTA takes the
+// smallest head of the lists kNN times.
+//
+// Bound by the latency of the row's reads and insertions, so a row gets up to
+// 256 threads with four reads in flight each (as few as 32 where the lists fill
+// shared memory): with one thread per row of a block of 32 (self) and one warp
+// per row (dense rows), 10 neighbours of 6,007 samples took 3.1 ms and 5 of one
+// row of 30,011 references 0.51 ms.
+template <bool SELF>
+__global__ void knn_lists_kernel(const float *__restrict__ vals, int64_t n_rows, int64_t n_cols,
+                                 int knn, int64_t diag0, int jaccard,
+                                 int64_t *__restrict__ j_out, float *__restrict__ d_out) {
+  extern __shared__ unsigned long long knn_list[];   // [knn][threads]
+  __shared__ unsigned long long warp_min[2][8];
+  const int tid = threadIdx.x, T = blockDim.x, warps = T / 32;
+  constexpr unsigned long long kNone = ~0ull;
   for (int64_t row = blockIdx.x; row < n_rows; row += gridDim.x) {
-    const float *v = vals + row * n_cols;
-    int count = 0;
-    float worst = FLT_MAX;
-    for (int64_t c = lane; c < n_cols; c += 32) {
+    const int64_t own = SELF ? row : (diag0 >= 0 ? diag0 + row : -1);
+    auto word = [&](int64_t c) -> unsigned long long {
       float d;
-      if (diag0 >= 0 && c == diag0 + row) {
+      if (c == own) {
         d = INFINITY;
       } else {
-        d = v[c];
+        d = SELF ? vals[c < row ? condensed(c, row, n_cols) : condensed(row, c, n_cols)]
+                 : vals[row * n_cols + c];
         if (jaccard) d = 1.0f - d;
       }
-      if (count < knn || d < worst) {
-        int pos = count < knn ? count++ : knn - 1;
-        while (pos > 0 && key[(pos - 1) * 32 + lane] > d) {
-          key[pos * 32 + lane] = key[(pos - 1) * 32 + lane];
-          idx[pos * 32 + lane] = idx[(pos - 1) * 32 + lane];
-          --pos;
+      return (static_cast<unsigned long long>(key_image(d)) << 32) | static_cast<uint32_t>(c);
+    };
+    unsigned long long *mine = knn_list + tid;
+    for (int e = 0; e < knn; ++e) mine[e * T] = kNone;
+    unsigned long long worst = kNone;
+    for (int64_t c0 = tid; c0 < n_cols; c0 += 4 * T) {
+      unsigned long long w[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) w[u] = c0 + u * T < n_cols ? word(c0 + u * T) : kNone;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (w[u] >= worst) continue;
+        int pos = knn - 1;
+        for (; pos > 0; --pos) {
+          const unsigned long long up = mine[(pos - 1) * T];
+          if (up < w[u]) break;
+          mine[pos * T] = up;
         }
-        key[pos * 32 + lane] = d;
-        idx[pos * 32 + lane] = static_cast<int32_t>(c);
-        worst = key[(count - 1) * 32 + lane];
+        mine[pos * T] = w[u];
+        worst = mine[(knn - 1) * T];
       }
     }
-    counts[lane] = count;
-    __syncwarp();
-    if (lane == 0) {
-      int head[32];
-      for (int l = 0; l < 32; ++l) head[l] = 0;
-      for (int e = 0; e < knn; ++e) {
-        int best = -1;
-        float bk = 0.0f;
-        int32_t bj = 0;
-        for (int l = 0; l < 32; ++l) {
-          if (head[l] >= counts[l]) continue;
-          const float k = key[head[l] * 32 + l];
-          const int32_t j = idx[head[l] * 32 + l];
-          if (best < 0 || k < bk || (k == bk && j < bj)) { best = l; bk = k; bj = j; }
+    int head = 0;
+    unsigned long long cur = mine[0];
+    for (int e = 0; e < knn; ++e) {
+      unsigned long long m = cur;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long v = __shfl_xor_sync(0xffffffffu, m, o);
+        m = v < m ? v : m;
+      }
+      if (warps > 1) {
+        if ((tid & 31) == 0) warp_min[e & 1][tid >> 5] = m;
+        __syncthreads();
+        for (int i = 0; i < warps; ++i) {
+          const unsigned long long v = warp_min[e & 1][i];
+          m = v < m ? v : m;
         }
-        if (best < 0) { j_out[row * knn + e] = -1; d_out[row * knn + e] = INFINITY; continue; }
-        ++head[best];
-        j_out[row * knn + e] = bj;
-        d_out[row * knn + e] = jaccard ? 1.0f - bk : bk;
+      }
+      if (cur == m) {   // one thread: words are unique (and there are at least kNN of them)
+        const float k = image_key(static_cast<uint32_t>(m >> 32));
+        j_out[row * knn + e] = static_cast<uint32_t>(m);
+        d_out[row * knn + e] = jaccard ? 1.0f - k : k;
+        ++head;
+        cur = head < knn ? mine[head * T] : kNone;
       }
     }
-    __syncwarp();
+    __syncthreads();   // warp_min is written again by the next row
   }
 }
 
 // Row kNN for any kNN up to the row length (the kernels above keep kNN lists
-// per lane in shared memory, up to kKnnListMax entries).  One CTA per row, in four steps:
+// per thread in shared memory, up to kKnnListMax entries).  One CTA per row, in four steps:
 //  1. radix select over the 32-bit order-preserving image of the key (four
 //     8-bit digits, most significant first; a 256-bin shared histogram per
 //     pass over the row) finds the bucket [lo, hi] of keys that holds the
@@ -286,16 +275,6 @@ __global__ void knn_rows_kernel(const float *__restrict__ vals, int64_t n_rows, 
 // 0) +inf, -0 read as +0.
 constexpr int kKnnSelectThreads = 512;
 constexpr int kKnnSmemList = 12288;   // 96 KiB of 64-bit words
-
-__device__ __forceinline__ uint32_t key_image(float f) {
-  if (f == 0.0f) f = 0.0f;
-  const uint32_t b = __float_as_uint(f);
-  return b ^ ((b >> 31) ? 0xFFFFFFFFu : 0x80000000u);
-}
-
-__device__ __forceinline__ float image_key(uint32_t u) {
-  return __uint_as_float(u ^ ((u >> 31) ? 0x80000000u : 0xFFFFFFFFu));
-}
 
 __global__ void __launch_bounds__(kKnnSelectThreads)
 knn_select_kernel(const float *__restrict__ vals, int64_t n_rows, int64_t n_cols, int knn,
@@ -559,18 +538,34 @@ cudaError_t launch_synth(const int32_t *parent, const uint32_t *thresh, int64_t 
   return cudaGetLastError();
 }
 
+namespace {
+
+// Threads per row: 256 while the lists leave room for two CTAs per SM, fewer
+// for longer lists or rows shorter than the threads' lists, 32 at least.
+template <bool SELF>
+cudaError_t launch_knn_lists(const float *vals, int64_t n_rows, int64_t n_cols, int32_t knn,
+                             int64_t diag0, int32_t jaccard, int64_t *j_out, float *d_out,
+                             cudaStream_t stream) {
+  int threads = 256;
+  while (threads > 32 && (threads * knn * 8 > 100 * 1024 || n_cols < 8 * threads)) threads /= 2;
+  const int smem = threads * knn * 8;
+  if (smem > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(knn_lists_kernel<SELF>,
+                                               cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+  }
+  const int blocks = static_cast<int>(n_rows < 148 * 64 ? n_rows : 148 * 64);
+  knn_lists_kernel<SELF><<<blocks > 0 ? blocks : 1, threads, smem, stream>>>(
+      vals, n_rows, n_cols, knn, diag0, jaccard, j_out, d_out);
+  return cudaGetLastError();
+}
+
+}  // namespace
+
 cudaError_t launch_knn_self(const float *col_vals, int64_t n, int32_t knn, int32_t jaccard,
                             int64_t *j_out, float *d_out, cudaStream_t stream) {
   if (knn > kKnnListMax || knn > n) return cudaErrorInvalidValue;
-  const int smem = 32 * knn * 8;
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(knn_self_kernel,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-  }
-  const int blocks = static_cast<int>((n + 31) / 32);
-  knn_self_kernel<<<blocks, 32, smem, stream>>>(col_vals, n, knn, jaccard, j_out, d_out);
-  return cudaGetLastError();
+  return launch_knn_lists<true>(col_vals, n, n, knn, -1, jaccard, j_out, d_out, stream);
 }
 
 cudaError_t launch_knn_rows(const float *vals, int64_t n_rows, int64_t n_cols, int32_t knn,
@@ -589,16 +584,7 @@ cudaError_t launch_knn_rows(const float *vals, int64_t n_rows, int64_t n_cols, i
         vals, n_rows, n_cols, knn, diag0, jaccard, j_out, d_out);
     return cudaGetLastError();
   }
-  const int smem = 32 * knn * 8;
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(knn_rows_kernel,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-  }
-  const int blocks = static_cast<int>(n_rows < 148 * 64 ? n_rows : 148 * 64);
-  knn_rows_kernel<<<blocks > 0 ? blocks : 1, 32, smem, stream>>>(vals, n_rows, n_cols, knn, diag0,
-                                                                 jaccard, j_out, d_out);
-  return cudaGetLastError();
+  return launch_knn_lists<false>(vals, n_rows, n_cols, knn, diag0, jaccard, j_out, d_out, stream);
 }
 
 cudaError_t launch_count_tables(double union_bits, int64_t n, float *jtab, double *ltab,
