@@ -40,7 +40,8 @@ enum ScratchSlot : int {
   kSlotSketchWords = 16,  // finished sketches, inverse minhashes, densify flags
   kSlotSketchTable = 17,  // k-mer count table of read sets
   kSlotCodes = 18,        // coded tiles (code_kernels.cu)
-  kSlotCount = 19
+  kSlotSketchRows = 19,   // per-row state of the low count
+  kSlotCount = 20
 };
 
 struct sk_ctx {

@@ -27,9 +27,10 @@
 //              3(k-1) of a 3k-2 window) are a rolling hash along each of the
 //              three phase subsequences: three states rotate, each stepping
 //              by a split rotation of three with the base 3k back leaving.
-//   counting   with min_count > 0 (read sets), hashes are counted in a device
-//              hash table and the insertion that brings a hash's count to
-//              min_count enters it in its bin: the reference's exact counter
+//   counting   with min_count > 0 (read sets), hashes are counted exactly (for
+//              large samples only those that can still win their bin) and the
+//              occurrence that brings a hash's count to min_count enters it in
+//              its bin: the reference's exact counter
 //              (HashCounter, src/sketch/countmin.cpp:55-72, `exact = true`),
 //              whose answer does not depend on read order.
 #include <cuda_runtime.h>
@@ -496,6 +497,191 @@ count_kernel(SketchArgs a) {
   if (s >= e) return;
   CountBatch emit{a, a.signs + static_cast<int64_t>(it.row) * a.nbins, {}, {}};
   roll_windows<kRc, kPhased>(a.codes, s, e, it.k, tab, emit);
+}
+
+// ---- exact counting from the low end of the bins
+//
+// A bin keeps the smallest hash that occurs min_count times, so only hashes
+// near the low end of their bin matter.  The first roll keeps those below
+// `low`, sized for about kLowPerBin windows per bin; as the test depends on the
+// hash alone, a kept hash is kept at every occurrence and its count is exact.
+// They are written to their item's list, then counted in a global table that
+// stays in L2.  A bin that some hash below `low` fills is done: any other
+// candidate is larger.  Bins still empty (27 in a million when 12.8 of the 128
+// windows are distinct k-mers that qualify) get a second roll that keeps every
+// hash of theirs, or, when that is most of the sample, the whole sample is
+// counted by groups (below).
+//
+// Against counting every hash of a sample by groups (two rolls, 8 bytes
+// written to a random sector per window): 20 Mbases of reads, per k: 430 us
+// before, 127 now (91 the roll, 31 the count, 5 clearing the table).
+struct LowArgs {
+  uint64_t low;                   // keep hashes of a bin below its start + low
+  const unsigned int *empty;      // [rows][words]: keep the hashes of these bins (null: below low)
+  int words;                      // bitmap words per row
+  unsigned long long *hashes;     // [items][cap]
+  unsigned int *count;            // [items] hashes kept (may exceed cap)
+  unsigned int cap;
+  struct TableSlot *tables;       // [tables][slots]
+  unsigned int *max_key;          // [tables] occurrences of the hash equal to kEmptyKey
+  uint64_t slots;                 // a power of two
+  int by_k;                       // table of an item: its k index, or 0
+  unsigned int *overflow;         // [rows] a list or table was too small
+};
+
+// The roll's emitter.  A thread puts its kept hashes into its own column of a
+// shared-memory array (a predicated store, no branch); when some lane of the
+// warp has more than half of its column filled, the lanes write theirs out
+// together.  Writing each kept hash at once took a branch in nearly every step
+// of a warp (105 us per k for 20 Mbases; 91 now, at two CTAs per SM).
+template <bool kBitmap>
+struct LowKeep {
+  static constexpr int kBatch = 8;
+  static constexpr int kColumn = 2 * kBatch;   // a batch fits on top of a half-filled column
+  unsigned long long *column;   // [kColumn][kSketchThreads], this thread's first entry
+  unsigned long long *out;
+  unsigned int *kept;           // entries of the item's list so far
+  unsigned int cap;
+  uint64_t binsize, magic, low;
+  const unsigned int *empty;
+  int n = 0;
+
+  __device__ __forceinline__ void put(uint64_t h, bool valid) {
+    const uint64_t sign = mod_sign(h);
+    const uint32_t q = bin_of(sign, binsize, magic);
+    bool keep = valid;
+    if (kBitmap) keep = keep && ((empty[q >> 5] >> (q & 31)) & 1u);
+    else keep = keep && sign - q * binsize < low;
+    if (keep) column[n * kSketchThreads] = h;
+    n += keep ? 1 : 0;
+  }
+  __device__ __forceinline__ void drain() {
+    if (n == 0) return;
+    const unsigned int at = atomicAdd(kept, static_cast<unsigned int>(n));
+    for (int i = 0; i < n; ++i)
+      if (at + i < cap) out[at + i] = column[i * kSketchThreads];
+    n = 0;
+  }
+  __device__ __forceinline__ void flush() {
+    if (__any_sync(__activemask(), n > kColumn - kBatch)) drain();
+  }
+};
+
+// What roll_windows takes by value: a reference to the emitter above.
+template <bool kBitmap>
+struct LowEmit {
+  static constexpr int kBatch = LowKeep<kBitmap>::kBatch;
+  LowKeep<kBitmap> &keep;
+  __device__ __forceinline__ void put(int, uint64_t h, bool valid) { keep.put(h, valid); }
+  __device__ __forceinline__ void flush() { keep.flush(); }
+};
+
+template <bool kRc, bool kPhased, bool kBitmap>
+__global__ void __launch_bounds__(kSketchThreads, 2)
+low_roll_kernel(SketchArgs a, LowArgs la) {
+  extern __shared__ unsigned long long low_columns[];   // [kColumn][kSketchThreads]
+  __shared__ RollTable tab;
+  __shared__ unsigned int kept;
+  const SketchItem it = a.items[blockIdx.x];
+  if (threadIdx.x < 64) {
+    const ulonglong2 *src = reinterpret_cast<const ulonglong2 *>(a.tables + it.tab);
+    reinterpret_cast<ulonglong2 *>(&tab)[threadIdx.x] = src[threadIdx.x];
+  }
+  if (threadIdx.x == 0) kept = 0;
+  __syncthreads();
+  LowKeep<kBitmap> keep{low_columns + threadIdx.x,
+                        la.hashes + static_cast<int64_t>(blockIdx.x) * la.cap, &kept, la.cap,
+                        a.binsize, a.magic, la.low,
+                        kBitmap ? la.empty + static_cast<int64_t>(it.row) * la.words : nullptr};
+  const int64_t s = it.begin + static_cast<int64_t>(threadIdx.x) * it.per;
+  const int64_t e = min(s + it.per, it.end);
+  if (s < e) {
+    roll_windows<kRc, kPhased>(a.codes, s, e, it.k, tab, LowEmit<kBitmap>{keep});
+    keep.drain();
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    la.count[blockIdx.x] = kept;
+    if (kept > la.cap) la.overflow[it.row] = 1u;
+  }
+}
+
+// Counts the hashes of one item's list; the occurrence that brings a hash's
+// count to min_count puts it in its bin.  A probe chain over kMaxProbes marks
+// the row for the full count (a dropped occurrence only lowers counts, so what
+// is already in the bins stays right).
+constexpr int kMaxProbes = 128;
+constexpr int kLowCountThreads = 256;
+constexpr int kLowCountSplit = 4;     // CTAs per list
+__global__ void __launch_bounds__(kLowCountThreads) low_count_kernel(SketchArgs a, LowArgs la) {
+  const int item = blockIdx.x / kLowCountSplit, part = blockIdx.x % kLowCountSplit;
+  const SketchItem it = a.items[item];
+  const unsigned int n = min(la.count[item], la.cap);
+  const unsigned long long *in = la.hashes + static_cast<int64_t>(item) * la.cap;
+  const int t = la.by_k ? it.tab : 0;
+  TableSlot *table = la.tables + static_cast<int64_t>(t) * la.slots;
+  unsigned long long *row = a.signs + static_cast<int64_t>(it.row) * a.nbins;
+  for (unsigned int i = part * kLowCountThreads + threadIdx.x; i < n;
+       i += kLowCountSplit * kLowCountThreads) {
+    const unsigned long long h = in[i];
+    unsigned int old = 0;
+    if (h == kEmptyKey) {
+      old = atomicAdd(la.max_key + t, 1u);
+    } else {
+      uint64_t slot = table_slot(h, la.slots - 1);
+      int probe = 0;
+      for (; probe < kMaxProbes; ++probe) {
+        TableSlot *ts = table + slot;
+        unsigned long long cur = *reinterpret_cast<volatile unsigned long long *>(&ts->key);
+        if (cur == kEmptyKey) {
+          cur = atomicCAS(&ts->key, kEmptyKey, h);
+          if (cur == kEmptyKey) cur = h;
+        }
+        if (cur == h) {
+          old = atomicAdd(&ts->count, 1u);
+          break;
+        }
+        slot = (slot + 1) & (la.slots - 1);
+      }
+      if (probe == kMaxProbes) {
+        la.overflow[it.row] = 1u;
+        continue;
+      }
+    }
+    if (old + 1 == a.min_count) {
+      const uint64_t sign = mod_sign(h);
+      const uint32_t q = bin_of(sign, a.binsize, a.magic);
+      if (sign < row[q]) atomicMin(row + q, static_cast<unsigned long long>(sign));
+    }
+  }
+}
+
+__global__ void low_clear_kernel(TableSlot *__restrict__ t, uint64_t n, unsigned int *max_key,
+                                 int n_tables) {
+  const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
+  for (uint64_t i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; i < n; i += stride)
+    reinterpret_cast<uint4 *>(t)[i] = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u);
+  if (blockIdx.x == 0 && threadIdx.x < n_tables) max_key[threadIdx.x] = 0;
+}
+
+// Bitmap and number of a row's empty bins (one CTA per row).
+__global__ void __launch_bounds__(256)
+empty_bins_kernel(const unsigned long long *__restrict__ signs, int nbins, int words,
+                  unsigned int *__restrict__ empty, unsigned int *__restrict__ n_empty) {
+  __shared__ unsigned int total;
+  if (threadIdx.x == 0) total = 0;
+  __syncthreads();
+  const unsigned long long *row = signs + static_cast<int64_t>(blockIdx.x) * nbins;
+  for (int i0 = 0; i0 < 32 * words; i0 += 256) {
+    const int i = i0 + threadIdx.x;
+    const unsigned int m = __ballot_sync(0xffffffffu, i < nbins && row[i] == kEmptyKey);
+    if ((threadIdx.x & 31) == 0 && i < 32 * words) {
+      empty[static_cast<int64_t>(blockIdx.x) * words + i / 32] = m;
+      atomicAdd(&total, static_cast<unsigned int>(__popc(m)));
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) n_empty[blockIdx.x] = total;
 }
 
 // ---- partitioned exact counting
@@ -1001,99 +1187,299 @@ sk_status count_partitioned(SketchCall &c, const Batch &b, SketchArgs &args, std
   return e == cudaSuccess ? SK_OK : cuda_fail(ctx, e, "sketch counting");
 }
 
-// Bins rows of one batch with the exact count filter, a hash entering its bin
-// when its count reaches min_count.  Per sample and k the hashes are counted
-// by groups (count_partitioned) when the sample's hash buffer fits the table
-// budget and its groups fit shared memory; otherwise in a global table of
-// twice the sample's windows (in bin-range passes when that exceeds the
-// budget).  The table pass's items are an eighth of the hashing ones (no
-// per-CTA bins to amortise; more CTAs in flight hide the table's memory
-// latency).
+// Every hash of sample s counted at the k indices `ks`, a hash entering its bin
+// when its count reaches min_count.  Per k the hashes are counted by groups
+// (count_partitioned) when the sample's hash buffer fits the table budget and
+// its groups fit shared memory; otherwise in a global table of twice the
+// sample's windows (in bin-range passes when that exceeds the budget).  The
+// table pass's items are an eighth of the hashing ones (no per-CTA bins to
+// amortise; more CTAs in flight hide the table's memory latency).
 constexpr int64_t kCountItemWindows = kItemWindows / 8;
 
+sk_status count_full(SketchCall &c, const Batch &b, SketchArgs &args, std::vector<SketchItem> &items,
+                     int64_t s, const std::vector<int> &ks, uint64_t kTableBudget) {
+  sk_ctx *ctx = c.ctx;
+  const int64_t windows = c.seq_off[c.sample_seqs[s + 1]] - c.seq_off[c.sample_seqs[s]];
+  if (windows <= 0) return SK_OK;
+  int log2p = 0;
+  while (log2p < kMaxLog2Parts && (kPartHashes << log2p) < windows) ++log2p;
+  const int64_t per_part = (windows + (int64_t(1) << log2p) - 1) >> log2p;
+  // 1.5 slots per base of a group: the distinct hashes (at most the
+  // bases) fill at most two thirds of a table
+  const int part_slots =
+      static_cast<int>(std::max<uint64_t>(2048, next_pow2(static_cast<uint64_t>(per_part) * 3 / 2)));
+  // items of the grouped count: two per SM, at least 4 P windows each
+  const int64_t per_item = std::min<int64_t>(
+      kItemWindows, std::max<int64_t>(int64_t(4) << log2p, (windows + 2 * ctx->sm_count - 1) / (2 * ctx->sm_count)));
+  const int64_t max_items = (windows + per_item - 1) / per_item + 1;   // items of one k
+  const uint64_t part_bytes = static_cast<uint64_t>(windows) * 8 + ((uint64_t(3) << log2p) + 1) * 4 +
+                              (static_cast<uint64_t>(max_items) << log2p) * 4 + 256;
+  if (part_slots <= kMaxPartSlots && windows < (int64_t(1) << 32) && part_bytes <= kTableBudget) {
+    void *tk = nullptr;
+    sk_status st = scratch(ctx, kSlotSketchTable, part_bytes, &tk);
+    if (st != SK_OK) return st;
+    PartArgs pa{};
+    pa.hashes = static_cast<unsigned long long *>(tk);
+    pa.count = reinterpret_cast<unsigned int *>(pa.hashes + windows);
+    pa.cursor = pa.count + (1 << log2p);
+    pa.start = pa.cursor + (1 << log2p);
+    pa.cta_count = pa.start + (1 << log2p) + 1;
+    pa.log2p = log2p;
+    pa.table_slots = part_slots;
+    for (int k : ks) {
+      st = count_partitioned(c, b, args, items, s, k, per_item, pa);
+      if (st != SK_OK) return st;
+    }
+    return SK_OK;
+  }
+  const uint64_t want = next_pow2(static_cast<uint64_t>(windows) * 2);
+  const uint64_t passes = std::max<uint64_t>(1, (want * sizeof(TableSlot) + kTableBudget - 1) / kTableBudget);
+  const uint64_t slots = std::max<uint64_t>(1024, next_pow2((want + passes - 1) / passes));
+  void *tk = nullptr;
+  sk_status st = scratch(ctx, kSlotSketchTable, slots * sizeof(TableSlot) + 16, &tk);
+  if (st != SK_OK) return st;
+  args.table = static_cast<TableSlot *>(tk);
+  args.max_key_count = reinterpret_cast<unsigned int *>(static_cast<char *>(tk) + slots * sizeof(TableSlot));
+  args.table_mask = slots - 1;
+  args.min_count = static_cast<unsigned int>(c.min_count);
+  for (int k : ks) {
+    items.clear();
+    make_items(c, b, s, s + 1, k, items, kCountItemWindows);
+    if (items.empty()) continue;
+    void *p = nullptr;
+    st = scratch(ctx, kSlotSketchItems, items.size() * sizeof(SketchItem), &p);
+    if (st == SK_OK) st = upload(ctx, p, items.data(), items.size() * sizeof(SketchItem));
+    if (st != SK_OK) return st;
+    args.items = static_cast<SketchItem *>(p);
+    for (uint64_t pass = 0; pass < passes; ++pass) {
+      args.bin_lo = static_cast<uint32_t>(c.nbins * pass / passes);
+      args.bin_hi = static_cast<uint32_t>(c.nbins * (pass + 1) / passes);
+      table_clear_kernel<<<static_cast<unsigned>(std::min<uint64_t>(4096, (slots + 255) / 256)), 256, 0,
+                           ctx->stream>>>(args.table, slots, args.max_key_count);
+      cudaError_t e = cudaGetLastError();
+      if (e == cudaSuccess) {
+        auto kern = c.codon_phased ? (c.use_rc ? count_kernel<true, true> : count_kernel<false, true>)
+                                   : (c.use_rc ? count_kernel<true, false> : count_kernel<false, false>);
+        kern<<<static_cast<unsigned>(items.size()), kSketchThreads, 0, ctx->stream>>>(args);
+        e = cudaGetLastError();
+      }
+      if (e != cudaSuccess) return cuda_fail(ctx, e, "sketch counting");
+    }
+  }
+  return SK_OK;
+}
+
+// Windows of a bin that the first roll of the low count keeps on average, and
+// the fewest windows per bin for which that roll is worth its while: two read
+// sets at K = 8, 9,984 bins, counted in full and from the low end, took 1.52
+// and 1.73 ms with 200 windows per bin, 2.09 and 1.45 with 400, 3.57 and 2.16
+// with 1,000.
+constexpr int64_t kLowPerBin = 128;
+constexpr int64_t kLowMinPerBin = 256;
+
+int64_t sample_windows(const SketchCall &c, int64_t s) {
+  return c.seq_off[c.sample_seqs[s + 1]] - c.seq_off[c.sample_seqs[s]];
+}
+
+// Buffers of one low count: lists of the items, tables and their counters.
+struct LowPlan {
+  uint64_t slots = 0;
+  unsigned int cap = 0;
+  size_t lists_off = 0, counts_off = 0, bytes = 0;
+};
+
+// For items of at most per_item windows of which a fraction f is kept, n_tables
+// tables each holding the `kept` hashes of one (sample, k) at two thirds at most.
+LowPlan low_plan(double f, int64_t per_item, size_t n_items, int n_tables, double kept) {
+  LowPlan p;
+  p.slots = std::max<uint64_t>(1024, next_pow2(static_cast<uint64_t>(kept * 1.5)));
+  p.cap = static_cast<unsigned int>(per_item * f * 1.25) + 512;
+  p.lists_off = static_cast<size_t>(n_tables) * p.slots * sizeof(TableSlot);
+  p.counts_off = p.lists_off + n_items * p.cap * 8;
+  p.bytes = p.counts_off + (n_items + n_tables) * 4;
+  return p;
+}
+
+// One low count over `items` (uploaded here): tables cleared, roll, count.
+sk_status run_low(SketchCall &c, SketchArgs &args, const std::vector<SketchItem> &items,
+                  const LowPlan &p, int n_tables, LowArgs la) {
+  sk_ctx *ctx = c.ctx;
+  void *tk = nullptr, *di = nullptr;
+  sk_status st = scratch(ctx, kSlotSketchTable, p.bytes, &tk);
+  if (st == SK_OK) st = scratch(ctx, kSlotSketchItems, items.size() * sizeof(SketchItem), &di);
+  if (st == SK_OK) st = upload(ctx, di, items.data(), items.size() * sizeof(SketchItem));
+  if (st != SK_OK) return st;
+  char *base = static_cast<char *>(tk);
+  la.tables = reinterpret_cast<TableSlot *>(base);
+  la.slots = p.slots;
+  la.hashes = reinterpret_cast<unsigned long long *>(base + p.lists_off);
+  la.cap = p.cap;
+  la.count = reinterpret_cast<unsigned int *>(base + p.counts_off);
+  la.max_key = la.count + items.size();
+  la.by_k = n_tables > 1;
+  args.items = static_cast<SketchItem *>(di);
+  const unsigned grid = static_cast<unsigned>(items.size());
+  low_clear_kernel<<<ctx->sm_count * 8, 256, 0, ctx->stream>>>(la.tables, n_tables * p.slots,
+                                                              la.max_key, n_tables);
+  const auto roll =
+      la.empty ? (c.codon_phased ? (c.use_rc ? low_roll_kernel<true, true, true> : low_roll_kernel<false, true, true>)
+                                 : (c.use_rc ? low_roll_kernel<true, false, true> : low_roll_kernel<false, false, true>))
+               : (c.codon_phased ? (c.use_rc ? low_roll_kernel<true, true, false> : low_roll_kernel<false, true, false>)
+                                 : (c.use_rc ? low_roll_kernel<true, false, false> : low_roll_kernel<false, false, false>));
+  constexpr int smem = LowKeep<false>::kColumn * kSketchThreads * 8;
+  const cudaError_t attr = cudaFuncSetAttribute(roll, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (attr != cudaSuccess) return cuda_fail(ctx, attr, "sketch counting");
+  roll<<<grid, kSketchThreads, smem, ctx->stream>>>(args, la);
+  low_count_kernel<<<grid * kLowCountSplit, kLowCountThreads, 0, ctx->stream>>>(args, la);
+  const cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? SK_OK : cuda_fail(ctx, e, "sketch counting");
+}
+
+// Bins rows of one batch with the exact count filter.  Samples of at least
+// kLowMinPerBin windows per bin are counted from the low end of their bins, all
+// k in one roll; what that leaves (bins still empty, lists or tables too small)
+// and the other samples are counted in full.
 sk_status count_batch(SketchCall &c, const Batch &b, SketchArgs &args, std::vector<SketchItem> &items) {
   sk_ctx *ctx = c.ctx;
   const int K = static_cast<int>(c.kmers.size());
   // bytes of table per pass: a quarter of the context's memory limit when one
   // is set, else a quarter of the free device memory less 2 GiB (at least 1 GiB)
-  uint64_t kTableBudget = 0;
+  uint64_t budget = 0;
   if (ctx->mem_limit > 0) {
-    kTableBudget = std::max<uint64_t>(1ULL << 16, static_cast<uint64_t>(ctx->mem_limit) / 4);
+    budget = std::max<uint64_t>(1ULL << 16, static_cast<uint64_t>(ctx->mem_limit) / 4);
   } else {
     size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) free_b = 0;
-    kTableBudget = std::max<uint64_t>(1ULL << 30, free_b > (2ULL << 30) ? (free_b - (2ULL << 30)) / 4 : 0);
+    budget = std::max<uint64_t>(1ULL << 30, free_b > (2ULL << 30) ? (free_b - (2ULL << 30)) / 4 : 0);
   }
   args.min_count = static_cast<unsigned int>(c.min_count);
-  for (int64_t s = b.s0; s < b.s1; ++s) {
-    const int64_t windows = c.seq_off[c.sample_seqs[s + 1]] - c.seq_off[c.sample_seqs[s]];
-    if (windows <= 0) continue;
-    int log2p = 0;
-    while (log2p < kMaxLog2Parts && (kPartHashes << log2p) < windows) ++log2p;
-    const int64_t per_part = (windows + (int64_t(1) << log2p) - 1) >> log2p;
-    // 1.5 slots per base of a group: the distinct hashes (at most the
-    // bases) fill at most two thirds of a table
-    const int part_slots =
-        static_cast<int>(std::max<uint64_t>(2048, next_pow2(static_cast<uint64_t>(per_part) * 3 / 2)));
-    // items of the grouped count: two per SM, at least 4 P windows each
-    const int64_t per_item = std::min<int64_t>(
-        kItemWindows, std::max<int64_t>(int64_t(4) << log2p, (windows + 2 * ctx->sm_count - 1) / (2 * ctx->sm_count)));
-    const int64_t max_items = (windows + per_item - 1) / per_item + 1;   // items of one k
-    const uint64_t part_bytes = static_cast<uint64_t>(windows) * 8 + ((uint64_t(3) << log2p) + 1) * 4 +
-                                (static_cast<uint64_t>(max_items) << log2p) * 4 + 256;
-    if (part_slots <= kMaxPartSlots && windows < (int64_t(1) << 32) && part_bytes <= kTableBudget) {
-      void *tk = nullptr;
-      sk_status st = scratch(ctx, kSlotSketchTable, part_bytes, &tk);
+  std::vector<int> all(K);
+  for (int k = 0; k < K; ++k) all[k] = k;
+
+  // ---- the low end of every large sample
+  const int64_t rows = (b.s1 - b.s0) * K;
+  const int words = (c.nbins + 31) / 32;
+  std::vector<char> low(static_cast<size_t>(b.s1 - b.s0), 0);
+  unsigned int *d_rows = nullptr;   // overflow [rows], empty bins [rows], bitmaps [rows][words]
+  LowArgs la{};
+  la.words = words;
+  bool any = false;
+  auto low_sample = [&](int64_t s) -> sk_status {
+    const int64_t windows = sample_windows(c, s);
+    if (windows < kLowMinPerBin * c.nbins || windows >= (int64_t(1) << 32)) return SK_OK;
+    const double f = static_cast<double>(kLowPerBin) * c.nbins / static_cast<double>(windows);
+    items.clear();
+    make_items(c, b, s, s + 1, -1, items);
+    const LowPlan p = low_plan(f, kItemWindows, items.size(), K, f * static_cast<double>(windows));
+    if (items.empty() || p.bytes > budget) return SK_OK;
+    if (!any) {
+      void *r = nullptr;
+      const sk_status st = scratch(ctx, kSlotSketchRows, static_cast<size_t>(rows) * (2 + words) * 4, &r);
       if (st != SK_OK) return st;
-      PartArgs pa{};
-      pa.hashes = static_cast<unsigned long long *>(tk);
-      pa.count = reinterpret_cast<unsigned int *>(pa.hashes + windows);
-      pa.cursor = pa.count + (1 << log2p);
-      pa.start = pa.cursor + (1 << log2p);
-      pa.cta_count = pa.start + (1 << log2p) + 1;
-      pa.log2p = log2p;
-      pa.table_slots = part_slots;
-      for (int k = 0; k < K; ++k) {
-        st = count_partitioned(c, b, args, items, s, k, per_item, pa);
-        if (st != SK_OK) return st;
-      }
-      continue;
+      d_rows = static_cast<unsigned int *>(r);
+      const cudaError_t e = cudaMemsetAsync(d_rows, 0, static_cast<size_t>(rows) * 4, ctx->stream);
+      if (e != cudaSuccess) return cuda_fail(ctx, e, "sketch counting");
+      la.overflow = d_rows;
+      any = true;
     }
-    const uint64_t want = next_pow2(static_cast<uint64_t>(windows) * 2);
-    const uint64_t passes = std::max<uint64_t>(1, (want * sizeof(TableSlot) + kTableBudget - 1) / kTableBudget);
-    const uint64_t slots = std::max<uint64_t>(1024, next_pow2((want + passes - 1) / passes));
-    void *tk = nullptr;
-    sk_status st = scratch(ctx, kSlotSketchTable, slots * sizeof(TableSlot) + 16, &tk);
+    la.low = static_cast<uint64_t>(static_cast<double>(c.binsize) * f);
+    low[s - b.s0] = 1;
+    return run_low(c, args, items, p, K, la);
+  };
+  // host bases of more than one chunk of samples go up on the copy stream, the
+  // next chunk while this one is counted
+  const std::vector<Batch> parts = c.device_in ? std::vector<Batch>{b} : upload_chunks(c, b);
+  auto copy_part = [&](size_t i) -> sk_status {
+    const int64_t bytes = parts[i].b1 - parts[i].b0;
+    cudaError_t e = cudaSuccess;
+    if (bytes > 0)
+      e = cudaMemcpyAsync(c.d_codes + (parts[i].b0 - b.b0), c.bases + parts[i].b0,
+                          static_cast<size_t>(bytes), cudaMemcpyHostToDevice, ctx->copy_stream);
+    if (e == cudaSuccess) e = cudaEventRecord(ctx->ev_ready[i & 1], ctx->copy_stream);
+    return e == cudaSuccess ? SK_OK : cuda_fail(ctx, e, "sketch upload");
+  };
+  sk_status st = SK_OK;
+  const bool chunked = !c.device_in && parts.size() > 1;
+  if (!c.device_in && !chunked)
+    st = upload(ctx, c.d_codes, c.bases + b.b0, static_cast<size_t>(b.b1 - b.b0));
+  if (chunked) {
+    st = ensure_copy_stream(ctx);
     if (st != SK_OK) return st;
-    args.table = static_cast<TableSlot *>(tk);
-    args.max_key_count = reinterpret_cast<unsigned int *>(static_cast<char *>(tk) + slots * sizeof(TableSlot));
-    args.table_mask = slots - 1;
-    args.min_count = static_cast<unsigned int>(c.min_count);
-    for (int k = 0; k < K; ++k) {
-      items.clear();
-      make_items(c, b, s, s + 1, k, items, kCountItemWindows);
-      if (items.empty()) continue;
-      void *p = nullptr;
-      st = scratch(ctx, kSlotSketchItems, items.size() * sizeof(SketchItem), &p);
-      if (st == SK_OK) st = upload(ctx, p, items.data(), items.size() * sizeof(SketchItem));
-      if (st != SK_OK) return st;
-      args.items = static_cast<SketchItem *>(p);
-      for (uint64_t pass = 0; pass < passes; ++pass) {
-        args.bin_lo = static_cast<uint32_t>(c.nbins * pass / passes);
-        args.bin_hi = static_cast<uint32_t>(c.nbins * (pass + 1) / passes);
-        table_clear_kernel<<<static_cast<unsigned>(std::min<uint64_t>(4096, (slots + 255) / 256)), 256, 0,
-                             ctx->stream>>>(args.table, slots, args.max_key_count);
-        cudaError_t e = cudaGetLastError();
-        if (e == cudaSuccess) {
-          auto kern = c.codon_phased ? (c.use_rc ? count_kernel<true, true> : count_kernel<false, true>)
-                                     : (c.use_rc ? count_kernel<true, false> : count_kernel<false, false>);
-          kern<<<static_cast<unsigned>(items.size()), kSketchThreads, 0, ctx->stream>>>(args);
-          e = cudaGetLastError();
+    // the copies start after the buffers' set-up on the context's stream
+    cudaError_t e = cudaEventRecord(ctx->ev_free[0], ctx->stream);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(ctx->copy_stream, ctx->ev_free[0], 0);
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "sketch upload");
+    st = copy_part(0);
+  }
+  for (size_t i = 0; st == SK_OK && i < parts.size(); ++i) {
+    if (chunked) {
+      const cudaError_t e = cudaStreamWaitEvent(ctx->stream, ctx->ev_ready[i & 1], 0);
+      if (e != cudaSuccess) return cuda_fail(ctx, e, "sketch upload");
+    }
+    st = make_codes(c, b, parts[i], ctx->stream);
+    for (int64_t s = parts[i].s0; st == SK_OK && s < parts[i].s1; ++s) st = low_sample(s);
+    if (st == SK_OK && chunked && i + 1 < parts.size()) st = copy_part(i + 1);
+  }
+  if (st != SK_OK) return st;
+  std::vector<unsigned int> state;   // overflow and empty bins per row
+  if (any) {
+    empty_bins_kernel<<<static_cast<unsigned>(rows), 256, 0, ctx->stream>>>(
+        args.signs, c.nbins, words, d_rows + 2 * rows, d_rows + rows);
+    state.resize(static_cast<size_t>(2 * rows));
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(state.data(), d_rows, state.size() * 4, cudaMemcpyDeviceToHost, ctx->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "sketch counting");
+    la.empty = d_rows + 2 * rows;
+  }
+
+  // ---- what is left
+  for (int64_t s = b.s0; s < b.s1; ++s) {
+    std::vector<int> full = all;
+    if (low[s - b.s0]) {
+      full.clear();
+      const int64_t windows = sample_windows(c, s);
+      for (int k = 0; k < K; ++k) {
+        const int64_t row = (s - b.s0) * K + k;
+        const unsigned int empty = state[rows + row];
+        if (state[row]) {
+          full.push_back(k);
+        } else if (empty > 0) {
+          // every hash of the empty bins, unless that is most of the sample
+          const double f = static_cast<double>(empty) / c.nbins;
+          items.clear();
+          make_items(c, b, s, s + 1, k, items);
+          const LowPlan p = low_plan(f, kItemWindows, items.size(), 1,
+                                     f * static_cast<double>(windows) + 1024);
+          if (f > 0.25 || p.bytes > budget) {
+            full.push_back(k);
+            continue;
+          }
+          const sk_status st = run_low(c, args, items, p, 1, la);
+          if (st != SK_OK) return st;
         }
-        if (e != cudaSuccess) return cuda_fail(ctx, e, "sketch counting");
       }
     }
+    if (full.empty()) continue;
+    const sk_status st = count_full(c, b, args, items, s, full, budget);
+    if (st != SK_OK) return st;
   }
+  if (!any) return SK_OK;
+  // a second roll's list or table that was too small: that row in full
+  bool second = false;
+  for (int64_t r = 0; r < rows && !second; ++r)
+    second = low[r / K] && !state[r] && state[rows + r] > 0;
+  if (!second) return SK_OK;
+  std::vector<unsigned int> now(static_cast<size_t>(rows));
+  cudaError_t e = cudaMemcpyAsync(now.data(), d_rows, now.size() * 4, cudaMemcpyDeviceToHost, ctx->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+  if (e != cudaSuccess) return cuda_fail(ctx, e, "sketch counting");
+  for (int64_t r = 0; r < rows; ++r)
+    if (now[r] && !state[r]) {
+      const sk_status st = count_full(c, b, args, items, b.s0 + r / K, {static_cast<int>(r % K)}, budget);
+      if (st != SK_OK) return st;
+    }
   return SK_OK;
 }
 
@@ -1194,9 +1580,7 @@ sk_status sketch_batch(SketchCall &c, const Batch &b, std::vector<SketchItem> &i
   args.magic = c.magic;
   args.status = ctx->status_dev;
   if (c.min_count > 0) {
-    if (!c.device_in) st = upload(ctx, c.d_codes, c.bases + b.b0, static_cast<size_t>(bytes));
-    if (st == SK_OK) st = make_codes(c, b, b, ctx->stream);
-    if (st == SK_OK) st = count_batch(c, b, args, items);
+    st = count_batch(c, b, args, items);
   } else {
     st = hash_batch(c, b, args, items);
   }
