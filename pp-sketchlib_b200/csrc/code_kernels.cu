@@ -148,6 +148,7 @@ code_rows_kernel(const CodeTask t) {
         row_tables[b * kTableBytes + v[b]] = static_cast<unsigned char>(row);
       __syncthreads();
       bool mine[kPassBins];
+      uint32_t own[kPassBins];   // a standing row's code
       unsigned int bal[kPassBins];
 #pragma unroll
       for (int b = 0; b < kPassBins; ++b) {
@@ -169,6 +170,7 @@ code_rows_kernel(const CodeTask t) {
         uint16_t *l = list + (q * kPassBins + b) * kCodeGroup;   // word 2q + b / 2, half b % 2
         if (mine[b]) {
           const int rank = before + __popc(bal[b] & ((1u << lane) - 1u));
+          own[b] = rank + 1;
           row_tables[b * kTableBytes + v[b]] = static_cast<unsigned char>(rank + 1);
           l[rank] = static_cast<uint16_t>(v[b]);
         }
@@ -178,7 +180,7 @@ code_rows_kernel(const CodeTask t) {
       uint32_t c = 0;
 #pragma unroll
       for (int b = 0; b < kPassBins; ++b)
-        c |= static_cast<uint32_t>(row_tables[b * kTableBytes + v[b]]) << (8 * b);
+        c |= (mine[b] ? own[b] : static_cast<uint32_t>(row_tables[b * kTableBytes + v[b]])) << (8 * b);
       code[q] = c;
       __syncthreads();
     }
@@ -239,7 +241,7 @@ __device__ __forceinline__ void prefetch_l2(const void *p) {
 // block per lookup, loads one pass ahead of their use (a pass then lasts one
 // memory latency): 6.6 ms; list entries loaded by the lookup warps that also
 // filled the tables, all passes unrolled (instruction fetch): 4.5 to 5.1 ms.
-// As it stands 3.8 ms, 42% of the shared-memory pipe (ncu): 1,100 cycles a pass
+// As it stands 3.6 ms, 42% of the shared-memory pipe (ncu): 1,050 cycles a pass
 // where the lookups of the 11 warps that have columns on average need 290, the
 // rest of it waits between barriers and the transposes and stores at the end of
 // an item.
@@ -364,10 +366,10 @@ __global__ void __launch_bounds__(kColThreads, 1) code_columns_kernel(const Code
   };
   bool active;
   const uint4 *val = values_of(chunk, kb, active);
-  uint4 w[2] = {make_uint4(0u, 0u, 0u, 0u), make_uint4(0u, 0u, 0u, 0u)};   // value words j, j + 1
+  uint4 w[4] = {};   // value words j .. j + 3
   if (active) {
-    w[0] = val[0];
-    w[1] = val[ld4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) w[j] = val[j * ld4];
   }
   __syncthreads();
   while (true) {
@@ -376,7 +378,10 @@ __global__ void __launch_bounds__(kColThreads, 1) code_columns_kernel(const Code
     const int4 next = t.chunks[more ? next_ci : ci];
     bool next_active;
     const uint4 *next_val = values_of(next, more ? next_kb : kb, next_active);
-    if (more && next_active && lane % 8 == 0) {   // one lane per 128-byte line
+    // where few row blocks share the columns, nobody else has brought the next
+    // item's lines to L2 (300 queries: 4.1 ms without, 3.4 with; an all-vs-all of
+    // 4,096 3.6 and 3.7); one lane per 128-byte line
+    if (more && next_active && t.n_rb <= 8 && lane % 8 == 0) {
 #pragma unroll
       for (int j = 0; j < 16; ++j) prefetch_l2(next_val + j * ld4);
     }
@@ -389,11 +394,11 @@ __global__ void __launch_bounds__(kColThreads, 1) code_columns_kernel(const Code
     uint32_t code[2][kColSamples][8];
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
-      const uint4 v = w[j & 1];
-      if (j < 14) {
-        if (active) w[j & 1] = val[(j + 2) * ld4];
+      const uint4 v = w[j & 3];
+      if (j < 12) {
+        if (active) w[j & 3] = val[(j + 4) * ld4];
       } else if (more && next_active) {
-        w[j & 1] = next_val[(j - 14) * ld4];
+        w[j & 3] = next_val[(j - 12) * ld4];
       }
       if (active) {
         const unsigned char *tab = tables + (j & 1) * 2 * kPairTableBytes;
