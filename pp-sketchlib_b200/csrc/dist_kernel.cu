@@ -415,7 +415,7 @@ __global__ void __launch_bounds__(TileShape<QT, RT, TQ, TR, STAGES, CODED>::kBlo
         const int64_t gi = gi0 + q / TR;
         const int64_t gj = gj0 + q % TR;
         if (pair_valid(jp, gi, gj))
-          finish_pair_any<WIDE>(jp, gi, gj, my_counts + q, static_cast<int>(slot_k_stride));
+          finish_pair_any<WIDE, CODED>(jp, gi, gj, my_counts + q, static_cast<int>(slot_k_stride));
       }
     }
   }

@@ -214,9 +214,10 @@ __device__ __forceinline__ float corrected_jaccard(uint32_t count, double union_
 //   xm = sum x / n, ym = sum y / n,
 //   slope = sum (x - xm) y / sum (x - xm)^2, intercept = ym - slope xm,
 // without fused multiply-adds, in the same operation order as the oracle.
-template <int KMAX, bool CHUNKED>
+// count(k) is the pair's intersection count at k.
+template <int KMAX, class Count>
 __device__ __forceinline__ float2 fit_core_acc(const float (&jf)[KMAX], const JobParams &p,
-                                               const uint16_t *counts, int stride) {
+                                               Count count) {
   int first = -1, last = -1;
 #pragma unroll
   for (int k = 0; k < k_bound<KMAX>(p); ++k) {
@@ -244,8 +245,7 @@ __device__ __forceinline__ float2 fit_core_acc(const float (&jf)[KMAX], const Jo
 #pragma unroll
   for (int k = 0; k < k_bound<KMAX>(p); ++k) {
     if (k >= first && k <= last) {
-      const double y = p.ltab ? p.ltab[pair_count<CHUNKED>(p, counts, stride, k)]
-                              : log(static_cast<double>(jf[k]));
+      const double y = p.ltab ? p.ltab[count(k)] : log(static_cast<double>(jf[k]));
       const double dx = __dsub_rn(static_cast<double>(p.kmers[k]), xm);
       sy = __dadd_rn(sy, y);
       sxx = __dadd_rn(sxx, __dmul_rn(dx, dx));
@@ -327,8 +327,12 @@ __device__ __forceinline__ int64_t pair_row(const JobParams &p, int64_t gi, int6
 }
 
 // Finishes one pair from its K intersection counts (counts[k * stride]) and
-// writes its long-form row.
-template <int KMAX, bool CHUNKED>
+// writes its long-form row.  KEEP reads every count before the first is used and
+// keeps them for the fit, for counts parked in L2: an all-vs-all of 4,096 coded
+// samples takes 9.98 ms so, 10.41 reading each count where it is used.  The
+// kernel of the split tiles has its counts in shared memory, where the
+// registers cost it warps (86 to 113 us).
+template <int KMAX, bool CHUNKED, bool KEEP>
 __device__ __forceinline__ void finish_pair(const JobParams &p, int64_t gi, int64_t gj,
                                             const uint16_t *counts, int stride) {
   const int64_t row = pair_row(p, gi, gj);
@@ -345,12 +349,22 @@ __device__ __forceinline__ void finish_pair(const JobParams &p, int64_t gi, int6
     else static_cast<float *>(p.out)[row] = p.out_col == 0 ? ca.x : ca.y;
     return;
   }
+  uint32_t kept[KEEP ? KMAX : 1];
+  if constexpr (KEEP) {
+#pragma unroll
+    for (int k = 0; k < k_bound<KMAX>(p); ++k)
+      kept[k] = k < K ? pair_count<CHUNKED>(p, counts, stride, k) : 0u;
+  }
+  const auto count = [&](int k) -> uint32_t {
+    if constexpr (KEEP) return kept[k];
+    else return pair_count<CHUNKED>(p, counts, stride, k);
+  };
   float jf[KMAX];
 #pragma unroll
   for (int k = 0; k < k_bound<KMAX>(p); ++k) {
     jf[k] = 0.0f;
     if (k < K) {
-      const uint32_t c = pair_count<CHUNKED>(p, counts, stride, k);
+      const uint32_t c = count(k);
       jf[k] = p.jtab ? p.jtab[c] : corrected_jaccard(c, p.union_bits, random_match(p, k, gi, gj));
     }
   }
@@ -369,7 +383,7 @@ __device__ __forceinline__ void finish_pair(const JobParams &p, int64_t gi, int6
     static_cast<float *>(p.out)[row] = v;
     return;
   }
-  const float2 ca = fit_core_acc<KMAX, CHUNKED>(jf, p, counts, stride);
+  const float2 ca = fit_core_acc<KMAX>(jf, p, count);
   if (p.out_mode == kOutCoreAcc) {
     static_cast<float2 *>(p.out)[row] = ca;
   } else {
@@ -382,17 +396,17 @@ __device__ __forceinline__ void finish_pair(const JobParams &p, int64_t gi, int6
 // instance finishes up to kNarrowKmers k-mer lengths with unrolled arrays;
 // the wide one finishes wider k sets, and sketches counted in chunks, with
 // loops over arrays in local memory.
-template <bool WIDE>
+template <bool WIDE, bool KEEP = false>
 __device__ __forceinline__ void finish_pair_any(const JobParams &p, int64_t gi, int64_t gj,
                                                 const uint16_t *counts, int stride) {
   if constexpr (WIDE) {
-    if (p.nchunk == 1 && p.n_kmers <= 8) finish_pair<8, false>(p, gi, gj, counts, stride);
-    else if (p.nchunk == 1 && p.n_kmers <= 16) finish_pair<16, false>(p, gi, gj, counts, stride);
-    else finish_pair<kMaxKmers, true>(p, gi, gj, counts, stride);
+    if (p.nchunk == 1 && p.n_kmers <= 8) finish_pair<8, false, KEEP>(p, gi, gj, counts, stride);
+    else if (p.nchunk == 1 && p.n_kmers <= 16) finish_pair<16, false, KEEP>(p, gi, gj, counts, stride);
+    else finish_pair<kMaxKmers, true, false>(p, gi, gj, counts, stride);
   } else {
-    if (p.n_kmers <= 8) finish_pair<8, false>(p, gi, gj, counts, stride);
-    else if (p.n_kmers <= 16) finish_pair<16, false>(p, gi, gj, counts, stride);
-    else finish_pair<kNarrowKmers, false>(p, gi, gj, counts, stride);
+    if (p.n_kmers <= 8) finish_pair<8, false, KEEP>(p, gi, gj, counts, stride);
+    else if (p.n_kmers <= 16) finish_pair<16, false, KEEP>(p, gi, gj, counts, stride);
+    else finish_pair<kNarrowKmers, false, KEEP>(p, gi, gj, counts, stride);
   }
 }
 
