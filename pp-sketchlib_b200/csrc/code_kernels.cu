@@ -6,8 +6,8 @@
 // nothing, whatever it is.  So each bin of a block of 128 rows gets a
 // dictionary of its distinct values (codes 1 .. D, D <= 128), rows and columns
 // are rewritten as codes (0: not in the dictionary), and the distance kernel
-// compares ceil(log2(D + 1)) <= 8 bit planes instead of 14 (10.4 ms instead of
-// 18.9 at 4,096 samples, K = 8, 156 words; encoding takes 5.0).  Equality of
+// compares ceil(log2(D + 1)) <= 8 bit planes instead of 14 (10.0 ms instead of
+// 18.9 at 4,096 samples, K = 8, 156 words; encoding takes 4.1).  Equality of
 // codes is equality of values, so the counts are the same integers.  D depends on
 // the data (about 60 .. 80 of 128 rows on random trees: 7 planes; 40 .. 60 in
 // clades: 6), its bound does not.
@@ -38,11 +38,13 @@ constexpr int kTableBytes = 1 << kBbits;   // one byte per bin value
 constexpr int kPassBins = 4;               // bins per pass of the row encoder: 8 passes per block
 constexpr int kRowThreads = kCodeGroup;    // one row per thread
 constexpr int kLookupThreads = kCodeChunkGroups * 32;
-constexpr int kColThreads = kLookupThreads + 128;   // and four table warps: 512 x 112 + 128 x 32 registers
+constexpr int kTableWarps = 4;             // (bin, row block) of a pass each
+constexpr int kColThreads = kLookupThreads + 32 * kTableWarps;   // and four table warps: 512 x 112 + 128 x 32 registers
 constexpr int kColSamples = 4;             // columns per thread
 constexpr int kPairTableBytes = 2 * kTableBytes + 16;   // 2-byte entries, one spare
 // two sets of two tables, two buffers of two dictionary lists
-constexpr int kColTableBytes = 4 * kPairTableBytes + 2 * 2 * kCodeListWords * 2;
+constexpr int kTableSets = 3;              // passes the table warps may be ahead
+constexpr int kColTableBytes = 2 * kTableSets * kPairTableBytes + 2 * 2 * kCodeListWords * 2;
 constexpr uint64_t kListWaitNs = 2000000000ull;   // 2 s bounded wait
 constexpr int kValueThreads = 256;
 
@@ -117,7 +119,7 @@ code_rows_kernel(const CodeTask t) {
   extern __shared__ unsigned char row_tables[];   // [kPassBins][kTableBytes]
   __shared__ int warp_count[kRowThreads / 32][kPassBins];
   __shared__ int s_max;
-  if (cancelled(t.status)) return;
+  if (__syncthreads_or(cancelled(t.status))) return;   // all of the CTA or none
   const int row = threadIdx.x, warp = row >> 5, lane = row & 31;
   const int64_t items = static_cast<int64_t>(t.kb) * t.n_rb;
   for (int64_t item = blockIdx.x; item < items; item += gridDim.x) {
@@ -231,32 +233,38 @@ __device__ __forceinline__ void prefetch_l2(const void *p) {
 // kCodeChunkGroups column groups) at a time.  16 warps look columns up, four
 // consecutive columns per thread: a pass takes one value word (two bins) of
 // each, from tables indexed by the 14-bit value whose 16-bit entries hold the
-// codes of both row blocks.  Four more warps clear and fill the next pass's
-// tables meanwhile, one (bin, row block) each from the dictionary lists, which
-// come by bulk copy an item ahead; one barrier per pass, 16 passes.  A lookup's
-// 32 lanes fall on random banks (3.2 cycles of the shared-memory pipe per
-// warp), the bound of a full range.
+// codes of both row blocks.  Four more warps clear and fill the tables of the
+// passes ahead, one (bin, row block) each from the dictionary lists, which come
+// by bulk copy an item ahead.  Three sets of tables, each with an mbarrier for
+// "filled" and one for "read": no warp waits for the slowest of a pass, and one
+// that transposes and stores the codes of an item does so while others look up
+// the next.  A lookup's 32 lanes fall on random banks (3.2 cycles of the
+// shared-memory pipe per warp), the bound of a full range.
 //
 // What held earlier forms back, at 4,096 samples (K = 8, 156 words): one row
 // block per lookup, loads one pass ahead of their use (a pass then lasts one
 // memory latency): 6.6 ms; list entries loaded by the lookup warps that also
-// filled the tables, all passes unrolled (instruction fetch): 4.5 to 5.1 ms.
-// As it stands 3.6 ms, 42% of the shared-memory pipe (ncu): 1,050 cycles a pass
-// where the lookups of the 11 warps that have columns on average need 290, the
-// rest of it waits between barriers and the transposes and stores at the end of
-// an item.
+// filled the tables, all passes unrolled (instruction fetch): 4.5 to 5.1 ms; two
+// sets of tables and a barrier of the CTA per pass: 3.59 ms (8,000 samples 14.6
+// ms, 300 queries against 20,011 3.31).  As it stands 2.92 ms (10.2, 2.63), about
+// half of the shared-memory pipe's time.
 __global__ void __launch_bounds__(kColThreads, 1) code_columns_kernel(const CodeTask t) {
-  extern __shared__ __align__(128) unsigned char tables[];   // [2 sets][2 bins] tables
+  extern __shared__ __align__(128) unsigned char tables[];   // [kTableSets][2 bins] tables
   // dictionary lists of the current and the next item: [2][2 row blocks]
-  uint16_t *lists = reinterpret_cast<uint16_t *>(tables + 4 * kPairTableBytes);
+  uint16_t *lists = reinterpret_cast<uint16_t *>(tables + 2 * kTableSets * kPairTableBytes);
   __shared__ __align__(8) uint64_t list_bar[2];
-  if (cancelled(t.status)) return;
+  __shared__ __align__(8) uint64_t filled[kTableSets], read[kTableSets];
+  if (__syncthreads_or(cancelled(t.status))) return;   // all of the CTA or none
   const int tid = threadIdx.x, lane = tid & 31;
-  for (int i = tid; i < 4 * kPairTableBytes / 16; i += kColThreads)
+  for (int i = tid; i < 2 * kTableSets * kPairTableBytes / 16; i += kColThreads)
     reinterpret_cast<uint4 *>(tables)[i] = make_uint4(0u, 0u, 0u, 0u);
   if (tid == 0) {
     mbar_init(&list_bar[0], 1);
     mbar_init(&list_bar[1], 1);
+    for (int i = 0; i < kTableSets; ++i) {
+      mbar_init(&filled[i], kTableWarps);
+      mbar_init(&read[i], kLookupThreads / 32);
+    }
     fence_mbar_init();
   }
   // the work items, (kb, chunk) in steps of the grid; a chunk names the first
@@ -287,9 +295,12 @@ __global__ void __launch_bounds__(kColThreads, 1) code_columns_kernel(const Code
                  t.lists + (static_cast<int64_t>(c.x + r) * t.kb + k) * kCodeListWords,
                  kCodeListWords * 2, &list_bar[b]);
     };
-    // a list that never lands is recorded; its stale entries are still in range
-    auto wait = [&](int b, uint32_t parity) {
-      if (!mbar_wait_bounded(&list_bar[b], parity, kListWaitNs)) {
+    // a list that never lands, or a set never given back, is recorded, once;
+    // what is there instead is still in range
+    bool waits = true;
+    auto wait = [&](uint64_t *bar, uint32_t parity) {
+      if (waits && !mbar_wait_bounded(bar, parity, kListWaitNs)) {
+        waits = false;
         atomicOr(&t.status->error, 1u);
         t.status->where = 3;
       }
@@ -312,45 +323,44 @@ __global__ void __launch_bounds__(kColThreads, 1) code_columns_kernel(const Code
     };
     const int code = 4 * lane + 1;
     int b = 0;                    // list buffer of the current item
-    uint32_t phase[2] = {0, 0};
+    uint32_t list_phase[2] = {0, 0};
+    int set = 0;
+    uint32_t phase = 1;           // a new set's first wait passes
+    uint2 held[kTableSets];       // the sets' entries, the set to fill next first
+#pragma unroll
+    for (int i = 0; i < kTableSets; ++i) held[i] = make_uint2(~0u, ~0u);
     if (role == 0 && lane == 0) fetch(chunk, kb, 0);
-    wait(0, 0);
-    phase[0] = 1;
-    uint2 even = entries(chunk, 0, 0), odd = make_uint2(~0u, ~0u);   // set in tables 0 / 1
-    put(0, even, code);
-    __syncthreads();
     while (true) {
       int next_kb = kb, next_ci = ci;
       const bool more = advance(next_kb, next_ci);
       const int4 next = t.chunks[more ? next_ci : ci];
-      // the other buffer was last read two barriers ago
+      // every table warp is done with the other buffer
+      asm volatile("bar.sync 1, %0;" ::"n"(kTableWarps * 32) : "memory");
       if (more && role == 0 && lane == 0) fetch(next, next_kb, b ^ 1);
+      wait(&list_bar[b], list_phase[b]);
+      list_phase[b] ^= 1u;
 #pragma unroll 1
-      for (int pass = 0; pass < 16; pass += 2) {
-        put(1, odd, -1);
-        odd = entries(chunk, b, pass + 1);
+      for (int pass = 0; pass < 16; ++pass) {
+        const uint2 vals = entries(chunk, b, pass);
+        wait(&read[set], phase);
+        put(set, held[0], -1);
         __syncwarp();
-        put(1, odd, code);
-        __syncthreads();   // end of an even pass
-        put(0, even, -1);
-        if (pass < 14) {
-          even = entries(chunk, b, pass + 2);
-        } else if (more) {
-          wait(b ^ 1, phase[b ^ 1]);
-          even = entries(next, b ^ 1, 0);
-        } else {
-          even = make_uint2(~0u, ~0u);
+        put(set, vals, code);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&filled[set]);
+#pragma unroll
+        for (int i = 0; i + 1 < kTableSets; ++i) held[i] = held[i + 1];
+        held[kTableSets - 1] = vals;
+        if (++set == kTableSets) {
+          set = 0;
+          phase ^= 1u;
         }
-        __syncwarp();
-        put(0, even, code);
-        __syncthreads();   // end of an odd pass
       }
       if (!more) return;
       kb = next_kb;
       ci = next_ci;
       chunk = next;
       b ^= 1;
-      phase[b] ^= 1u;
     }
   }
 
@@ -371,7 +381,9 @@ __global__ void __launch_bounds__(kColThreads, 1) code_columns_kernel(const Code
 #pragma unroll
     for (int j = 0; j < 4; ++j) w[j] = val[j * ld4];
   }
-  __syncthreads();
+  int set = 0;
+  uint32_t phase = 0;
+  bool waits = true;
   while (true) {
     int next_kb = kb, next_ci = ci;
     const bool more = advance(next_kb, next_ci);
@@ -400,8 +412,13 @@ __global__ void __launch_bounds__(kColThreads, 1) code_columns_kernel(const Code
       } else if (more && next_active) {
         w[j & 3] = next_val[(j - 12) * ld4];
       }
+      if (waits && !mbar_wait_bounded(&filled[set], phase, kListWaitNs)) {
+        waits = false;
+        atomicOr(&t.status->error, 1u);
+        t.status->where = 4;
+      }
       if (active) {
-        const unsigned char *tab = tables + (j & 1) * 2 * kPairTableBytes;
+        const unsigned char *tab = tables + set * 2 * kPairTableBytes;
         const uint32_t vv[kColSamples] = {v.x, v.y, v.z, v.w};   // entry offsets: 2 x value
 #pragma unroll
         for (int i = 0; i < kColSamples; ++i) {
@@ -419,7 +436,12 @@ __global__ void __launch_bounds__(kColThreads, 1) code_columns_kernel(const Code
           }
         }
       }
-      __syncthreads();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&read[set]);
+      if (++set == kTableSets) {
+        set = 0;
+        phase ^= 1u;
+      }
     }
     if (active) {
       const int64_t s = static_cast<int64_t>(chunk.y) * kCodeGroup + tid * kColSamples;

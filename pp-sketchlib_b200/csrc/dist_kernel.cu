@@ -79,10 +79,6 @@ struct TileShape {
   static_assert(!CODED || (QT == kCodeGroup && RT == kCodeGroup), "a coded tile is one group by one");
 };
 
-__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
-}
-
 // Adds one 32-bin block's matches of a thread's TQ x TR pairs to its counts:
 // the block's PLANES bit planes of the rows at qb and the columns at rb, LD
 // words from one plane to the next.  Counts of columns 2c and 2c + 1 share a
