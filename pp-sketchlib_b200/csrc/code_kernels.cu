@@ -225,10 +225,6 @@ code_values_kernel(const uint32_t *__restrict__ packed, int32_t kb, int32_t ng, 
   }
 }
 
-__device__ __forceinline__ void prefetch_l2(const void *p) {
-  asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
-}
-
 // One CTA per (kb, two neighbouring row blocks, range of up to
 // kCodeChunkGroups column groups) at a time.  16 warps look columns up, four
 // consecutive columns per thread: a pass takes one value word (two bins) of
@@ -246,8 +242,10 @@ __device__ __forceinline__ void prefetch_l2(const void *p) {
 // memory latency): 6.6 ms; list entries loaded by the lookup warps that also
 // filled the tables, all passes unrolled (instruction fetch): 4.5 to 5.1 ms; two
 // sets of tables and a barrier of the CTA per pass: 3.59 ms (8,000 samples 14.6
-// ms, 300 queries against 20,011 3.31).  As it stands 2.92 ms (10.2, 2.63), about
-// half of the shared-memory pipe's time.
+// ms, 300 queries against 20,011 3.31).  As it stands 2.92 ms (10.2, 2.53), about
+// half of the shared-memory pipe's time.  The next item's lines prefetched to L2,
+// which helped few row blocks at a barrier per pass, costs since (2.63 for 2.53,
+// 3.00 for 2.91); loads 8 words ahead instead of 4 spill (3.60).
 __global__ void __launch_bounds__(kColThreads, 1) code_columns_kernel(const CodeTask t) {
   extern __shared__ __align__(128) unsigned char tables[];   // [kTableSets][2 bins] tables
   // dictionary lists of the current and the next item: [2][2 row blocks]
@@ -390,13 +388,6 @@ __global__ void __launch_bounds__(kColThreads, 1) code_columns_kernel(const Code
     const int4 next = t.chunks[more ? next_ci : ci];
     bool next_active;
     const uint4 *next_val = values_of(next, more ? next_kb : kb, next_active);
-    // where few row blocks share the columns, nobody else has brought the next
-    // item's lines to L2 (300 queries: 4.1 ms without, 3.4 with; an all-vs-all of
-    // 4,096 3.6 and 3.7); one lane per 128-byte line
-    if (more && next_active && t.n_rb <= 8 && lane % 8 == 0) {
-#pragma unroll
-      for (int j = 0; j < 16; ++j) prefetch_l2(next_val + j * ld4);
-    }
     // planes of the pair of blocks kb belongs to (the count per row block is even)
     uint32_t pair_planes[2];
 #pragma unroll
