@@ -8,6 +8,9 @@
 
 #include <cfloat>
 #include <cstdint>
+#include <map>
+#include <mutex>
+#include <utility>
 
 #include "sk_common.h"
 #include "sk_device.cuh"
@@ -529,6 +532,21 @@ cudaError_t launch_unpack(const uint32_t *packed, int64_t n, int32_t n_kmers, in
   return cudaGetLastError();
 }
 
+cudaError_t raise_smem_limit(const void *kernel, size_t bytes) {
+  static std::mutex mu;
+  static std::map<std::pair<int, const void *>, size_t> limits;
+  int device = 0;
+  cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return e;
+  std::lock_guard<std::mutex> lock(mu);
+  size_t &limit = limits[{device, kernel}];
+  if (bytes <= limit) return cudaSuccess;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           static_cast<int>(bytes));
+  if (e == cudaSuccess) limit = bytes;
+  return e;
+}
+
 cudaError_t launch_synth(const int32_t *parent, const uint32_t *thresh, int64_t n,
                          int32_t n_kmers, int32_t s64, uint64_t seed, uint64_t *words,
                          cudaStream_t stream) {
@@ -549,11 +567,8 @@ cudaError_t launch_knn_lists(const float *vals, int64_t n_rows, int64_t n_cols, 
   int threads = 256;
   while (threads > 32 && (threads * knn * 8 > 100 * 1024 || n_cols < 8 * threads)) threads /= 2;
   const int smem = threads * knn * 8;
-  if (smem > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(knn_lists_kernel<SELF>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-  }
+  const cudaError_t e = raise_smem_limit(knn_lists_kernel<SELF>, smem);
+  if (e != cudaSuccess) return e;
   const int blocks = static_cast<int>(n_rows < 148 * 64 ? n_rows : 148 * 64);
   knn_lists_kernel<SELF><<<blocks > 0 ? blocks : 1, threads, smem, stream>>>(
       vals, n_rows, n_cols, knn, diag0, jaccard, j_out, d_out);
@@ -574,11 +589,8 @@ cudaError_t launch_knn_rows(const float *vals, int64_t n_rows, int64_t n_cols, i
   if (knn > n_cols) return cudaErrorInvalidValue;
   if (knn > kKnnListMax) {
     const int smem = knn <= kKnnSmemList ? knn * 8 : 0;
-    if (smem > 48 * 1024) {
-      const cudaError_t attr = cudaFuncSetAttribute(
-          knn_select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kKnnSmemList * 8);
-      if (attr != cudaSuccess) return attr;
-    }
+    const cudaError_t attr = raise_smem_limit(knn_select_kernel, smem);
+    if (attr != cudaSuccess) return attr;
     const int blocks = static_cast<int>(n_rows < 148 * 4 ? n_rows : 148 * 4);
     knn_select_kernel<<<blocks > 0 ? blocks : 1, kKnnSelectThreads, smem, stream>>>(
         vals, n_rows, n_cols, knn, diag0, jaccard, j_out, d_out);

@@ -469,16 +469,8 @@ __global__ void __launch_bounds__(kColThreads, 1) code_columns_kernel(const Code
 }  // namespace
 
 cudaError_t prepare_code_kernels() {
-  static cudaError_t status = [] {
-    cudaError_t e = cudaFuncSetAttribute(code_rows_kernel,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         kPassBins * kTableBytes);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(code_columns_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               kColTableBytes);
-    return e;
-  }();
-  return status;
+  const cudaError_t e = raise_smem_limit(code_rows_kernel, kPassBins * kTableBytes);
+  return e == cudaSuccess ? raise_smem_limit(code_columns_kernel, kColTableBytes) : e;
 }
 
 cudaError_t launch_code_values(const uint32_t *packed, int32_t kb, int32_t ng, int32_t g0,

@@ -34,6 +34,14 @@ inline size_t count_slot_bytes(const TileConfig &cfg, int k_slots) {
   return static_cast<size_t>(k_slots) * cfg.tile_rows * cfg.tile_cols * 2;
 }
 
+// aux_kernels.cu: lets `kernel` be launched with `bytes` of dynamic shared
+// memory.  The limit belongs to the process, not to a context, so it is only
+// ever raised: a launch of another thread keeps the size it asked for.
+cudaError_t raise_smem_limit(const void *kernel, size_t bytes);
+template <class... A>
+cudaError_t raise_smem_limit(void (*kernel)(A...), size_t bytes) {
+  return raise_smem_limit(reinterpret_cast<const void *>(kernel), bytes);
+}
 
 // code_kernels.cu: bin values of granules g0 .. g0 + n_g - 1 of a packed array
 // of ng granules; the row and column encoders of one task.

@@ -1102,7 +1102,7 @@ sk_status launch_hash(sk_ctx *ctx, const SketchCall &c, SketchArgs args, const S
   if (shared) {
     auto kern = c.codon_phased ? (c.use_rc ? sketch_kernel<true, true, true> : sketch_kernel<true, false, true>)
                                : (c.use_rc ? sketch_kernel<true, true, false> : sketch_kernel<true, false, false>);
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    e = raise_smem_limit(kern, smem);
     if (e == cudaSuccess) kern<<<grid, kSketchThreads, smem, stream>>>(args);
   } else {
     auto kern = c.codon_phased ? (c.use_rc ? sketch_kernel<false, true, true> : sketch_kernel<false, false, true>)
@@ -1167,13 +1167,9 @@ sk_status count_partitioned(SketchCall &c, const Batch &b, SketchArgs &args, std
                              : (c.use_rc ? part_kernel<true, false, false> : part_kernel<false, false, false>);
   auto scat = c.codon_phased ? (c.use_rc ? part_kernel<true, true, true> : part_kernel<false, true, true>)
                              : (c.use_rc ? part_kernel<true, false, true> : part_kernel<false, false, true>);
-  cudaError_t e = cudaFuncSetAttribute(hist, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       static_cast<int>(part_smem));
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(scat, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(part_smem));
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(part_count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(table_smem));
+  cudaError_t e = raise_smem_limit(hist, part_smem);
+  if (e == cudaSuccess) e = raise_smem_limit(scat, part_smem);
+  if (e == cudaSuccess) e = raise_smem_limit(part_count_kernel, table_smem);
   if (e == cudaSuccess) e = cudaMemsetAsync(pa.count, 0, part_smem, ctx->stream);
   const unsigned grid = static_cast<unsigned>(items.size());
   if (e == cudaSuccess) {
@@ -1327,7 +1323,7 @@ sk_status run_low(SketchCall &c, SketchArgs &args, const std::vector<SketchItem>
                : (c.codon_phased ? (c.use_rc ? low_roll_kernel<true, true, false> : low_roll_kernel<false, true, false>)
                                  : (c.use_rc ? low_roll_kernel<true, false, false> : low_roll_kernel<false, false, false>));
   constexpr int smem = LowKeep<false>::kColumn * kSketchThreads * 8;
-  const cudaError_t attr = cudaFuncSetAttribute(roll, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  const cudaError_t attr = raise_smem_limit(roll, smem);
   if (attr != cudaSuccess) return cuda_fail(ctx, attr, "sketch counting");
   roll<<<grid, kSketchThreads, smem, ctx->stream>>>(args, la);
   low_count_kernel<<<grid * kLowCountSplit, kLowCountThreads, 0, ctx->stream>>>(args, la);
