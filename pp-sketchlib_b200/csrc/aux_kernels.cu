@@ -174,20 +174,32 @@ __device__ __forceinline__ float image_key(uint32_t u) {
   return __uint_as_float(u ^ ((u >> 31) ? 0x80000000u : 0xFFFFFFFFu));
 }
 
-// kNN lists of at most kKnnListMax entries, one CTA per row: SELF, row i of a
-// condensed single column (its own column is +inf, src/api.cpp:365), else a row
-// of a dense (n_rows, n_cols) column; diag0 >= 0: row r is sample diag0 + r of
-// the column set, whose own column counts as +inf.  Keys are the distances, or
-// 1 - J for Jaccard (src/api.cpp:370-371), as 64-bit words (key image, column):
-// unique, and in the order of (key, column).  Each thread keeps the kNN best of
-// every blockDim-th column, sorted, in shared memory; then the CTA takes the
-// smallest head of the lists kNN times.
+// Key of column c in a row: SELF, row i of a condensed single column, else a
+// row of a dense (n_rows, n_cols) column.  The row's own column is +inf
+// (src/api.cpp:365); keys are the distances, or 1 - J for Jaccard
+// (src/api.cpp:370-371).
+template <bool SELF>
+__device__ __forceinline__ float knn_key(const float *__restrict__ vals, int64_t row, int64_t c,
+                                         int64_t n_cols, int64_t own, int jaccard) {
+  if (c == own) return INFINITY;
+  const float d = SELF ? vals[c < row ? condensed(c, row, n_cols) : condensed(row, c, n_cols)]
+                       : vals[row * n_cols + c];
+  return jaccard ? 1.0f - d : d;
+}
+
+// kNN lists of at most kKnnListMax entries, one CTA per row (SELF: of the
+// condensed column; else of a dense one, where diag0 >= 0 says that row r is
+// sample diag0 + r of the column set).  Keys become 64-bit words (key image,
+// column): unique, and in the order of (key, column).  Each thread keeps the kNN
+// best of every blockDim-th column, sorted, in shared memory; then the CTA takes
+// the smallest head of the lists kNN times.
 //
 // Bound by the latency of the row's reads and insertions, so a row gets up to
-// 256 threads with four reads in flight each (as few as 32 where the lists fill
-// shared memory): with one thread per row of a block of 32 (self) and one warp
-// per row (dense rows), 10 neighbours of 6,007 samples took 3.1 ms and 5 of one
-// row of 30,011 references 0.51 ms.
+// 256 threads with four reads in flight each: with one thread per row of a block
+// of 32 (self) and one warp per row (dense rows), 10 neighbours of 6,007 samples
+// took 3.1 ms (0.6 now) and 5 of one row of 30,011 references 0.51.  A list costs
+// each of its threads kNN steps per insertion, so this form is for short lists
+// only: see kKnnListMax.
 template <bool SELF>
 __global__ void knn_lists_kernel(const float *__restrict__ vals, int64_t n_rows, int64_t n_cols,
                                  int knn, int64_t diag0, int jaccard,
@@ -199,14 +211,7 @@ __global__ void knn_lists_kernel(const float *__restrict__ vals, int64_t n_rows,
   for (int64_t row = blockIdx.x; row < n_rows; row += gridDim.x) {
     const int64_t own = SELF ? row : (diag0 >= 0 ? diag0 + row : -1);
     auto word = [&](int64_t c) -> unsigned long long {
-      float d;
-      if (c == own) {
-        d = INFINITY;
-      } else {
-        d = SELF ? vals[c < row ? condensed(c, row, n_cols) : condensed(row, c, n_cols)]
-                 : vals[row * n_cols + c];
-        if (jaccard) d = 1.0f - d;
-      }
+      const float d = knn_key<SELF>(vals, row, c, n_cols, own, jaccard);
       return (static_cast<unsigned long long>(key_image(d)) << 32) | static_cast<uint32_t>(c);
     };
     unsigned long long *mine = knn_list + tid;
@@ -258,8 +263,8 @@ __global__ void knn_lists_kernel(const float *__restrict__ vals, int64_t n_rows,
   }
 }
 
-// Row kNN for any kNN up to the row length (the kernels above keep kNN lists
-// per thread in shared memory, up to kKnnListMax entries).  One CTA per row, in four steps:
+// Row kNN for any kNN up to the row length, over the same two forms of
+// input.  One CTA per row, in four steps:
 //  1. radix select over the 32-bit order-preserving image of the key (four
 //     8-bit digits, most significant first; a 256-bin shared histogram per
 //     pass over the row) finds the bucket [lo, hi] of keys that holds the
@@ -274,11 +279,10 @@ __global__ void knn_lists_kernel(const float *__restrict__ vals, int64_t n_rows,
 //     output slots (j_out, 8 bytes per entry) when the list is larger than
 //     kKnnSmemList;
 //  4. the words become (column, key) outputs.
-// Keys are the distances (1 - J for Jaccard), the row's own column (diag0 >=
-// 0) +inf, -0 read as +0.
 constexpr int kKnnSelectThreads = 512;
 constexpr int kKnnSmemList = 12288;   // 96 KiB of 64-bit words
 
+template <bool SELF>
 __global__ void __launch_bounds__(kKnnSelectThreads)
 knn_select_kernel(const float *__restrict__ vals, int64_t n_rows, int64_t n_cols, int knn,
                   int64_t diag0, int jaccard, int64_t *__restrict__ j_out,
@@ -290,12 +294,9 @@ knn_select_kernel(const float *__restrict__ vals, int64_t n_rows, int64_t n_cols
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   constexpr int NW = kKnnSelectThreads / 32;
   for (int64_t row = blockIdx.x; row < n_rows; row += gridDim.x) {
-    const float *v = vals + row * n_cols;
-    const int64_t own = diag0 >= 0 ? diag0 + row : -1;
+    const int64_t own = SELF ? row : (diag0 >= 0 ? diag0 + row : -1);
     auto image = [&](int64_t c) -> uint32_t {
-      float d = c == own ? INFINITY : v[c];
-      if (jaccard && c != own) d = 1.0f - d;
-      return key_image(d);
+      return key_image(knn_key<SELF>(vals, row, c, n_cols, own, jaccard));
     };
 
     // 1. the bucket of the kNN-th smallest key
@@ -558,17 +559,27 @@ cudaError_t launch_synth(const int32_t *parent, const uint32_t *thresh, int64_t 
 
 namespace {
 
-// Threads per row: 256 while the lists leave room for two CTAs per SM, fewer
-// for longer lists or rows shorter than the threads' lists, 32 at least.
+template <bool SELF>
+cudaError_t launch_knn_select(const float *vals, int64_t n_rows, int64_t n_cols, int32_t knn,
+                              int64_t diag0, int32_t jaccard, int64_t *j_out, float *d_out,
+                              cudaStream_t stream) {
+  const int smem = knn <= kKnnSmemList ? knn * 8 : 0;
+  const cudaError_t e = raise_smem_limit(knn_select_kernel<SELF>, smem);
+  if (e != cudaSuccess) return e;
+  const int blocks = static_cast<int>(n_rows < 148 * 4 ? n_rows : 148 * 4);
+  knn_select_kernel<SELF><<<blocks > 0 ? blocks : 1, kKnnSelectThreads, smem, stream>>>(
+      vals, n_rows, n_cols, knn, diag0, jaccard, j_out, d_out);
+  return cudaGetLastError();
+}
+
+// Threads per row: 256, fewer for rows shorter than the threads' lists.
 template <bool SELF>
 cudaError_t launch_knn_lists(const float *vals, int64_t n_rows, int64_t n_cols, int32_t knn,
                              int64_t diag0, int32_t jaccard, int64_t *j_out, float *d_out,
                              cudaStream_t stream) {
   int threads = 256;
-  while (threads > 32 && (threads * knn * 8 > 100 * 1024 || n_cols < 8 * threads)) threads /= 2;
+  while (threads > 32 && n_cols < 8 * threads) threads /= 2;
   const int smem = threads * knn * 8;
-  const cudaError_t e = raise_smem_limit(knn_lists_kernel<SELF>, smem);
-  if (e != cudaSuccess) return e;
   const int blocks = static_cast<int>(n_rows < 148 * 64 ? n_rows : 148 * 64);
   knn_lists_kernel<SELF><<<blocks > 0 ? blocks : 1, threads, smem, stream>>>(
       vals, n_rows, n_cols, knn, diag0, jaccard, j_out, d_out);
@@ -579,24 +590,17 @@ cudaError_t launch_knn_lists(const float *vals, int64_t n_rows, int64_t n_cols, 
 
 cudaError_t launch_knn_self(const float *col_vals, int64_t n, int32_t knn, int32_t jaccard,
                             int64_t *j_out, float *d_out, cudaStream_t stream) {
-  if (knn > kKnnListMax || knn > n) return cudaErrorInvalidValue;
-  return launch_knn_lists<true>(col_vals, n, n, knn, -1, jaccard, j_out, d_out, stream);
+  if (knn > n) return cudaErrorInvalidValue;
+  const auto launch = knn <= kKnnListMax ? launch_knn_lists<true> : launch_knn_select<true>;
+  return launch(col_vals, n, n, knn, -1, jaccard, j_out, d_out, stream);
 }
 
 cudaError_t launch_knn_rows(const float *vals, int64_t n_rows, int64_t n_cols, int32_t knn,
                             int64_t diag0, int32_t jaccard, int64_t *j_out, float *d_out,
                             cudaStream_t stream) {
   if (knn > n_cols) return cudaErrorInvalidValue;
-  if (knn > kKnnListMax) {
-    const int smem = knn <= kKnnSmemList ? knn * 8 : 0;
-    const cudaError_t attr = raise_smem_limit(knn_select_kernel, smem);
-    if (attr != cudaSuccess) return attr;
-    const int blocks = static_cast<int>(n_rows < 148 * 4 ? n_rows : 148 * 4);
-    knn_select_kernel<<<blocks > 0 ? blocks : 1, kKnnSelectThreads, smem, stream>>>(
-        vals, n_rows, n_cols, knn, diag0, jaccard, j_out, d_out);
-    return cudaGetLastError();
-  }
-  return launch_knn_lists<false>(vals, n_rows, n_cols, knn, diag0, jaccard, j_out, d_out, stream);
+  const auto launch = knn <= kKnnListMax ? launch_knn_lists<false> : launch_knn_select<false>;
+  return launch(vals, n_rows, n_cols, knn, diag0, jaccard, j_out, d_out, stream);
 }
 
 cudaError_t launch_count_tables(double union_bits, int64_t n, float *jtab, double *ltab,

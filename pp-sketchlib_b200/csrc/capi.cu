@@ -1601,8 +1601,7 @@ sk_status sk_dists_knn(sk_ctx *ctx, const sk_db *db, const sk_random *random, in
   const int out_col = jaccard ? 2 + dist_col : dist_col;
   const size_t budget = dense_budget(ctx);
   cudaError_t e = cudaSuccess;
-  if (static_cast<size_t>(pairs) * 4 > budget || kNN > kKnnListMax) {
-    // longer lists are selected over dense rows: rows in blocks against every column
+  if (static_cast<size_t>(pairs) * 4 > budget) {   // rows in blocks against every column
     st = knn_blocked(ctx, db, db, true, random, kNN, out_col, jaccard, d_j, d_d, budget);
     if (st != SK_OK) return st;
   } else {

@@ -71,10 +71,15 @@ cudaError_t launch_unpack(const uint32_t *packed, int64_t n, int32_t n_kmers, in
 cudaError_t launch_synth(const int32_t *parent, const uint32_t *thresh, int64_t n,
                          int32_t n_kmers, int32_t s64, uint64_t seed, uint64_t *words,
                          cudaStream_t stream);
-// kNN lists of at most kKnnListMax entries are kept per lane in shared memory
-// (the condensed self column and dense rows); longer ones only over dense
-// rows, by radix select and a bitonic sort per row.
-constexpr int kKnnListMax = 800;
+// kNN over a condensed self column, or over dense rows.  Lists of at most
+// kKnnListMax entries are kept per thread in shared memory, longer ones come from
+// a radix select and a bitonic sort per row: the select costs its passes over the
+// row whatever kNN is, the lists grow with kNN.  Lists and select, self calls in
+// ms: 12,007 samples 4.7 and 5.9 with 1 neighbour, 5.5 and 6.1 with 16, 9.8 and
+// 6.8 with 48, 65 and 16 with 200; 6,007 samples 1.3 and 1.6, 1.75 and 1.75, 3.2
+// and 2.0, 19 and 2.9 (264 and 15 with 800).  100 rows of 30,011 references: 0.29
+// and 0.30, 0.32 and 0.30, 0.48 and 0.31, 2.9 and 0.32.
+constexpr int kKnnListMax = 16;
 cudaError_t launch_knn_self(const float *col_vals, int64_t n, int32_t knn, int32_t jaccard,
                             int64_t *j_out, float *d_out, cudaStream_t stream);
 cudaError_t launch_knn_rows(const float *vals, int64_t n_rows, int64_t n_cols, int32_t knn,
