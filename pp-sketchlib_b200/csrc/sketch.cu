@@ -116,9 +116,10 @@ uint64_t srol_n(uint64_t v, unsigned n) {
 struct SketchItem {
   int64_t begin, end;     // window starts, offsets into the code buffer
   int32_t row;            // sample * K + k index (bins row)
-  int32_t k;
-  int32_t tab;            // k index (table row)
+  int16_t k;
+  int16_t tab;            // k index (roll table)
   int32_t per;            // window starts per thread (a multiple of 16, at most kPerThread)
+  int32_t table;          // low count: its table among the launch's
 };
 
 // Rolling table of one k, indexed by (entering base | leaving base << 3):
@@ -505,16 +506,27 @@ count_kernel(SketchArgs a) {
 // near the low end of their bin matter.  The first roll keeps those below
 // `low`, sized for about kLowPerBin windows per bin; as the test depends on the
 // hash alone, a kept hash is kept at every occurrence and its count is exact.
-// They are written to their item's list, then counted in a global table that
-// stays in L2.  A bin that some hash below `low` fills is done: any other
-// candidate is larger.  Bins still empty (27 in a million when 12.8 of the 128
-// windows are distinct k-mers that qualify) get a second roll that keeps every
-// hash of theirs, or, when that is most of the sample, the whole sample is
-// counted by groups (below).
+// They are written to their item's list, then counted in a global table per
+// (sample, k), 33 MB at 9,984 bins.  A bin that some hash below `low` fills is
+// done: any other candidate is larger.  Bins still empty (27 in a million when
+// 12.8 of the 128 windows are distinct k-mers that qualify) get a second roll
+// that keeps every hash of theirs, or, where they are more than a quarter of the
+// bins, the sample is counted by groups (below) at that k.
+//
+// How many bins that leaves depends on the coverage, which nobody knows
+// beforehand.  So a sample's longest k, which errors and read ends leave the
+// fewest hashes, is rolled first; where it leaves more than a quarter of its bins
+// empty, the launch of the other k returns at once (`gate`, read on the device)
+// and the sample is counted by groups at every k.  The second rolls of a batch of
+// samples share a launch: one of 4 M windows fills a ninth of the device.
 //
 // Against counting every hash of a sample by groups (two rolls, 8 bytes
 // written to a random sector per window): 20 Mbases of reads, per k: 430 us
-// before, 127 now (91 the roll, 31 the count, 5 clearing the table).
+// before, 127 now (91 the roll, 31 the count, 5 clearing the table).  Two read
+// sets of 4 M bases (K = 8, host bases), in ms, counted by groups, with all k
+// rolled at once and a second roll per row, and now: 2x coverage and min_count 5
+// (a quarter to a half of the bins empty) 2.53, 4.33 and 2.84; 3x and 5 (2% to 20%
+// empty, 6 M bases) 2.53, 5.54 and 2.30; 2x and 3 (a few bins) 2.05, 2.87 and 1.60.
 struct LowArgs {
   uint64_t low;                   // keep hashes of a bin below its start + low
   const unsigned int *empty;      // [rows][words]: keep the hashes of these bins (null: below low)
@@ -525,8 +537,12 @@ struct LowArgs {
   struct TableSlot *tables;       // [tables][slots]
   unsigned int *max_key;          // [tables] occurrences of the hash equal to kEmptyKey
   uint64_t slots;                 // a power of two
-  int by_k;                       // table of an item: its k index, or 0
+  int n_tables;
+  const unsigned int *gate;       // null, or the empty bins of the sample's first row:
+  unsigned int gate_max;          //   nothing is rolled above gate_max
   unsigned int *overflow;         // [rows] a list or table was too small
+
+  __device__ __forceinline__ bool closed() const { return gate && *gate > gate_max; }
 };
 
 // The roll's emitter.  A thread puts its kept hashes into its own column of a
@@ -589,6 +605,10 @@ low_roll_kernel(SketchArgs a, LowArgs la) {
   }
   if (threadIdx.x == 0) kept = 0;
   __syncthreads();
+  if (la.closed()) {
+    if (threadIdx.x == 0) la.count[blockIdx.x] = 0;
+    return;
+  }
   LowKeep<kBitmap> keep{low_columns + threadIdx.x,
                         la.hashes + static_cast<int64_t>(blockIdx.x) * la.cap, &kept, la.cap,
                         a.binsize, a.magic, la.low,
@@ -618,7 +638,7 @@ __global__ void __launch_bounds__(kLowCountThreads) low_count_kernel(SketchArgs 
   const SketchItem it = a.items[item];
   const unsigned int n = min(la.count[item], la.cap);
   const unsigned long long *in = la.hashes + static_cast<int64_t>(item) * la.cap;
-  const int t = la.by_k ? it.tab : 0;
+  const int t = it.table;
   TableSlot *table = la.tables + static_cast<int64_t>(t) * la.slots;
   unsigned long long *row = a.signs + static_cast<int64_t>(it.row) * a.nbins;
   for (unsigned int i = part * kLowCountThreads + threadIdx.x; i < n;
@@ -656,12 +676,14 @@ __global__ void __launch_bounds__(kLowCountThreads) low_count_kernel(SketchArgs 
   }
 }
 
-__global__ void low_clear_kernel(TableSlot *__restrict__ t, uint64_t n, unsigned int *max_key,
-                                 int n_tables) {
+__global__ void low_clear_kernel(LowArgs la) {
+  if (la.closed()) return;
+  const uint64_t n = static_cast<uint64_t>(la.n_tables) * la.slots;
+  const uint64_t first = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x;
   const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
-  for (uint64_t i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; i < n; i += stride)
-    reinterpret_cast<uint4 *>(t)[i] = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u);
-  if (blockIdx.x == 0 && threadIdx.x < n_tables) max_key[threadIdx.x] = 0;
+  for (uint64_t i = first; i < n; i += stride)
+    reinterpret_cast<uint4 *>(la.tables)[i] = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u);
+  for (uint64_t i = first; i < static_cast<uint64_t>(la.n_tables); i += stride) la.max_key[i] = 0;
 }
 
 // Bitmap and number of a row's empty bins (one CTA per row).
@@ -1055,11 +1077,12 @@ std::vector<Batch> upload_chunks(const SketchCall &c, const Batch &b) {
 
 // Work items of samples [s0, s1) of batch b (code offsets relative to b.b0):
 // window starts of each sample in equal pieces of at most kItemWindows (so
-// the threads of every item get the same share), every k of a piece adjacent
-// (they read the same bases).  Windows end inside their sample, so a sample's
+// the threads of every item get the same share), every k (index) of a piece
+// adjacent (they read the same bases).  Windows end inside their sample, so a sample's
 // items read no other sample's codes that they depend on.
-void make_items(const SketchCall &c, const Batch &b, int64_t s0, int64_t s1, int k_only,
-                std::vector<SketchItem> &items, int64_t max_windows = kItemWindows) {
+void make_items(const SketchCall &c, const Batch &b, int64_t s0, int64_t s1,
+                const std::vector<int> &ks, std::vector<SketchItem> &items,
+                int64_t max_windows = kItemWindows) {
   const int K = static_cast<int>(c.kmers.size());
   for (int64_t s = s0; s < s1; ++s) {
     const int64_t a = c.seq_off[c.sample_seqs[s]] - b.b0, e = c.seq_off[c.sample_seqs[s + 1]] - b.b0;
@@ -1069,8 +1092,7 @@ void make_items(const SketchCall &c, const Batch &b, int64_t s0, int64_t s1, int
         std::max<int64_t>(16, ((piece + kSketchThreads - 1) / kSketchThreads + 15) / 16 * 16));
     const int64_t step = static_cast<int64_t>(per) * kSketchThreads;
     for (int64_t p = a; p < e; p += step)
-      for (int k = 0; k < K; ++k) {
-        if (k_only >= 0 && k != k_only) continue;
+      for (int k : ks) {
         SketchItem it{};
         it.begin = p;
         it.per = per;
@@ -1078,11 +1100,17 @@ void make_items(const SketchCall &c, const Batch &b, int64_t s0, int64_t s1, int
         it.end = std::min(p + step, e - window + 1);
         if (it.end <= it.begin) continue;
         it.row = static_cast<int32_t>((s - b.s0) * K + k);
-        it.k = c.kmers[k];
-        it.tab = k;
+        it.k = static_cast<int16_t>(c.kmers[k]);
+        it.tab = static_cast<int16_t>(k);
         items.push_back(it);
       }
   }
+}
+
+std::vector<int> all_k(const SketchCall &c) {
+  std::vector<int> ks(c.kmers.size());
+  for (size_t k = 0; k < ks.size(); ++k) ks[k] = static_cast<int>(k);
+  return ks;
 }
 
 sk_status upload(sk_ctx *ctx, void *dst, const void *src, size_t bytes) {
@@ -1153,7 +1181,7 @@ sk_status count_partitioned(SketchCall &c, const Batch &b, SketchArgs &args, std
   sk_ctx *ctx = c.ctx;
   const int K = static_cast<int>(c.kmers.size());
   items.clear();
-  make_items(c, b, s, s + 1, k, items, per_item);
+  make_items(c, b, s, s + 1, {k}, items, per_item);
   if (items.empty()) return SK_OK;
   void *p = nullptr;
   sk_status st = scratch(ctx, kSlotSketchItems, items.size() * sizeof(SketchItem), &p);
@@ -1240,7 +1268,7 @@ sk_status count_full(SketchCall &c, const Batch &b, SketchArgs &args, std::vecto
   args.min_count = static_cast<unsigned int>(c.min_count);
   for (int k : ks) {
     items.clear();
-    make_items(c, b, s, s + 1, k, items, kCountItemWindows);
+    make_items(c, b, s, s + 1, {k}, items, kCountItemWindows);
     if (items.empty()) continue;
     void *p = nullptr;
     st = scratch(ctx, kSlotSketchItems, items.size() * sizeof(SketchItem), &p);
@@ -1277,19 +1305,39 @@ int64_t sample_windows(const SketchCall &c, int64_t s) {
   return c.seq_off[c.sample_seqs[s + 1]] - c.seq_off[c.sample_seqs[s]];
 }
 
+// Bins left empty above which the sample is counted in full at that k: a second
+// roll and the first cost about half of a full count, and what the second keeps
+// is counted on top.
+int64_t low_max_empty(const SketchCall &c) { return c.nbins / 4; }
+
+// Window starts per item of a low roll over `windows` windows in all: about
+// four items per SM (two CTAs at a time), of at least 64 windows per thread (each
+// first rolls over k - 1 bases), in the steps of make_items.
+int64_t low_item_windows(const sk_ctx *ctx, int64_t windows) {
+  constexpr int64_t kStep = 16 * kSketchThreads;
+  const int64_t per = (windows / (4 * ctx->sm_count) + kStep - 1) / kStep * kStep;
+  return std::min(kItemWindows, std::max<int64_t>(4 * kStep, per));
+}
+
 // Buffers of one low count: lists of the items, tables and their counters.
 struct LowPlan {
   uint64_t slots = 0;
   unsigned int cap = 0;
+  int n_tables = 0;
   size_t lists_off = 0, counts_off = 0, bytes = 0;
 };
 
-// For items of at most per_item windows of which a fraction f is kept, n_tables
-// tables each holding the `kept` hashes of one (sample, k) at two thirds at most.
-LowPlan low_plan(double f, int64_t per_item, size_t n_items, int n_tables, double kept) {
+// Slots of a table that holds `kept` hashes at two thirds at most.
+uint64_t low_slots(double kept) {
+  return std::max<uint64_t>(1024, next_pow2(static_cast<uint64_t>(kept * 1.5)));
+}
+
+// For items of at most per_item windows of which a fraction f is kept.
+LowPlan low_plan(double f, int64_t per_item, size_t n_items, int n_tables, uint64_t slots) {
   LowPlan p;
-  p.slots = std::max<uint64_t>(1024, next_pow2(static_cast<uint64_t>(kept * 1.5)));
+  p.slots = slots;
   p.cap = static_cast<unsigned int>(per_item * f * 1.25) + 512;
+  p.n_tables = n_tables;
   p.lists_off = static_cast<size_t>(n_tables) * p.slots * sizeof(TableSlot);
   p.counts_off = p.lists_off + n_items * p.cap * 8;
   p.bytes = p.counts_off + (n_items + n_tables) * 4;
@@ -1297,26 +1345,29 @@ LowPlan low_plan(double f, int64_t per_item, size_t n_items, int n_tables, doubl
 }
 
 // One low count over `items` (uploaded here): tables cleared, roll, count.
-sk_status run_low(SketchCall &c, SketchArgs &args, const std::vector<SketchItem> &items,
-                  const LowPlan &p, int n_tables, LowArgs la) {
+// Below 64 KB, as the items of a sample of up to 70 M bases are, the upload does
+// not queue behind the bases of the next chunk on the copy engine.
+sk_status run_low(SketchCall &c, SketchArgs args, const std::vector<SketchItem> &items,
+                  const LowPlan &p, LowArgs la) {
+  const size_t n_items = items.size();
+  if (n_items == 0) return SK_OK;
   sk_ctx *ctx = c.ctx;
   void *tk = nullptr, *di = nullptr;
   sk_status st = scratch(ctx, kSlotSketchTable, p.bytes, &tk);
-  if (st == SK_OK) st = scratch(ctx, kSlotSketchItems, items.size() * sizeof(SketchItem), &di);
-  if (st == SK_OK) st = upload(ctx, di, items.data(), items.size() * sizeof(SketchItem));
+  if (st == SK_OK) st = scratch(ctx, kSlotSketchItems, n_items * sizeof(SketchItem), &di);
+  if (st == SK_OK) st = upload(ctx, di, items.data(), n_items * sizeof(SketchItem));
   if (st != SK_OK) return st;
   char *base = static_cast<char *>(tk);
   la.tables = reinterpret_cast<TableSlot *>(base);
   la.slots = p.slots;
+  la.n_tables = p.n_tables;
   la.hashes = reinterpret_cast<unsigned long long *>(base + p.lists_off);
   la.cap = p.cap;
   la.count = reinterpret_cast<unsigned int *>(base + p.counts_off);
-  la.max_key = la.count + items.size();
-  la.by_k = n_tables > 1;
+  la.max_key = la.count + n_items;
   args.items = static_cast<SketchItem *>(di);
-  const unsigned grid = static_cast<unsigned>(items.size());
-  low_clear_kernel<<<ctx->sm_count * 8, 256, 0, ctx->stream>>>(la.tables, n_tables * p.slots,
-                                                              la.max_key, n_tables);
+  const unsigned grid = static_cast<unsigned>(n_items);
+  low_clear_kernel<<<ctx->sm_count * 8, 256, 0, ctx->stream>>>(la);
   const auto roll =
       la.empty ? (c.codon_phased ? (c.use_rc ? low_roll_kernel<true, true, true> : low_roll_kernel<false, true, true>)
                                  : (c.use_rc ? low_roll_kernel<true, false, true> : low_roll_kernel<false, false, true>))
@@ -1332,25 +1383,19 @@ sk_status run_low(SketchCall &c, SketchArgs &args, const std::vector<SketchItem>
 }
 
 // Bins rows of one batch with the exact count filter.  Samples of at least
-// kLowMinPerBin windows per bin are counted from the low end of their bins, all
-// k in one roll; what that leaves (bins still empty, lists or tables too small)
-// and the other samples are counted in full.
+// kLowMinPerBin windows per bin are counted from the low end of their bins, the
+// longest k first and then the others in one roll; what that leaves is counted
+// again (bins still empty) or in full (too many of them, lists or tables too
+// small), as are the other samples.
 sk_status count_batch(SketchCall &c, const Batch &b, SketchArgs &args, std::vector<SketchItem> &items) {
   sk_ctx *ctx = c.ctx;
   const int K = static_cast<int>(c.kmers.size());
-  // bytes of table per pass: a quarter of the context's memory limit when one
-  // is set, else a quarter of the free device memory less 2 GiB (at least 1 GiB)
-  uint64_t budget = 0;
-  if (ctx->mem_limit > 0) {
-    budget = std::max<uint64_t>(1ULL << 16, static_cast<uint64_t>(ctx->mem_limit) / 4);
-  } else {
-    size_t free_b = 0, total_b = 0;
-    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) free_b = 0;
-    budget = std::max<uint64_t>(1ULL << 30, free_b > (2ULL << 30) ? (free_b - (2ULL << 30)) / 4 : 0);
-  }
+  uint64_t budget = 0;   // bytes of tables and lists, set below
   args.min_count = static_cast<unsigned int>(c.min_count);
-  std::vector<int> all(K);
-  for (int k = 0; k < K; ++k) all[k] = k;
+  const std::vector<int> all = all_k(c);
+  const int longest = static_cast<int>(std::max_element(c.kmers.begin(), c.kmers.end()) - c.kmers.begin());
+  std::vector<int> others = all;
+  others.erase(others.begin() + longest);
 
   // ---- the low end of every large sample
   const int64_t rows = (b.s1 - b.s0) * K;
@@ -1364,10 +1409,16 @@ sk_status count_batch(SketchCall &c, const Batch &b, SketchArgs &args, std::vect
     const int64_t windows = sample_windows(c, s);
     if (windows < kLowMinPerBin * c.nbins || windows >= (int64_t(1) << 32)) return SK_OK;
     const double f = static_cast<double>(kLowPerBin) * c.nbins / static_cast<double>(windows);
-    items.clear();
-    make_items(c, b, s, s + 1, -1, items);
-    const LowPlan p = low_plan(f, kItemWindows, items.size(), K, f * static_cast<double>(windows));
-    if (items.empty() || p.bytes > budget) return SK_OK;
+    const double kept = f * static_cast<double>(windows);
+    const int64_t per_first = low_item_windows(ctx, windows), per_rest = low_item_windows(ctx, windows * (K - 1));
+    std::vector<SketchItem> first, rest;
+    make_items(c, b, s, s + 1, {longest}, first, per_first);
+    make_items(c, b, s, s + 1, others, rest, per_rest);
+    for (SketchItem &it : rest) it.table = it.tab - (it.tab > longest);
+    const LowPlan p_first = low_plan(f, per_first, first.size(), 1, low_slots(kept));
+    const LowPlan p_rest = low_plan(f, per_rest, rest.size(), std::max(1, K - 1), low_slots(kept));
+    const size_t bytes = std::max(p_first.bytes, p_rest.bytes);
+    if (first.size() + rest.size() == 0 || bytes > budget) return SK_OK;
     if (!any) {
       void *r = nullptr;
       const sk_status st = scratch(ctx, kSlotSketchRows, static_cast<size_t>(rows) * (2 + words) * 4, &r);
@@ -1380,7 +1431,23 @@ sk_status count_batch(SketchCall &c, const Batch &b, SketchArgs &args, std::vect
     }
     la.low = static_cast<uint64_t>(static_cast<double>(c.binsize) * f);
     low[s - b.s0] = 1;
-    return run_low(c, args, items, p, K, la);
+    void *p = nullptr;   // grown once, to the larger of the two
+    sk_status st = scratch(ctx, kSlotSketchTable, bytes, &p);
+    if (st == SK_OK)
+      st = scratch(ctx, kSlotSketchItems, std::max(first.size(), rest.size()) * sizeof(SketchItem), &p);
+    if (st == SK_OK) st = run_low(c, args, first, p_first, la);
+    if (st != SK_OK || rest.empty()) return st;
+    const int64_t row = (s - b.s0) * K + longest;
+    LowArgs gated = la;
+    if (!first.empty()) {   // (no windows at the longest k: its bins are all empty, whatever the others hold)
+      empty_bins_kernel<<<1, 256, 0, ctx->stream>>>(args.signs + row * c.nbins, c.nbins, words,
+                                                    d_rows + 2 * rows + row * words, d_rows + rows + row);
+      const cudaError_t e = cudaGetLastError();
+      if (e != cudaSuccess) return cuda_fail(ctx, e, "sketch counting");
+      gated.gate = d_rows + rows + row;
+      gated.gate_max = static_cast<unsigned int>(low_max_empty(c));
+    }
+    return run_low(c, args, rest, p_rest, gated);
   };
   // host bases of more than one chunk of samples go up on the copy stream, the
   // next chunk while this one is counted
@@ -1407,6 +1474,16 @@ sk_status count_batch(SketchCall &c, const Batch &b, SketchArgs &args, std::vect
     if (e != cudaSuccess) return cuda_fail(ctx, e, "sketch upload");
     st = copy_part(0);
   }
+  // bytes of tables and lists, asked for while the first bases go up: a quarter
+  // of the context's memory limit when one is set, else a quarter of the free
+  // device memory less 2 GiB (at least 1 GiB)
+  if (ctx->mem_limit > 0) {
+    budget = std::max<uint64_t>(1ULL << 16, static_cast<uint64_t>(ctx->mem_limit) / 4);
+  } else {
+    size_t free_b = 0, total_b = 0;
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) free_b = 0;
+    budget = std::max<uint64_t>(1ULL << 30, free_b > (2ULL << 30) ? (free_b - (2ULL << 30)) / 4 : 0);
+  }
   for (size_t i = 0; st == SK_OK && i < parts.size(); ++i) {
     if (chunked) {
       const cudaError_t e = cudaStreamWaitEvent(ctx->stream, ctx->ev_ready[i & 1], 0);
@@ -1431,35 +1508,69 @@ sk_status count_batch(SketchCall &c, const Batch &b, SketchArgs &args, std::vect
   }
 
   // ---- what is left
+  std::vector<int64_t> again;   // rows to roll a second time, for their empty bins
   for (int64_t s = b.s0; s < b.s1; ++s) {
     std::vector<int> full = all;
     if (low[s - b.s0]) {
       full.clear();
-      const int64_t windows = sample_windows(c, s);
       for (int k = 0; k < K; ++k) {
         const int64_t row = (s - b.s0) * K + k;
         const unsigned int empty = state[rows + row];
-        if (state[row]) {
-          full.push_back(k);
-        } else if (empty > 0) {
-          // every hash of the empty bins, unless that is most of the sample
-          const double f = static_cast<double>(empty) / c.nbins;
-          items.clear();
-          make_items(c, b, s, s + 1, k, items);
-          const LowPlan p = low_plan(f, kItemWindows, items.size(), 1,
-                                     f * static_cast<double>(windows) + 1024);
-          if (f > 0.25 || p.bytes > budget) {
-            full.push_back(k);
-            continue;
-          }
-          const sk_status st = run_low(c, args, items, p, 1, la);
-          if (st != SK_OK) return st;
-        }
+        if (state[row] || empty > low_max_empty(c)) full.push_back(k);
+        else if (empty > 0) again.push_back(row);
       }
     }
     if (full.empty()) continue;
     const sk_status st = count_full(c, b, args, items, s, full, budget);
     if (st != SK_OK) return st;
+  }
+  // the second rolls, those with the most to keep first: as many in a launch as
+  // fit the budget, with tables of one size for rows within a factor of eight
+  auto windows_of = [&](int64_t row) { return sample_windows(c, b.s0 + row / K); };
+  auto fraction = [&](int64_t row) { return static_cast<double>(state[rows + row]) / c.nbins; };
+  auto slots_of = [&](int64_t row) {
+    return low_slots(fraction(row) * static_cast<double>(windows_of(row)) + 1024);
+  };
+  std::sort(again.begin(), again.end(), [&](int64_t x, int64_t y) {
+    return slots_of(x) != slots_of(y) ? slots_of(x) > slots_of(y) : x < y;
+  });
+  for (size_t i = 0; i < again.size();) {
+    const uint64_t slots = slots_of(again[i]);
+    size_t end = i;
+    int64_t windows = 0;
+    double f = 0.0;
+    LowPlan p;
+    while (end < again.size() && slots_of(again[end]) * 8 >= slots) {
+      const int64_t w = windows + windows_of(again[end]);
+      const double g = std::max(f, fraction(again[end]));
+      const int64_t per = low_item_windows(ctx, w);
+      const size_t at_most = static_cast<size_t>(w / per) + 2 * (end + 1 - i);   // items
+      const LowPlan q = low_plan(g, per, at_most, static_cast<int>(end + 1 - i), slots);
+      if (q.bytes > budget) break;
+      p = q;
+      windows = w;
+      f = g;
+      ++end;
+    }
+    if (end == i) {   // one row alone is over the budget
+      const sk_status st = count_full(c, b, args, items, b.s0 + again[i] / K,
+                                      {static_cast<int>(again[i] % K)}, budget);
+      if (st != SK_OK) return st;
+      ++i;
+      continue;
+    }
+    const int64_t per = low_item_windows(ctx, windows);
+    items.clear();
+    for (size_t r = i; r < end; ++r) {
+      const size_t at = items.size();
+      const int64_t s = b.s0 + again[r] / K;
+      make_items(c, b, s, s + 1, {static_cast<int>(again[r] % K)}, items, per);
+      for (size_t j = at; j < items.size(); ++j) items[j].table = static_cast<int32_t>(r - i);
+    }
+    p = low_plan(f, per, items.size(), static_cast<int>(end - i), slots);
+    const sk_status st = run_low(c, args, items, p, la);
+    if (st != SK_OK) return st;
+    i = end;
   }
   if (!any) return SK_OK;
   // a second roll's list or table that was too small: that row in full
@@ -1491,7 +1602,7 @@ sk_status hash_batch(SketchCall &c, const Batch &b, SketchArgs &args, std::vecto
   std::vector<size_t> first(parts.size() + 1, 0);
   items.clear();
   for (size_t i = 0; i < parts.size(); ++i) {
-    make_items(c, b, parts[i].s0, parts[i].s1, -1, items);
+    make_items(c, b, parts[i].s0, parts[i].s1, all_k(c), items);
     first[i + 1] = items.size();
   }
   void *p = nullptr;
