@@ -548,7 +548,8 @@ struct LowArgs {
 // The roll's emitter.  A thread puts its kept hashes into its own column of a
 // shared-memory array (a predicated store, no branch); when some lane of the
 // warp has more than half of its column filled, the lanes write theirs out
-// together.  Writing each kept hash at once took a branch in nearly every step
+// together (each by itself in a warp whose lanes do not all have a full share of
+// windows, and so do not take the same steps).  Writing each kept hash at once took a branch in nearly every step
 // of a warp (105 us per k for 20 Mbases; 91 now, at two CTAs per SM).
 template <bool kBitmap>
 struct LowKeep {
@@ -560,6 +561,7 @@ struct LowKeep {
   unsigned int cap;
   uint64_t binsize, magic, low;
   const unsigned int *empty;
+  bool together;                // the warp's lanes roll equally many windows
   int n = 0;
 
   __device__ __forceinline__ void put(uint64_t h, bool valid) {
@@ -579,7 +581,8 @@ struct LowKeep {
     n = 0;
   }
   __device__ __forceinline__ void flush() {
-    if (__any_sync(__activemask(), n > kColumn - kBatch)) drain();
+    const bool full = n > kColumn - kBatch;
+    if (together ? __any_sync(0xffffffffu, full) : full) drain();
   }
 };
 
@@ -609,12 +612,13 @@ low_roll_kernel(SketchArgs a, LowArgs la) {
     if (threadIdx.x == 0) la.count[blockIdx.x] = 0;
     return;
   }
+  const int64_t s = it.begin + static_cast<int64_t>(threadIdx.x) * it.per;
+  const int64_t e = min(s + it.per, it.end);
   LowKeep<kBitmap> keep{low_columns + threadIdx.x,
                         la.hashes + static_cast<int64_t>(blockIdx.x) * la.cap, &kept, la.cap,
                         a.binsize, a.magic, la.low,
-                        kBitmap ? la.empty + static_cast<int64_t>(it.row) * la.words : nullptr};
-  const int64_t s = it.begin + static_cast<int64_t>(threadIdx.x) * it.per;
-  const int64_t e = min(s + it.per, it.end);
+                        kBitmap ? la.empty + static_cast<int64_t>(it.row) * la.words : nullptr,
+                        __all_sync(0xffffffffu, s + it.per <= it.end) != 0};
   if (s < e) {
     roll_windows<kRc, kPhased>(a.codes, s, e, it.k, tab, LowEmit<kBitmap>{keep});
     keep.drain();
