@@ -222,9 +222,12 @@ extern "C" sk_status sk_query_db_ready(sk_ctx *ctx, const sk_host_sketches *ref,
   lb[1] = lb[0];
   lb[1].lp.cta_scratch = static_cast<uint16_t *>(cta_b);
   lb[1].lp.split_scratch = static_cast<uint16_t *>(split_b);
-  // the second compute stream starts after the status reset and the work list
+  // the second compute stream starts after the status reset and the work list,
+  // and so does the pack stream where it writes column values: an earlier call
+  // that was only queued may still be reading the code buffer
   cudaError_t e = cudaEventRecord(ctx->ev_join, ctx->stream);
   if (e == cudaSuccess) e = cudaStreamWaitEvent(ctx->stream_b, ctx->ev_join, 0);
+  if (e == cudaSuccess && coded) e = cudaStreamWaitEvent(ctx->pack_stream, ctx->ev_join, 0);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "work list upload");
 
   // ---- upload units: the query side whole (in chunk-sized pieces), then the
