@@ -91,6 +91,16 @@ size_t batch_code_budget(const std::vector<JobParams> &jobs, const TileConfig &c
   return std::min({codes, size_t(8) << 30, free_b / 4 - values});
 }
 
+// The jobs' plan under one tile shape, in the context's scratch.
+sk_status plan_to_time(sk_ctx *ctx, const std::vector<JobParams> &jobs, const TileConfig &cfg,
+                       Plan &plan, LaunchBuffers &buf) {
+  return plan_with_codes(ctx, jobs, cfg, [&](size_t code_budget) {
+    plan = Plan{};
+    const sk_status st = make_plan(ctx, jobs, cfg, code_budget, plan);
+    return st == SK_OK ? upload_plan(ctx, plan, buf, false) : st;
+  });
+}
+
 // Times `repeats` launches of the plan (after one warm-up), in milliseconds.
 sk_status time_plan(sk_ctx *ctx, const Plan &plan, const LaunchBuffers &buf, int repeats,
                     float *ms) {
@@ -141,11 +151,10 @@ sk_status sk_batch_create(sk_ctx *ctx, const sk_job *jobs, int32_t n_jobs, int32
       int64_t pairs = 0;
       st = build_jobs(ctx, jobs, n_jobs, *c, jp, &pairs);
       if (st != SK_OK) return st;
+      if (resident_grid(ctx, *c) < 1) continue;
       Plan plan;
-      st = make_plan(ctx, jp, *c, code_budget_for(ctx, jp, *c), plan);
-      if (st != SK_OK) continue;
       LaunchBuffers buf;
-      st = upload_plan(ctx, plan, buf, false);
+      st = plan_to_time(ctx, jp, *c, plan, buf);
       if (st != SK_OK) return st;
       float ms = 0.0f;
       st = time_plan(ctx, plan, buf, 2, &ms);
@@ -276,10 +285,10 @@ sk_status sk_autotune(sk_ctx *ctx, const sk_db *ref, const sk_db *query, const s
     int64_t p = 0;
     st = build_jobs(ctx, &job, 1, *c, jp, &p);
     if (st != SK_OK) return st;
+    if (resident_grid(ctx, *c) < 1) continue;
     Plan plan;
-    if (make_plan(ctx, jp, *c, code_budget_for(ctx, jp, *c), plan) != SK_OK) continue;
     LaunchBuffers buf;
-    st = upload_plan(ctx, plan, buf, false);
+    st = plan_to_time(ctx, jp, *c, plan, buf);
     if (st != SK_OK) return st;
     float ms = 0.0f;
     st = time_plan(ctx, plan, buf, std::max(1, repeats), &ms);

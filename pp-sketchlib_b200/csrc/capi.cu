@@ -14,6 +14,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <functional>
 #include <limits>
 #include <fstream>
 #include <map>
@@ -63,8 +64,8 @@ sk_status attach_count_tables(sk_ctx *ctx, JobParams *jp, bool alloc) {
     if (!alloc) return SK_OK;
     float *jt = nullptr;
     double *lt = nullptr;
-    cudaError_t e = cudaMalloc(&jt, (bins + 1) * sizeof(float));
-    if (e == cudaSuccess) e = cudaMalloc(&lt, (bins + 1) * sizeof(double));
+    cudaError_t e = device_alloc(ctx, &jt, (bins + 1) * sizeof(float));
+    if (e == cudaSuccess) e = device_alloc(ctx, &lt, (bins + 1) * sizeof(double));
     if (e == cudaSuccess) e = launch_count_tables(jp->union_bits, bins + 1, jt, lt, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) {
@@ -133,6 +134,28 @@ DeviceGuard::DeviceGuard(int dev) {
 }
 DeviceGuard::~DeviceGuard() { cudaSetDevice(prev_); }
 
+// Frees the context's code buffer, which a call can do without; true if there
+// was one.  Not between a plan's upload and its last launch.
+bool release_codes(sk_ctx *ctx) {
+  Scratch &s = ctx->scratch[kSlotCodes];
+  if (!s.ptr) return false;
+  for (cudaStream_t st : {ctx->stream, ctx->stream_b, ctx->pack_stream})
+    if (st) cudaStreamSynchronize(st);
+  cudaFree(s.ptr);
+  s = Scratch{};
+  return true;
+}
+
+// cudaMalloc, with the code buffer given back where memory is short.
+cudaError_t device_alloc(sk_ctx *ctx, void **p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    if (release_codes(ctx)) e = cudaMalloc(p, bytes);
+  }
+  return e;
+}
+
 // Grows the context's device scratch buffer `slot` to at least `bytes`.
 sk_status scratch(sk_ctx *ctx, int slot, size_t bytes, void **out) {
   Scratch &s = ctx->scratch[slot];
@@ -143,8 +166,11 @@ sk_status scratch(sk_ctx *ctx, int slot, size_t bytes, void **out) {
       s.ptr = nullptr;
       s.bytes = 0;
     }
-    cudaError_t e = cudaMalloc(&s.ptr, bytes);
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "scratch allocation");
+    const cudaError_t e = device_alloc(ctx, &s.ptr, bytes);
+    if (e != cudaSuccess) {
+      s.ptr = nullptr;
+      return cuda_fail(ctx, e, "scratch allocation");
+    }
     s.bytes = bytes;
   }
   *out = s.ptr;
@@ -254,7 +280,7 @@ sk_status ensure_jv(sk_ctx *ctx, sk_db *db, int use_rc) {
   if (db->jv && db->jv_rc == use_rc) return SK_OK;
   const std::vector<double> jv = equal_base_factors(db, use_rc);
   if (!db->jv) {
-    cudaError_t e = cudaMalloc(&db->jv, jv.size() * sizeof(double));
+    cudaError_t e = device_alloc(ctx, &db->jv, jv.size() * sizeof(double));
     if (e != cudaSuccess) return cuda_fail(ctx, e, "random-match factors");
   }
   cudaError_t e = cudaMemcpy(db->jv, jv.data(), jv.size() * sizeof(double), cudaMemcpyHostToDevice);
@@ -348,7 +374,7 @@ sk_status build_job(sk_ctx *ctx, const sk_db *ref, const sk_db *query, const sk_
     if (!r->jgpu || r->jgpu_rc != random->use_rc) {
       const std::vector<float> t = equal_base_gpu(r, random->use_rc);
       if (!r->jgpu) {
-        cudaError_t e = cudaMalloc(&r->jgpu, t.size() * sizeof(float));
+        cudaError_t e = device_alloc(ctx, &r->jgpu, t.size() * sizeof(float));
         if (e != cudaSuccess) return cuda_fail(ctx, e, "random-match chances");
       }
       cudaError_t e = cudaMemcpy(r->jgpu, t.data(), t.size() * sizeof(float), cudaMemcpyHostToDevice);
@@ -731,7 +757,7 @@ sk_status upload_plan(sk_ctx *ctx, Plan &plan, LaunchBuffers &buf, bool owned) {
     *ptrs[i] = nullptr;
     if (sizes[i] == 0) continue;
     if (owned) {
-      const cudaError_t e = cudaMalloc(ptrs[i], sizes[i]);
+      const cudaError_t e = device_alloc(ctx, ptrs[i], sizes[i]);
       if (e != cudaSuccess) return cuda_fail(ctx, e, "batch buffers");
     } else {
       const sk_status st = scratch(ctx, slots[i], sizes[i], ptrs[i]);
@@ -886,6 +912,22 @@ sk_status make_plan(sk_ctx *ctx, const std::vector<JobParams> &jobs, const TileC
   return SK_OK;
 }
 
+// Makes and uploads a plan by `make(code budget)`: with the codes the context
+// grants these jobs, or without any where their buffer and the buffers that the
+// call cannot do without do not fit together (the latter come first).
+sk_status plan_with_codes(sk_ctx *ctx, const std::vector<JobParams> &jobs, const TileConfig &cfg,
+                          const std::function<sk_status(size_t)> &make) {
+  const size_t budget = code_budget_for(ctx, jobs, cfg);
+  sk_status st = make(budget);
+  if (st == SK_ENOMEM && budget > 0) {
+    release_codes(ctx);
+    cudaGetLastError();
+    ctx->err.clear();
+    st = make(0);
+  }
+  return st;
+}
+
 // Whether a query job goes to the few-queries kernel: no tile shape forced or
 // tuned, narrow, and few rows.  Both kernels run at the same LOP3 rate, so the
 // line is the padding: groups of 1 .. 16 rows there, tiles of 64 or 128 rows
@@ -914,12 +956,13 @@ sk_status launch_job(sk_ctx *ctx, const JobParams &jp, const TileConfig &cfg) {
     return e == cudaSuccess ? SK_OK : cuda_fail(ctx, e, "query kernel launch");
   }
   Plan plan;
-  sk_status st = make_plan(ctx, {jp}, cfg, code_budget_for(ctx, {jp}, cfg), plan);
-  if (st != SK_OK) return st;
   LaunchBuffers buf;
-  st = upload_plan(ctx, plan, buf, false);
-  if (st != SK_OK) return st;
-  return enqueue_plan(ctx, plan, buf);
+  const sk_status st = plan_with_codes(ctx, {jp}, cfg, [&](size_t code_budget) {
+    plan = Plan{};
+    const sk_status made = make_plan(ctx, {jp}, cfg, code_budget, plan);
+    return made == SK_OK ? upload_plan(ctx, plan, buf, false) : made;
+  });
+  return st == SK_OK ? enqueue_plan(ctx, plan, buf) : st;
 }
 
 int64_t n_pairs(const sk_db *ref, const sk_db *query) {
@@ -961,13 +1004,14 @@ sk_status ensure_copy_stream(sk_ctx *ctx) {
 }
 
 // Device bytes a dense call may use to stage its output: the context's limit,
-// else the free memory less a 2 GiB margin.  The output staging buffer the
-// context already holds counts as available: growing it frees it first.
+// else the free memory less a 2 GiB margin.  What the context already holds for
+// staged output and for codes counts as available: growing the one frees it
+// first, the other is given back when memory runs out.
 size_t dense_budget(sk_ctx *ctx) {
   if (ctx->mem_limit > 0) return static_cast<size_t>(ctx->mem_limit);
   size_t free_b = 0, total_b = 0;
   if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return 0;
-  free_b += ctx->scratch[kSlotOut].bytes;
+  free_b += ctx->scratch[kSlotOut].bytes + ctx->scratch[kSlotCodes].bytes;
   const size_t margin = size_t(2) << 30;
   return free_b > 2 * margin ? free_b - margin : free_b / 2;
 }
@@ -1022,21 +1066,25 @@ sk_status dense_blocked_to_host(sk_ctx *ctx, const sk_db *ref, const sk_db *quer
   for (int c = 0; c < nblk; ++c) jobs[c].out = buf[c & 1];
   Plan plan;
   LaunchBuffers lb;
-  st = plan.start(ctx, *cfg, code_budget_for(ctx, {base}, *cfg));
-  const bool coded = plan.can_code(base);
   std::vector<size_t> sub_end(nblk);   // launches of blocks 0 .. c
-  for (int c = 0; st == SK_OK && c < nblk; ++c) {
-    if (coded) {
-      plan.add_coded(jobs[c], static_cast<int32_t>(cut[c]), static_cast<int32_t>(cut[c + 1]), 0,
-                     base.n_col_tiles, 0);
-    } else {
-      const int at = plan.add_job(jobs[c]);
-      for (int64_t t = first_tile(cut[c]); t < first_tile(cut[c + 1]); ++t) plan.add_tile(at, t);
+  st = plan_with_codes(ctx, {base}, *cfg, [&](size_t code_budget) {
+    plan = Plan{};
+    sk_status made = plan.start(ctx, *cfg, code_budget);
+    if (made != SK_OK) return made;
+    const bool coded = plan.can_code(base);
+    for (int c = 0; c < nblk; ++c) {
+      if (coded) {
+        plan.add_coded(jobs[c], static_cast<int32_t>(cut[c]), static_cast<int32_t>(cut[c + 1]), 0,
+                       base.n_col_tiles, 0);
+      } else {
+        const int at = plan.add_job(jobs[c]);
+        for (int64_t t = first_tile(cut[c]); t < first_tile(cut[c + 1]); ++t) plan.add_tile(at, t);
+      }
+      if (!plan.open_empty()) plan.close_launch();
+      sub_end[c] = plan.subs.size();
     }
-    if (!plan.open_empty()) plan.close_launch();
-    sub_end[c] = plan.subs.size();
-  }
-  if (st == SK_OK) st = upload_plan(ctx, plan, lb, false);
+    return upload_plan(ctx, plan, lb, false);
+  });
   if (st == SK_OK) st = reset_plan(ctx, lb);
   if (st != SK_OK) return st;
   cudaError_t e = cudaSuccess;
@@ -1308,7 +1356,7 @@ sk_status db_alloc(sk_ctx *ctx, int64_t n, const int32_t *kmers, int32_t K, int3
     db->packed = static_cast<uint32_t *>(buf);
     db->own_packed = false;
   } else {
-    cudaError_t e = cudaMalloc(&db->packed, packed_words * 4);
+    cudaError_t e = device_alloc(ctx, &db->packed, packed_words * 4);
     if (e != cudaSuccess) {
       delete db;
       ctx_release(ctx);
@@ -1351,7 +1399,7 @@ static sk_status db_create_impl(sk_ctx *ctx, const uint64_t *words, bool on_devi
   const uint64_t *d_words = words;
   uint64_t *tmp = nullptr;
   if (!on_device && n > 0) {
-    e = cudaMalloc(&tmp, in_words * 8);
+    e = device_alloc(ctx, &tmp, in_words * 8);
     if (e == cudaSuccess) e = cudaMemcpyAsync(tmp, words, in_words * 8, cudaMemcpyHostToDevice, ctx->stream);
     d_words = tmp;
   }
@@ -1412,7 +1460,7 @@ sk_status sk_db_set_sample_info(sk_db *db, const uint16_t *cluster, const uint64
     std::copy(cluster, cluster + db->n, cl.begin());
     db->max_cluster = db->n > 0 ? *std::max_element(cluster, cluster + db->n) : 0;
     if (!db->cluster) {
-      cudaError_t e = cudaMalloc(&db->cluster, npad * sizeof(uint16_t));
+      cudaError_t e = device_alloc(ctx, &db->cluster, npad * sizeof(uint16_t));
       if (e != cudaSuccess) return cuda_fail(ctx, e, "cluster ids");
     }
     cudaError_t e = cudaMemcpy(db->cluster, cl.data(), npad * sizeof(uint16_t), cudaMemcpyHostToDevice);
@@ -1468,7 +1516,7 @@ sk_status sk_random_create(sk_ctx *ctx, int32_t mode, int32_t use_rc, const int3
     }
     r->n_clusters = n_clusters;
     const size_t sz = static_cast<size_t>(n_kmers) * n_clusters * n_clusters * sizeof(float);
-    cudaError_t e = cudaMalloc(&r->table, sz);
+    cudaError_t e = device_alloc(ctx, &r->table, sz);
     if (e == cudaSuccess) e = cudaMemcpy(r->table, table, sz, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
       if (r->table) cudaFree(r->table);
@@ -1850,8 +1898,8 @@ sk_status sk_synth_device(sk_ctx *ctx, const int32_t *parent, const uint32_t *th
     if (parent[s] >= s) return fail(ctx, SK_EINVAL, "parents must precede their children");
   int32_t *d_parent = nullptr;
   uint32_t *d_thresh = nullptr;
-  cudaError_t e = cudaMalloc(&d_parent, n_samples * 4);
-  if (e == cudaSuccess) e = cudaMalloc(&d_thresh, n_samples * n_kmers * 4);
+  cudaError_t e = device_alloc(ctx, &d_parent, n_samples * 4);
+  if (e == cudaSuccess) e = device_alloc(ctx, &d_thresh, n_samples * n_kmers * 4);
   if (e == cudaSuccess) e = cudaMemcpyAsync(d_parent, parent, n_samples * 4, cudaMemcpyHostToDevice, ctx->stream);
   if (e == cudaSuccess) e = cudaMemcpyAsync(d_thresh, thresh, n_samples * n_kmers * 4, cudaMemcpyHostToDevice, ctx->stream);
   if (e == cudaSuccess) e = launch_synth(d_parent, d_thresh, n_samples, n_kmers, sketchsize64, seed, d_words, ctx->stream);

@@ -173,50 +173,56 @@ extern "C" sk_status sk_query_db_ready(sk_ctx *ctx, const sk_host_sketches *ref,
       }
     }
   }
-  // the two compute streams alternate between the halves of the code buffer
-  Plan plan;
-  st = plan.start(ctx, *cfg, code_budget_for(ctx, {jp}, *cfg) / 2);
-  if (st != SK_OK) return st;
-  plan.values_by_caller = true;   // chunk by chunk, behind each pack
-  const bool coded = plan.can_code(jp) && !blocked;
-  const int whole = coded ? -1 : plan.add_job(jp);
-  std::vector<size_t> sub0(n_chunks), sub1(n_chunks);   // launches of each chunk
-  std::vector<int> side(n_chunks);                      // compute stream of each chunk
-  for (int k = 0, launches = 0; k < n_chunks; ++k) {
-    const int c = reverse ? n_chunks - 1 - k : k;       // in upload order
-    sub0[c] = plan.subs.size();
-    side[c] = launches & 1;
-    if (coded) {
-      // self: the row tiles that start in the chunk, over every column from
-      // the diagonal on; query: every row tile over the chunk's columns
-      const auto tile_at = [&](int64_t s, int32_t n) {
-        return static_cast<int32_t>(std::min<int64_t>(s / kCodeGroup, n));
-      };
-      if (jp.self)
-        plan.add_coded(jp, tile_at(c * cs, jp.n_row_tiles), tile_at((c + 1) * cs, jp.n_row_tiles),
-                       0, jp.n_col_tiles, side[c]);
-      else
-        plan.add_coded(jp, 0, jp.n_row_tiles, tile_at(c * cs, jp.n_col_tiles),
-                       c + 1 == n_chunks ? jp.n_col_tiles
-                                         : tile_at((c + 1) * cs, jp.n_col_tiles), side[c]);
-    } else if (!blocked) {
-      for (int64_t t : bucket[c]) plan.add_tile(whole, t);
-    }
-    if (!plan.open_empty()) plan.close_launch();
-    sub1[c] = plan.subs.size();
-    if (sub1[c] > sub0[c]) ++launches;
-  }
-
-  // ---- device buffers: the plan, count scratch for the second stream, staging
+  // ---- launches and device buffers: the plan, count scratch for the second
+  // stream, staging; the two compute streams alternate between the halves of
+  // the code buffer
   const int64_t wps = static_cast<int64_t>(n_kmers) * sketchsize64 * bbits;   // words per sample
+  Plan plan;
   LaunchBuffers lb[2];
   void *staging = nullptr, *cta_b = nullptr, *split_b = nullptr;
-  st = upload_plan(ctx, plan, lb[0], false);
-  if (st == SK_OK)
-    st = scratch(ctx, kSlotCountsB,
-                 static_cast<size_t>(plan.grid) * count_slot_bytes(*cfg, plan.k_slots), &cta_b);
-  if (st == SK_OK) st = scratch(ctx, kSlotSplitCountsB, plan.split_bytes(), &split_b);
-  if (st == SK_OK) st = scratch(ctx, kSlotStaging, static_cast<size_t>(2 * cs * wps) * 8, &staging);
+  bool coded = false;
+  std::vector<size_t> sub0(n_chunks), sub1(n_chunks);   // launches of each chunk
+  std::vector<int> side(n_chunks);                      // compute stream of each chunk
+  auto make = [&](size_t code_budget) {
+    plan = Plan{};
+    sk_status made = plan.start(ctx, *cfg, code_budget / 2);
+    if (made != SK_OK) return made;
+    plan.values_by_caller = true;   // chunk by chunk, behind each pack
+    coded = plan.can_code(jp) && !blocked;
+    const int whole = coded ? -1 : plan.add_job(jp);
+    for (int k = 0, launches = 0; k < n_chunks; ++k) {
+      const int c = reverse ? n_chunks - 1 - k : k;       // in upload order
+      sub0[c] = plan.subs.size();
+      side[c] = launches & 1;
+      if (coded) {
+        // self: the row tiles that start in the chunk, over every column from
+        // the diagonal on; query: every row tile over the chunk's columns
+        const auto tile_at = [&](int64_t s, int32_t n) {
+          return static_cast<int32_t>(std::min<int64_t>(s / kCodeGroup, n));
+        };
+        if (jp.self)
+          plan.add_coded(jp, tile_at(c * cs, jp.n_row_tiles), tile_at((c + 1) * cs, jp.n_row_tiles),
+                         0, jp.n_col_tiles, side[c]);
+        else
+          plan.add_coded(jp, 0, jp.n_row_tiles, tile_at(c * cs, jp.n_col_tiles),
+                         c + 1 == n_chunks ? jp.n_col_tiles
+                                           : tile_at((c + 1) * cs, jp.n_col_tiles), side[c]);
+      } else if (!blocked) {
+        for (int64_t t : bucket[c]) plan.add_tile(whole, t);
+      }
+      if (!plan.open_empty()) plan.close_launch();
+      sub1[c] = plan.subs.size();
+      if (sub1[c] > sub0[c]) ++launches;
+    }
+    // the plan's own buffers last: its codes come after all that must be had
+    made = scratch(ctx, kSlotStaging, static_cast<size_t>(2 * cs * wps) * 8, &staging);
+    if (made == SK_OK)
+      made = scratch(ctx, kSlotCountsB,
+                     static_cast<size_t>(plan.grid) * count_slot_bytes(*cfg, plan.k_slots), &cta_b);
+    if (made == SK_OK) made = scratch(ctx, kSlotSplitCountsB, plan.split_bytes(), &split_b);
+    return made == SK_OK ? upload_plan(ctx, plan, lb[0], false) : made;
+  };
+  st = blocked ? make(0) : plan_with_codes(ctx, {jp}, *cfg, make);
   if (st == SK_OK) st = reset_plan(ctx, lb[0]);
   if (st != SK_OK) return st;
   lb[1] = lb[0];

@@ -596,6 +596,13 @@ sk_status sk_server_create(sk_ctx *ctx, const sk_db *ref, const sk_random *rando
     sv->slots.emplace_back();
     int64_t bytes = 0;
     st = make_slot(sv, ctx, sv->slots.back(), &bytes);
+    if (st == SK_ENOMEM && release_codes(ctx)) {   // the references' context can do without its codes
+      free_slot(sv->slots.back());
+      cudaGetLastError();
+      ctx->err.clear();
+      bytes = 0;
+      st = make_slot(sv, ctx, sv->slots.back(), &bytes);
+    }
     if (st != SK_OK) break;
     if (i == 0) {
       sv->slot_bytes = bytes;

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <functional>
 #include <map>
 #include <mutex>
 #include <string>
@@ -207,6 +208,12 @@ sk_status fail(sk_ctx *ctx, sk_status st, const char *fmt, ...);
 void ctx_retain(sk_ctx *ctx);
 void ctx_release(sk_ctx *ctx);
 sk_status cuda_fail(sk_ctx *ctx, cudaError_t e, const char *what);
+bool release_codes(sk_ctx *ctx);
+cudaError_t device_alloc(sk_ctx *ctx, void **p, size_t bytes);
+template <class T>
+cudaError_t device_alloc(sk_ctx *ctx, T **p, size_t bytes) {
+  return device_alloc(ctx, reinterpret_cast<void **>(p), bytes);
+}
 sk_status scratch(sk_ctx *ctx, int slot, size_t bytes, void **out);
 sk_status begin_call(sk_ctx *ctx);
 sk_status finish_call(sk_ctx *ctx);
@@ -235,6 +242,8 @@ size_t code_reserve(sk_ctx *ctx, size_t values, size_t codes);
 void code_wants(const std::vector<JobParams> &jobs, const TileConfig &cfg, size_t *values,
                 size_t *codes);
 size_t code_budget_for(sk_ctx *ctx, const std::vector<JobParams> &jobs, const TileConfig &cfg);
+sk_status plan_with_codes(sk_ctx *ctx, const std::vector<JobParams> &jobs, const TileConfig &cfg,
+                          const std::function<sk_status(size_t)> &make);
 double padded_pairs(const TileConfig &cfg, int64_t n_ref, int64_t n_query);
 sk_status db_alloc(sk_ctx *ctx, int64_t n, const int32_t *kmers, int32_t K, int32_t s64,
                    int32_t bbits, sk_db **out, int packed_slot = -1);
