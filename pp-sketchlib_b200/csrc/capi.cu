@@ -949,11 +949,16 @@ sk_status launch_job(sk_ctx *ctx, const JobParams &jp, const TileConfig &cfg) {
   if (jp.n_tiles == 0) return SK_OK;
   if (few_queries(ctx, jp)) {
     void *parts = nullptr;
-    sk_status st = scratch(ctx, kSlotSplitCounts, few_queries_bytes(jp, ctx->sm_count), &parts);
-    if (st != SK_OK) return st;
-    const cudaError_t e = launch_few_queries(jp, static_cast<uint16_t *>(parts), ctx->status_dev,
-                                             ctx->cancel_dev, ctx->sm_count, ctx->stream);
-    return e == cudaSuccess ? SK_OK : cuda_fail(ctx, e, "query kernel launch");
+    const size_t bytes = few_queries_bytes(jp, ctx->sm_count, ctx->few_limit);
+    const sk_status st = scratch(ctx, kSlotSplitCounts, bytes, &parts);
+    if (st == SK_OK) {
+      const cudaError_t e = launch_few_queries(jp, static_cast<uint16_t *>(parts), bytes, ctx->status_dev,
+                                               ctx->cancel_dev, ctx->sm_count, ctx->stream);
+      return e == cudaSuccess ? SK_OK : cuda_fail(ctx, e, "query kernel launch");
+    }
+    if (st != SK_ENOMEM) return st;
+    cudaGetLastError();   // tiles may need less
+    ctx->err.clear();
   }
   Plan plan;
   LaunchBuffers buf;

@@ -12,7 +12,8 @@
 // The blocks of each k are cut into ranges so that a small reference set still
 // fills the device; a range's counts go to a uint16 array [k][range][query]
 // [reference], and a second kernel adds the ranges up and finishes the pairs,
-// one per thread.
+// one per thread.  The array is bounded; more references than it holds the counts
+// of are taken a part at a time.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -32,8 +33,8 @@ constexpr int kFinishPairs = 128;
 
 template <int NQ>
 __global__ void __launch_bounds__(kThreads)
-few_queries_kernel(const JobParams jp, int groups, int ranges, uint16_t *__restrict__ parts, int64_t ldc,
-                   DevStatus *status, const volatile int *cancel) {
+few_queries_kernel(const JobParams jp, int groups, int ranges, uint16_t *__restrict__ parts,
+                   int64_t col_begin, int64_t ldc, DevStatus *status, const volatile int *cancel) {
   __shared__ __align__(16) uint32_t qw[kTileBlocks * kBbits * NQ];
   __shared__ int s_stop;
   if (threadIdx.x == 0) s_stop = poll_cancelled(status, cancel) ? 1 : 0;
@@ -43,8 +44,9 @@ few_queries_kernel(const JobParams jp, int groups, int ranges, uint16_t *__restr
   const int q0 = (blockIdx.x % groups) * NQ;   // this CTA's queries: q0 .. q0 + NQ - 1
   const int b0 = static_cast<int>(static_cast<int64_t>(jp.nb) * range / ranges);
   const int b1 = static_cast<int>(static_cast<int64_t>(jp.nb) * (range + 1) / ranges);
-  const int64_t col = static_cast<int64_t>(blockIdx.x / groups) * kCols + 4 * threadIdx.x;
-  const bool active = col < ldc;
+  const int64_t local = static_cast<int64_t>(blockIdx.x / groups) * kCols + 4 * threadIdx.x;
+  const int64_t col = col_begin + local;
+  const bool active = local < ldc;
   const uint32_t *src = jp.col_words + (col / kGranule) * kStripeWords + col % kGranule;
   const int64_t stride = static_cast<int64_t>(jp.ng_cols) * kStripeWords;   // words per block
   const uint32_t one = jp.one, hi_one = one << 16;
@@ -106,7 +108,7 @@ few_queries_kernel(const JobParams jp, int groups, int ranges, uint16_t *__restr
   for (int q = 0; q < NQ; ++q)
     if (q0 + q < jp.n_rows)
       *reinterpret_cast<uint2 *>(
-          parts + (static_cast<int64_t>(blockIdx.y) * jp.n_rows + q0 + q) * ldc + col) =
+          parts + (static_cast<int64_t>(blockIdx.y) * jp.n_rows + q0 + q) * ldc + local) =
           make_uint2(cnt[q][0], cnt[q][1]);
 }
 
@@ -114,7 +116,7 @@ few_queries_kernel(const JobParams jp, int groups, int ranges, uint16_t *__restr
 // of 8 references at every eighth k (128-bit loads), then finishes one pair.
 __global__ void __launch_bounds__(kFinishPairs)
 few_queries_finish_kernel(const JobParams jp, int ranges, const uint16_t *__restrict__ parts,
-                          int64_t ldc, const DevStatus *status) {
+                          int64_t col_begin, int64_t ldc, const DevStatus *status) {
   __shared__ __align__(16) uint16_t sums[kNarrowKmers * kFinishPairs];
   if (reinterpret_cast<const volatile DevStatus *>(status)->error != 0) return;
   const int64_t gi = blockIdx.y, col0 = static_cast<int64_t>(blockIdx.x) * kFinishPairs;
@@ -130,7 +132,7 @@ few_queries_finish_kernel(const JobParams jp, int ranges, const uint16_t *__rest
     *reinterpret_cast<uint4 *>(sums + k * kFinishPairs + 8 * g) = c;
   }
   __syncthreads();
-  const int64_t gj = col0 + threadIdx.x;
+  const int64_t gj = col_begin + col0 + threadIdx.x;
   if (gj < jp.n_cols) finish_pair_any<false>(jp, gi, gj, sums + threadIdx.x, kFinishPairs);
 }
 
@@ -148,15 +150,19 @@ Groups query_groups(int64_t n) {
   return by12 * 12 < by16 * 16 ? Groups{12, by12} : Groups{16, by16};
 }
 
-// Block ranges per k: enough CTAs for eight per SM, of at least eight blocks.
-int query_ranges(const JobParams &jp, int sm_count) {
-  const int64_t ctas = (jp.n_cols + kCols - 1) / kCols * query_groups(jp.n_rows).groups * jp.n_kmers;
+// Block ranges per k over n references: enough CTAs for eight per SM, of at
+// least eight blocks.
+int query_ranges(const JobParams &jp, int64_t n, int sm_count) {
+  const int64_t ctas = (n + kCols - 1) / kCols * query_groups(jp.n_rows).groups * jp.n_kmers;
   const int64_t want = (8 * static_cast<int64_t>(sm_count) + ctas - 1) / ctas;
   return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(want, jp.nb / 8)));
 }
 
-int64_t padded_cols(const JobParams &jp) {
-  return (jp.n_cols + kFinishPairs - 1) / kFinishPairs * kFinishPairs;
+int64_t padded_cols(int64_t n) { return (n + kFinishPairs - 1) / kFinishPairs * kFinishPairs; }
+
+// Bytes of the counts of n references in `ranges` block ranges per k.
+size_t parts_bytes(const JobParams &jp, int64_t n, int ranges) {
+  return static_cast<size_t>(ranges) * jp.n_kmers * jp.n_rows * padded_cols(n) * 2;
 }
 
 }  // namespace
@@ -166,32 +172,44 @@ int64_t few_queries_rows(int64_t n) {
   return static_cast<int64_t>(g.nq) * g.groups;
 }
 
-size_t few_queries_bytes(const JobParams &jp, int sm_count) {
-  return static_cast<size_t>(query_ranges(jp, sm_count)) * jp.n_kmers * jp.n_rows * padded_cols(jp) * 2;
+size_t few_queries_bytes(const JobParams &jp, int sm_count, size_t limit) {
+  const size_t all = parts_bytes(jp, jp.n_cols, query_ranges(jp, jp.n_cols, sm_count));
+  return std::min(all, std::max(limit, parts_bytes(jp, std::min<int64_t>(jp.n_cols, kCols), 1)));
 }
 
-cudaError_t launch_few_queries(const JobParams &jp, uint16_t *parts, DevStatus *status,
+cudaError_t launch_few_queries(const JobParams &jp, uint16_t *parts, size_t bytes, DevStatus *status,
                                const volatile int *cancel, int sm_count, cudaStream_t stream) {
-  const int ranges = query_ranges(jp, sm_count);
-  const int64_t ldc = padded_cols(jp);
   const Groups g = query_groups(jp.n_rows);
-  // a range's groups are neighbours, so that they share its references in L2
-  const dim3 grid(static_cast<unsigned int>((jp.n_cols + kCols - 1) / kCols * g.groups),
-                  static_cast<unsigned int>(jp.n_kmers * ranges));
-#define SK_FEW(N)                                                                              \
-  few_queries_kernel<N><<<grid, kThreads, 0, stream>>>(jp, g.groups, ranges, parts, ldc, status, \
-                                                       cancel)
-  switch (g.nq) {
-    case 1: SK_FEW(1); break;
-    case 2: SK_FEW(2); break;
-    case 4: SK_FEW(4); break;
-    case 8: SK_FEW(8); break;
-    case 12: SK_FEW(12); break;
-    default: SK_FEW(16); break;
+  // as many references at a time as their counts fit the workspace, in steps of
+  // what a CTA takes
+  int64_t step = jp.n_cols;
+  int ranges = query_ranges(jp, step, sm_count);
+  auto fits = [&] { return parts_bytes(jp, step, ranges) <= bytes; };
+  while (!fits() && step > kCols) {
+    step = (step / 2 + kCols - 1) / kCols * kCols;
+    ranges = query_ranges(jp, step, sm_count);
   }
+  while (!fits() && ranges > 1) --ranges;
+  for (int64_t c0 = 0; c0 < jp.n_cols; c0 += step) {
+    const int64_t n = std::min(step, jp.n_cols - c0), ldc = padded_cols(n);
+    // a range's groups are neighbours, so that they share its references in L2
+    const dim3 grid(static_cast<unsigned int>((n + kCols - 1) / kCols * g.groups),
+                    static_cast<unsigned int>(jp.n_kmers * ranges));
+#define SK_FEW(N)                                                                            \
+  few_queries_kernel<N><<<grid, kThreads, 0, stream>>>(jp, g.groups, ranges, parts, c0, ldc, \
+                                                       status, cancel)
+    switch (g.nq) {
+      case 1: SK_FEW(1); break;
+      case 2: SK_FEW(2); break;
+      case 4: SK_FEW(4); break;
+      case 8: SK_FEW(8); break;
+      case 12: SK_FEW(12); break;
+      default: SK_FEW(16); break;
+    }
 #undef SK_FEW
-  const dim3 finish(static_cast<unsigned int>(ldc / kFinishPairs), static_cast<unsigned int>(jp.n_rows));
-  few_queries_finish_kernel<<<finish, kFinishPairs, 0, stream>>>(jp, ranges, parts, ldc, status);
+    const dim3 finish(static_cast<unsigned int>(ldc / kFinishPairs), static_cast<unsigned int>(jp.n_rows));
+    few_queries_finish_kernel<<<finish, kFinishPairs, 0, stream>>>(jp, ranges, parts, c0, ldc, status);
+  }
   return cudaGetLastError();
 }
 

@@ -118,6 +118,9 @@ struct Slot {
 // K = 10 and 312 blocks, a little over one wave.
 constexpr size_t kSlotCodeBytes = size_t(2) << 30;
 
+// What a slot's few-queries workspace may take where its tiles need less.
+constexpr size_t kSlotFewBytes = size_t(16) << 20;
+
 // A request waiting longer than this goes ahead of every younger request.
 constexpr double kStarveSeconds = 2.0;
 
@@ -216,11 +219,15 @@ sk_status reserve_slice_scratch(sk_server *sv, Slot &s, int64_t *bytes) {
     cta = std::max(cta, static_cast<size_t>(grid) * count_slot_bytes(*c, job_slots(jp)));
     split = std::max(split, static_cast<size_t>(slots) * count_slot_bytes(*c, 1));
   }
+  // the few-queries kernel works in the memory that cut tiles need anyway
+  ctx->few_limit = std::min(kFewQueriesBytes, std::max(split, kSlotFewBytes));
+  size_t few_bytes = 0;
   for (int64_t nq = 1; nq <= std::min<int64_t>(sq, kFewQueries); ++nq) {
     JobParams few = jp;
     few.n_rows = nq;
-    if (few_queries(ctx, few)) split = std::max(split, few_queries_bytes(few, ctx->sm_count));
+    if (few_queries(ctx, few)) few_bytes = std::max(few_bytes, few_queries_bytes(few, ctx->sm_count, ctx->few_limit));
   }
+  split = std::max(split, few_bytes);
   void *p = nullptr;
   st = scratch(ctx, kSlotLaunchMeta, meta, &p);
   if (st == SK_OK) st = scratch(ctx, kSlotCounts, cta, &p);

@@ -50,12 +50,14 @@ cudaError_t launch_code_values(const uint32_t *packed, int32_t kb, int32_t ng, i
                                int32_t n_g, uint32_t *values, int sm_count, cudaStream_t stream);
 cudaError_t launch_codes(const CodeTask &t, int sm_count, cudaStream_t stream);
 
-// query_kernel.cu: a narrow query job of at most kFewQueries rows; `parts` holds
-// few_queries_bytes(jp).
+// query_kernel.cu: a narrow query job of at most kFewQueries rows.  `parts` is a
+// workspace of `bytes`: few_queries_bytes() holds every reference's counts, or as
+// many as fit `limit` (one CTA's at least), which are then taken part by part.
 constexpr int kFewQueries = 128;
+constexpr size_t kFewQueriesBytes = size_t(128) << 20;   // the limit of a context
 int64_t few_queries_rows(int64_t n);   // rows computed for n queries, padding included
-size_t few_queries_bytes(const JobParams &jp, int sm_count);
-cudaError_t launch_few_queries(const JobParams &jp, uint16_t *parts, DevStatus *status,
+size_t few_queries_bytes(const JobParams &jp, int sm_count, size_t limit);
+cudaError_t launch_few_queries(const JobParams &jp, uint16_t *parts, size_t bytes, DevStatus *status,
                                const volatile int *cancel, int sm_count, cudaStream_t stream);
 
 // aux_kernels.cu

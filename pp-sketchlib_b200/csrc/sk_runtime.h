@@ -59,6 +59,7 @@ struct sk_ctx {
   std::vector<cudaEvent_t> ev_out;      // chunk c's output rows written
   cudaEvent_t ev_join = nullptr;        // second compute stream done
   int64_t code_limit = 0;               // bytes of coded tiles (0: automatic, -1: none)
+  size_t few_limit = sk::kFewQueriesBytes;   // bytes of the few-queries workspace
   int64_t mem_limit = 0;                // bytes a dense call may stage output in (0 = free memory)
   int sm_count = 0;
   std::string err;
