@@ -114,8 +114,8 @@ struct Slot {
   bool high = false;                 // the running slice is on hi_stream
 };
 
-// Coded tiles a slot keeps at most: about 160 column tiles of 100 queries at
-// K = 10 and 312 blocks, a little over one wave.
+// Coded tiles a slot keeps at most: about 160 column tiles of a block of 128
+// queries at K = 10 and 312 blocks, a little over one wave.
 constexpr size_t kSlotCodeBytes = size_t(2) << 30;
 
 // What a slot's few-queries workspace may take where its tiles need less.
@@ -184,6 +184,20 @@ int64_t slot_buffer_bytes(const sk_db *ref, const sk_server_params &p, size_t wo
   return b;
 }
 
+// Meta bytes that hold the plan of any coded slice of at most jp's rows, with
+// `codes` bytes of codes.  A smaller slice is a prefix of the largest one's row
+// blocks, so it has no more launches, ranges or tiles; the cut tail of a launch
+// can be larger where it has fewer tiles, up to tail_bounds.
+size_t coded_meta_bytes(sk_ctx *ctx, const JobParams &jp, const TileConfig &cfg, size_t codes) {
+  Plan plan;
+  if (make_plan(ctx, {jp}, cfg, codes, plan) != SK_OK) return 0;
+  int64_t slots = 0, parts = 0;
+  tail_bounds(jp, plan.grid, &slots, &parts);
+  const size_t launches = plan.subs.size();
+  return meta_layout(plan.jobs.size(), static_cast<size_t>(jp.n_tiles + parts * launches),
+                     static_cast<size_t>(plan.grid) * launches, plan.chunks.size(), launches).bytes;
+}
+
 // Reserves, at start-up, the kernel scratch of the largest slice under every
 // tile shape a slice can take (the default shape and the 64-row one of small
 // batches).  Growing a scratch buffer mid-request would free the old one, and
@@ -228,26 +242,30 @@ sk_status reserve_slice_scratch(sk_server *sv, Slot &s, int64_t *bytes) {
     if (few_queries(ctx, few)) few_bytes = std::max(few_bytes, few_queries_bytes(few, ctx->sm_count, ctx->few_limit));
   }
   split = std::max(split, few_bytes);
-  void *p = nullptr;
-  st = scratch(ctx, kSlotLaunchMeta, meta, &p);
-  if (st == SK_OK) st = scratch(ctx, kSlotCounts, cta, &p);
-  if (st == SK_OK) st = scratch(ctx, kSlotSplitCounts, split, &p);
-  *bytes += static_cast<int64_t>(meta + cta + split);
-  if (st != SK_OK) return st;
   // coded tiles of the largest slice (in several launches above kSlotCodeBytes),
   // where the server's budget has room for them in every slot; a slot without
   // the buffer compares the 14 planes
   size_t values = 0, codes = 0;
   code_wants({jp}, *cfg, &values, &codes);
   codes = std::min(codes, kSlotCodeBytes);
-  const int64_t budget = sv->params.device_bytes;
   ctx->code_limit = -1;
-  if (codes > 0 && (budget == 0 || (*bytes + static_cast<int64_t>(values + codes)) *
-                                           sv->params.slots <= budget)) {
-    ctx->code_limit = static_cast<int64_t>(values + codes);
-    if (code_reserve(ctx, values, codes) == codes) *bytes += static_cast<int64_t>(values + codes);
-    else ctx->code_limit = -1;
+  if (codes > 0) {
+    const size_t coded_meta = coded_meta_bytes(ctx, jp, *cfg, codes);
+    const int64_t all = *bytes + static_cast<int64_t>(std::max(meta, coded_meta) + cta + split + values + codes);
+    const int64_t budget = sv->params.device_bytes;
+    if (budget == 0 || all * sv->params.slots <= budget) {
+      meta = std::max(meta, coded_meta);
+      ctx->code_limit = static_cast<int64_t>(values + codes);
+    }
   }
+  void *p = nullptr;
+  st = scratch(ctx, kSlotLaunchMeta, meta, &p);
+  if (st == SK_OK) st = scratch(ctx, kSlotCounts, cta, &p);
+  if (st == SK_OK) st = scratch(ctx, kSlotSplitCounts, split, &p);
+  *bytes += static_cast<int64_t>(meta + cta + split);
+  if (st != SK_OK || ctx->code_limit < 0) return st;
+  if (code_reserve(ctx, values, codes) == codes) *bytes += ctx->code_limit;
+  else ctx->code_limit = -1;
   return SK_OK;
 }
 
