@@ -133,6 +133,7 @@ struct sk_server {
   sk_server_params params{};
   size_t words_per_sample = 0;
   int64_t slot_bytes = 0;            // device bytes one slot holds
+  size_t code_share = 0;             // what one slot's coded tiles may take without a budget
   std::vector<Slot> slots;
   std::mutex mu;
   std::condition_variable cv;        // wakes the scheduler
@@ -243,8 +244,9 @@ sk_status reserve_slice_scratch(sk_server *sv, Slot &s, int64_t *bytes) {
   }
   split = std::max(split, few_bytes);
   // coded tiles of the largest slice (in several launches above kSlotCodeBytes),
-  // where the server's budget has room for them in every slot; a slot without
-  // the buffer compares the 14 planes
+  // where the server's budget has room for them in every slot, or without one
+  // the slots' share of a quarter of the device; a slot without the buffer
+  // compares the 14 planes
   size_t values = 0, codes = 0;
   code_wants({jp}, *cfg, &values, &codes);
   codes = std::min(codes, kSlotCodeBytes);
@@ -253,7 +255,7 @@ sk_status reserve_slice_scratch(sk_server *sv, Slot &s, int64_t *bytes) {
     const size_t coded_meta = coded_meta_bytes(ctx, jp, *cfg, codes);
     const int64_t all = *bytes + static_cast<int64_t>(std::max(meta, coded_meta) + cta + split + values + codes);
     const int64_t budget = sv->params.device_bytes;
-    if (budget == 0 || all * sv->params.slots <= budget) {
+    if (budget > 0 ? all * sv->params.slots <= budget : values + codes <= sv->code_share) {
       meta = std::max(meta, coded_meta);
       ctx->code_limit = static_cast<int64_t>(values + codes);
     }
@@ -613,6 +615,8 @@ sk_status sk_server_create(sk_ctx *ctx, const sk_db *ref, const sk_random *rando
   sv->params = p;
   if (sv->params.large_slice_queries == 0) sv->params.large_slice_queries = p.slice_queries;
   sv->words_per_sample = static_cast<size_t>(ref->K) * ref->s64 * kBbits;
+  size_t free_b = 0, total_b = 0;
+  if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) sv->code_share = free_b / 4 / p.slots;
   // Slots are made one at a time; under a budget, the first slot's measured
   // bytes decide how many fit.
   sk_status st = SK_OK;

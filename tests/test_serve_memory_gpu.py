@@ -1,4 +1,5 @@
-"""The device memory of server slots with coded tiles is all taken at the start."""
+"""The device memory of server slots with coded tiles: bounded without a budget,
+and all of it taken at the start."""
 import numpy as np
 import pytest
 
@@ -23,6 +24,16 @@ def references():
     yield ctx, ref, qwords
     ref.close()
     ctx.close()
+
+
+def test_slots_without_a_budget_leave_the_device_its_memory(references):
+    import torch
+    ctx, ref, _ = references
+    free = torch.cuda.mem_get_info()[0]
+    server = capi.Server(ctx, ref, slots=16, slice_queries=256, kNN=3)
+    used = free - torch.cuda.mem_get_info()[0]
+    server.close()
+    assert used < free // 4 + 16 * (600 << 20)
 
 
 @pytest.mark.parametrize("sizes", [(1024,), (129, 200, 1, 700, 1024)])
