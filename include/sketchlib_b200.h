@@ -359,8 +359,11 @@ sk_status sk_batch_info(const sk_batch *batch, int32_t *tile_config, int32_t *gr
 sk_status sk_batch_destroy(sk_batch *batch);
 
 /* Autotuner: times every tile shape on one job (out_mode core/accessory into
- * scratch), records the fastest for the job's (n_kmers, sketchsize64) class in
- * the context's tuning table and returns it. */
+ * scratch, whole bit planes), records the fastest for the job's (n_kmers,
+ * sketchsize64) class in the context's tuning table and returns it.  Queries few
+ * enough for a kernel of their own, and jobs large enough to be compared by
+ * dictionary codes, do not take the tuned shape; sk_ctx_set_tile_config forces
+ * one on every job. */
 sk_status sk_autotune(sk_ctx *ctx, const sk_db *ref, const sk_db *query,
                       const sk_random *random, int32_t repeats, int32_t *best_config);
 /* Writes the context's tuning table ("n_kmers sketchsize64 config_id" lines)

@@ -38,14 +38,24 @@ void free_buffers(LaunchBuffers &b) {
 }
 
 // The tile shape a batch uses: the context's forced shape, else the tuned
-// shape of the class holding the most pair-block work, else the default.
+// shape of the class holding the most pair-block work that is not coded where
+// that is most of the work, else the default, which has the coded instance.
 const TileConfig *batch_config(sk_ctx *ctx, const std::vector<JobParams> &jobs,
                                const std::vector<int> &s64) {
   if (ctx->tile_cfg > 0) return tile_config(ctx->tile_cfg);
   std::map<std::pair<int, int>, double> work;
-  for (size_t j = 0; j < jobs.size(); ++j)
-    work[{jobs[j].n_kmers, s64[j]}] +=
-        static_cast<double>(jobs[j].n_rows) * jobs[j].n_cols * jobs[j].n_kmers * jobs[j].nb;
+  double coded = 0, plain = 0;
+  for (size_t j = 0; j < jobs.size(); ++j) {
+    const JobParams &jp = jobs[j];
+    const double w = static_cast<double>(jp.n_rows) * jp.n_cols * jp.n_kmers * jp.nb;
+    if (use_codes(jp.n_rows, jp.n_cols, jp.n_kmers, jp.nb, jp.self != 0)) {
+      coded += w;
+    } else {
+      plain += w;
+      work[{jp.n_kmers, s64[j]}] += w;
+    }
+  }
+  if (coded > plain) return tile_config(kCodedConfig);
   std::pair<int, int> top{0, 0};
   double best = -1;
   for (auto &w : work)
@@ -89,16 +99,6 @@ size_t batch_code_budget(const std::vector<JobParams> &jobs, const TileConfig &c
   if (codes == 0 || cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || free_b / 4 <= values)
     return 0;
   return std::min({codes, size_t(8) << 30, free_b / 4 - values});
-}
-
-// The jobs' plan under one tile shape, in the context's scratch.
-sk_status plan_to_time(sk_ctx *ctx, const std::vector<JobParams> &jobs, const TileConfig &cfg,
-                       Plan &plan, LaunchBuffers &buf) {
-  return plan_with_codes(ctx, jobs, cfg, [&](size_t code_budget) {
-    plan = Plan{};
-    const sk_status st = make_plan(ctx, jobs, cfg, code_budget, plan);
-    return st == SK_OK ? upload_plan(ctx, plan, buf, false) : st;
-  });
 }
 
 // Times `repeats` launches of the plan (after one warm-up), in milliseconds.
@@ -154,7 +154,11 @@ sk_status sk_batch_create(sk_ctx *ctx, const sk_job *jobs, int32_t n_jobs, int32
       if (resident_grid(ctx, *c) < 1) continue;
       Plan plan;
       LaunchBuffers buf;
-      st = plan_to_time(ctx, jp, *c, plan, buf);
+      st = plan_with_codes(ctx, jp, *c, [&](size_t code_budget) {
+        plan = Plan{};
+        const sk_status made = make_plan(ctx, jp, *c, code_budget, plan);
+        return made == SK_OK ? upload_plan(ctx, plan, buf, false) : made;
+      });
       if (st != SK_OK) return st;
       float ms = 0.0f;
       st = time_plan(ctx, plan, buf, 2, &ms);
@@ -285,10 +289,11 @@ sk_status sk_autotune(sk_ctx *ctx, const sk_db *ref, const sk_db *query, const s
     int64_t p = 0;
     st = build_jobs(ctx, &job, 1, *c, jp, &p);
     if (st != SK_OK) return st;
-    if (resident_grid(ctx, *c) < 1) continue;
+    // on the plain planes: a coded job keeps to its own shape whatever is tuned
     Plan plan;
+    if (make_plan(ctx, jp, *c, 0, plan) != SK_OK) continue;
     LaunchBuffers buf;
-    st = plan_to_time(ctx, jp, *c, plan, buf);
+    st = upload_plan(ctx, plan, buf, false);
     if (st != SK_OK) return st;
     float ms = 0.0f;
     st = time_plan(ctx, plan, buf, std::max(1, repeats), &ms);

@@ -310,14 +310,17 @@ sk_status build_job(sk_ctx *ctx, const sk_db *ref, const sk_db *query, const sk_
   if (random && random->kmers != ref->kmers)
     return fail(ctx, SK_EMISMATCH, "Random match table k-mer lengths differ from the sketches");
   const TileConfig *cfg = choose_config(ctx, ref->K, ref->s64);
+  // Jobs large enough to be coded take the shape that has a coded instance: a
+  // tuned shape speaks of the plain planes (sk_autotune times those).
+  const bool codes = ctx->tile_cfg == 0 &&
+                     use_codes(query ? query->n : ref->n, ref->n, ref->K, 2 * ref->s64, !query);
+  if (codes) cfg = tile_config(kCodedConfig);
   // The 64 x 64 shape where 128 x 128 tiles would spend more on padding (rows
   // and columns past the samples, the lower half of diagonal tiles) than the
   // 5% it is slower by per pair, unless a shape was forced or tuned for this
   // (K, sketchsize64): 64 samples fill a quarter of a 128 x 128 tile, 150
-  // queries 150 of 256 rows.  Jobs large enough to be coded stay on the shape
-  // that has a coded instance.
-  if (cfg && cfg->id == 1 && ctx->tile_cfg == 0 &&
-      !use_codes(query ? query->n : ref->n, ref->n, ref->K, 2 * ref->s64, !query) &&
+  // queries 150 of 256 rows.
+  if (cfg && cfg->id == 1 && ctx->tile_cfg == 0 && !codes &&
       ctx->tuning.find({ref->K, ref->s64}) == ctx->tuning.end()) {
     const TileConfig *small = tile_config(kSmallTileConfig);
     if (small && small->max_kmers >= ref->K &&
@@ -928,8 +931,9 @@ sk_status plan_with_codes(sk_ctx *ctx, const std::vector<JobParams> &jobs, const
   return st;
 }
 
-// Whether a query job goes to the few-queries kernel: no tile shape forced or
-// tuned, narrow, and few rows.  Both kernels run at the same LOP3 rate, so the
+// Whether a query job goes to the few-queries kernel: no tile shape forced (a
+// tuned one is the best of the shapes, not better than this kernel), narrow, and
+// few rows.  Both kernels run at the same LOP3 rate, so the
 // line is the padding: groups of 1 .. 16 rows there, tiles of 64 or 128 rows
 // here.  Against 30,011 references (K = 10, 156 words), tiles and groups: 1
 // query 5.9 and 0.8 ms, 32 queries 6.0 and 2.8, 64 queries 6.0 and 5.5, 70
@@ -937,9 +941,7 @@ sk_status plan_with_codes(sk_ctx *ctx, const std::vector<JobParams> &jobs, const
 // Against few references a tile's parts fill the device better: 300 references,
 // 32 queries 130 and 100 us, 48 queries 114 and 120, 100 queries 189 and 242.
 bool few_queries(const sk_ctx *ctx, const JobParams &jp) {
-  if (jp.self || jp.n_rows > kFewQueries || needs_wide(jp) || ctx->tile_cfg != 0 ||
-      ctx->tuning.find({jp.n_kmers, jp.nb / 2}) != ctx->tuning.end())
-    return false;
+  if (jp.self || jp.n_rows > kFewQueries || needs_wide(jp) || ctx->tile_cfg != 0) return false;
   if (jp.n_rows <= 32) return true;
   return jp.n_cols >= 1000 &&
          1.05 * static_cast<double>(few_queries_rows(jp.n_rows)) <= (jp.n_rows <= 64 ? 64 : 128);

@@ -220,7 +220,7 @@ sk_status reserve_slice_scratch(sk_server *sv, Slot &s, int64_t *bytes) {
   if (st == SK_OK) st = attach_count_tables(ctx, &jp);
   if (st != SK_OK) return st;
   size_t meta = 0, cta = 16, split = 16;
-  for (const TileConfig *c : {choose_config(ctx, ref->K, ref->s64), tile_config(kSmallTileConfig)}) {
+  for (const TileConfig *c : {choose_config(ctx, ref->K, ref->s64), tile_config(kSmallTileConfig), cfg}) {
     if (!c || c->max_kmers < ref->K) continue;
     const int grid = resident_grid(ctx, *c);
     if (grid < 1) continue;
