@@ -296,6 +296,46 @@ sk_status check_compatible(sk_ctx *ctx, const sk_db *a, const sk_db *b) {
   return SK_OK;
 }
 
+// Whether a job on a reference database (n_query 0: all-vs-all) is to be coded.
+static bool job_codes(const sk_ctx *ctx, const sk_db *ref, int64_t n_query) {
+  return ctx->tile_cfg == 0 && ctx->code_limit >= 0 &&
+         use_codes(n_query ? n_query : ref->n, ref->n, ref->K, 2 * ref->s64, n_query == 0);
+}
+
+// The tile shape of such a job.
+static const TileConfig *job_shape(sk_ctx *ctx, const sk_db *ref, int64_t n_query) {
+  // Jobs large enough to be coded take the shape that has a coded instance: a
+  // tuned shape speaks of the plain planes (sk_autotune times those).
+  if (job_codes(ctx, ref, n_query)) return tile_config(kCodedConfig);
+  const TileConfig *cfg = choose_config(ctx, ref->K, ref->s64);
+  // The 64 x 64 shape where 128 x 128 tiles would spend more on padding (rows
+  // and columns past the samples, the lower half of diagonal tiles) than the
+  // 5% it is slower by per pair, unless a shape was forced or tuned for this
+  // (K, sketchsize64): 64 samples fill a quarter of a 128 x 128 tile, 150
+  // queries 150 of 256 rows.
+  if (cfg && cfg->id == 1 && ctx->tile_cfg == 0 &&
+      ctx->tuning.find({ref->K, ref->s64}) == ctx->tuning.end()) {
+    const TileConfig *small = tile_config(kSmallTileConfig);
+    if (small && small->max_kmers >= ref->K &&
+        1.05 * padded_pairs(*small, ref->n, n_query) < padded_pairs(*cfg, ref->n, n_query))
+      cfg = small;
+  }
+  return cfg;
+}
+
+// Query rows computed for n_query queries against `ref`, padding included.
+int64_t query_rows(sk_ctx *ctx, const sk_db *ref, int64_t n_query) {
+  JobParams jp{};
+  jp.n_rows = n_query;
+  jp.n_cols = ref->n;
+  jp.n_kmers = ref->K;
+  jp.nb = 2 * ref->s64;
+  jp.nchunk = (jp.nb + kMaxChunkBlocks - 1) / kMaxChunkBlocks;
+  if (few_queries(ctx, jp)) return few_queries_rows(n_query);
+  const int64_t t = job_shape(ctx, ref, n_query)->tile_rows;
+  return (n_query + t - 1) / t * t;
+}
+
 // Fills a JobParams for ref (columns) vs query (rows; NULL = all-vs-all).
 sk_status build_job(sk_ctx *ctx, const sk_db *ref, const sk_db *query, const sk_random *random,
                     int out_mode, int out_col, void *d_out, const TileConfig **cfg_out,
@@ -309,25 +349,7 @@ sk_status build_job(sk_ctx *ctx, const sk_db *ref, const sk_db *query, const sk_
   }
   if (random && random->kmers != ref->kmers)
     return fail(ctx, SK_EMISMATCH, "Random match table k-mer lengths differ from the sketches");
-  const TileConfig *cfg = choose_config(ctx, ref->K, ref->s64);
-  // Jobs large enough to be coded take the shape that has a coded instance: a
-  // tuned shape speaks of the plain planes (sk_autotune times those).
-  const bool codes = ctx->tile_cfg == 0 &&
-                     use_codes(query ? query->n : ref->n, ref->n, ref->K, 2 * ref->s64, !query);
-  if (codes) cfg = tile_config(kCodedConfig);
-  // The 64 x 64 shape where 128 x 128 tiles would spend more on padding (rows
-  // and columns past the samples, the lower half of diagonal tiles) than the
-  // 5% it is slower by per pair, unless a shape was forced or tuned for this
-  // (K, sketchsize64): 64 samples fill a quarter of a 128 x 128 tile, 150
-  // queries 150 of 256 rows.
-  if (cfg && cfg->id == 1 && ctx->tile_cfg == 0 && !codes &&
-      ctx->tuning.find({ref->K, ref->s64}) == ctx->tuning.end()) {
-    const TileConfig *small = tile_config(kSmallTileConfig);
-    if (small && small->max_kmers >= ref->K &&
-        1.05 * padded_pairs(*small, ref->n, query ? query->n : 0) <
-            padded_pairs(*cfg, ref->n, query ? query->n : 0))
-      cfg = small;
-  }
+  const TileConfig *cfg = job_shape(ctx, ref, query ? query->n : 0);
   if (!cfg || cfg->max_kmers < ref->K)
     return fail(ctx, SK_ENOTSUP, "No tile configuration holds %d k-mer lengths (at most %d)",
                 ref->K, cfg ? cfg->max_kmers : kMaxKmers);

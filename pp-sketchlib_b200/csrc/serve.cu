@@ -36,8 +36,8 @@
 //     (at least one), so a small request finds a slot free and waits at most
 //     for the slice already running, and the device still always has a large
 //     slice queued behind the running one;
-//   * rows left free in a slice's last query tile are filled with queries of
-//     larger requests: the kernel computes whole tiles anyway.
+//   * rows left free in a slice's last query tile (or group of few queries) are
+//     filled with queries of larger requests: the kernel computes them anyway.
 //
 // Per slice: the query words uploaded straight from a request's page-locked
 // buffer, or staged through the slot's pinned buffer when the caller's is
@@ -410,13 +410,6 @@ int64_t take(Slot &s, const std::shared_ptr<Request> &r, int64_t room) {
   return nq;
 }
 
-// Rows of the query tiles a slice of nq queries occupies: 64-row tiles where
-// 128-row ones would be mostly padding (build_job's choice).
-int64_t tile_rows_for(int64_t nq) {
-  const int64_t r64 = (nq + 63) / 64 * 64, r128 = (nq + 127) / 128 * 128;
-  return 1.05 * static_cast<double>(r64) < static_cast<double>(r128) ? r64 : r128;
-}
-
 // Fills a free slot with the next slice, or leaves it empty when nothing may
 // start now.  `order` is the pending requests in admission order.
 void compose_slice(sk_server *sv, Slot &s, const std::vector<std::shared_ptr<Request>> &order,
@@ -449,8 +442,9 @@ void compose_slice(sk_server *sv, Slot &s, const std::vector<std::shared_ptr<Req
       if (open(*r) && !small(*r)) take(s, r, cap - s.nq);
     }
   }
-  // free rows of the last query tile: queries of large requests ride along
-  const int64_t fill = std::min(tile_rows_for(s.nq), sq);
+  // rows computed anyway (of the last query tile or group): queries of large
+  // requests ride along
+  const int64_t fill = std::min(query_rows(s.ctx, sv->ref, s.nq), sq);
   for (const auto &r : order) {
     if (s.nq >= fill) break;
     if (open(*r) && !small(*r)) take(s, r, fill - s.nq);

@@ -224,6 +224,7 @@ sk_status build_job(sk_ctx *ctx, const sk_db *ref, const sk_db *query, const sk_
                     int out_mode, int out_col, void *d_out, const TileConfig **cfg_out,
                     JobParams *jp);
 bool few_queries(const sk_ctx *ctx, const JobParams &jp);
+int64_t query_rows(sk_ctx *ctx, const sk_db *ref, int64_t n_query);
 sk_status launch_job(sk_ctx *ctx, const JobParams &jp, const TileConfig &cfg);
 // Points a job without random-match correction at the context's Jaccard /
 // log-Jaccard tables by count for its union size, built on first use (one
