@@ -294,7 +294,9 @@ __global__ void __launch_bounds__(kColThreads, 1) code_columns_kernel(const Code
                  kCodeListWords * 2, &list_bar[b]);
     };
     // a list that never lands, or a set never given back, is recorded, once;
-    // what is there instead is still in range
+    // what is there instead is still in range.  No list is fetched after that,
+    // and those in flight land (or their wait runs out again) before the CTA's
+    // shared memory goes away.
     bool waits = true;
     auto wait = [&](uint64_t *bar, uint32_t parity) {
       if (waits && !mbar_wait_bounded(bar, parity, kListWaitNs)) {
@@ -334,9 +336,9 @@ __global__ void __launch_bounds__(kColThreads, 1) code_columns_kernel(const Code
       const int4 next = t.chunks[more ? next_ci : ci];
       // every table warp is done with the other buffer
       asm volatile("bar.sync 1, %0;" ::"n"(kTableWarps * 32) : "memory");
-      if (more && role == 0 && lane == 0) fetch(next, next_kb, b ^ 1);
+      if (more && waits && role == 0 && lane == 0) fetch(next, next_kb, b ^ 1);
       wait(&list_bar[b], list_phase[b]);
-      list_phase[b] ^= 1u;
+      if (waits) list_phase[b] ^= 1u;
 #pragma unroll 1
       for (int pass = 0; pass < 16; ++pass) {
         const uint2 vals = entries(chunk, b, pass);
@@ -354,7 +356,11 @@ __global__ void __launch_bounds__(kColThreads, 1) code_columns_kernel(const Code
           phase ^= 1u;
         }
       }
-      if (!more) return;
+      if (!more) {
+        if (!waits && role == 0 && lane == 0)
+          for (int i = 0; i < 2; ++i) mbar_wait_bounded(&list_bar[i], list_phase[i], kListWaitNs);
+        return;
+      }
       kb = next_kb;
       ci = next_ci;
       chunk = next;
