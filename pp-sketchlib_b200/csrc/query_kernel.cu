@@ -33,8 +33,8 @@ constexpr int kFinishPairs = 128;
 
 template <int NQ>
 __global__ void __launch_bounds__(kThreads)
-few_queries_kernel(const JobParams jp, int groups, int ranges, uint16_t *__restrict__ parts,
-                   int64_t col_begin, int64_t ldc, DevStatus *status, const volatile int *cancel) {
+few_queries_kernel(const JobParams jp, int groups, int ranges, uint16_t *__restrict__ parts, int64_t ldc,
+                   DevStatus *status, const volatile int *cancel) {
   __shared__ __align__(16) uint32_t qw[kTileBlocks * kBbits * NQ];
   __shared__ int s_stop;
   if (threadIdx.x == 0) s_stop = poll_cancelled(status, cancel) ? 1 : 0;
@@ -44,9 +44,8 @@ few_queries_kernel(const JobParams jp, int groups, int ranges, uint16_t *__restr
   const int q0 = (blockIdx.x % groups) * NQ;   // this CTA's queries: q0 .. q0 + NQ - 1
   const int b0 = static_cast<int>(static_cast<int64_t>(jp.nb) * range / ranges);
   const int b1 = static_cast<int>(static_cast<int64_t>(jp.nb) * (range + 1) / ranges);
-  const int64_t local = static_cast<int64_t>(blockIdx.x / groups) * kCols + 4 * threadIdx.x;
-  const int64_t col = col_begin + local;
-  const bool active = local < ldc;
+  const int64_t col = static_cast<int64_t>(blockIdx.x / groups) * kCols + 4 * threadIdx.x;
+  const bool active = col < ldc;
   const uint32_t *src = jp.col_words + (col / kGranule) * kStripeWords + col % kGranule;
   const int64_t stride = static_cast<int64_t>(jp.ng_cols) * kStripeWords;   // words per block
   const uint32_t one = jp.one, hi_one = one << 16;
@@ -108,7 +107,7 @@ few_queries_kernel(const JobParams jp, int groups, int ranges, uint16_t *__restr
   for (int q = 0; q < NQ; ++q)
     if (q0 + q < jp.n_rows)
       *reinterpret_cast<uint2 *>(
-          parts + (static_cast<int64_t>(blockIdx.y) * jp.n_rows + q0 + q) * ldc + local) =
+          parts + (static_cast<int64_t>(blockIdx.y) * jp.n_rows + q0 + q) * ldc + col) =
           make_uint2(cnt[q][0], cnt[q][1]);
 }
 
@@ -192,12 +191,14 @@ cudaError_t launch_few_queries(const JobParams &jp, uint16_t *parts, size_t byte
   while (!fits() && ranges > 1) --ranges;
   for (int64_t c0 = 0; c0 < jp.n_cols; c0 += step) {
     const int64_t n = std::min(step, jp.n_cols - c0), ldc = padded_cols(n);
+    JobParams part = jp;   // whose columns begin at c0, a whole number of granules
+    part.col_words += c0 / kGranule * kStripeWords;
     // a range's groups are neighbours, so that they share its references in L2
     const dim3 grid(static_cast<unsigned int>((n + kCols - 1) / kCols * g.groups),
                     static_cast<unsigned int>(jp.n_kmers * ranges));
-#define SK_FEW(N)                                                                            \
-  few_queries_kernel<N><<<grid, kThreads, 0, stream>>>(jp, g.groups, ranges, parts, c0, ldc, \
-                                                       status, cancel)
+#define SK_FEW(N)                                                                                \
+  few_queries_kernel<N><<<grid, kThreads, 0, stream>>>(part, g.groups, ranges, parts, ldc, status, \
+                                                       cancel)
     switch (g.nq) {
       case 1: SK_FEW(1); break;
       case 2: SK_FEW(2); break;
