@@ -693,12 +693,15 @@ size_t Plan::code_bytes() const {
 // Whether a job's tiles are worth encoding first (128 x 128 tiles of narrow
 // jobs).  The encoder costs about as much per row block and column as the
 // planes it saves in one tile, so it pays where a row block meets many columns
-// and, since it serves two row blocks per lookup, where there are two: an
-// all-vs-all at K = 8, 156 words on a random tree took 2.85 ms plain and 2.88
-// coded at 1,500 samples, 4.99 and 4.64 at 2,000, 11.5 and 9.5 at 3,000 (in
-// clades 2.86 and 2.72, 4.99 and 4.33, 11.0 and 9.1); 100 queries against
-// 20,000 samples 5.70 and 6.07, 300 queries 15.1 and 13.8, 300 against 2,000
-// 1.60 and 1.53.  Narrower sketches and fewer k cross at the same sizes.
+// and, since it serves two row blocks per lookup, where there are two.  Plain and
+// coded at K = 8, 156 words, in ms, on a random tree (7 planes), in clades (6) and
+// for unrelated samples (8): all-vs-all of 1,700 samples 3.75 and 3.31, 3.75 and
+// 3.20, 3.71 and 3.57; of 3,000 11.5 and 8.55, 11.4 and 8.41, 10.6 and 9.20; 300
+// queries against 20,011 15.2 and 12.8, 15.1 and 12.4, 14.5 and 13.3, against
+// 2,000 1.61 and 1.49, 1.61 and 1.43, 1.60 and 1.54.  Nearest the line the two are
+// close: 150 queries against 20,011 unrelated samples 8.85 and 8.95, against 1,000
+// 0.55 and 0.61, where a tree takes 0.56 and 0.60 and 256 queries 0.71 and 0.66.
+// Narrower sketches and fewer k cross at the same sizes.
 bool use_codes(int64_t n_rows, int64_t n_cols, int32_t n_kmers, int32_t nb, bool self) {
   if (n_kmers > kNarrowKmers || nb > kMaxChunkBlocks) return false;
   return self ? n_cols >= 1700 : n_rows > kCodeGroup && n_cols >= 1000;

@@ -42,8 +42,8 @@ constexpr int kTableWarps = 4;             // (bin, row block) of a pass each
 constexpr int kColThreads = kLookupThreads + 32 * kTableWarps;   // and four table warps: 512 x 112 + 128 x 32 registers
 constexpr int kColSamples = 4;             // columns per thread
 constexpr int kPairTableBytes = 2 * kTableBytes + 16;   // 2-byte entries, one spare
-// two sets of two tables, two buffers of two dictionary lists
 constexpr int kTableSets = 3;              // passes the table warps may be ahead
+// the sets of two tables, two buffers of two dictionary lists
 constexpr int kColTableBytes = 2 * kTableSets * kPairTableBytes + 2 * 2 * kCodeListWords * 2;
 constexpr uint64_t kListWaitNs = 2000000000ull;   // 2 s bounded wait
 constexpr int kValueThreads = 256;
@@ -118,7 +118,6 @@ __global__ void __launch_bounds__(kRowThreads, 3)
 code_rows_kernel(const CodeTask t) {
   extern __shared__ unsigned char row_tables[];   // [kPassBins][kTableBytes]
   __shared__ int warp_count[kRowThreads / 32][kPassBins];
-  __shared__ int s_max;
   if (__syncthreads_or(cancelled(t.status))) return;   // all of the CTA or none
   const int row = threadIdx.x, warp = row >> 5, lane = row & 31;
   const int64_t items = static_cast<int64_t>(t.kb) * t.n_rb;
@@ -136,7 +135,6 @@ code_rows_kernel(const CodeTask t) {
     for (int p = 0; p < kBbits; ++p) w[p] = src[p * kGranule];
     w[14] = w[15] = 0;
     transpose_planes(w);
-    if (row == 0) s_max = 0;
     uint16_t *list = t.lists + (static_cast<int64_t>(rb) * t.kb + kb) * kCodeListWords;
     uint32_t code[8];
     int most = 0;
@@ -186,9 +184,9 @@ code_rows_kernel(const CodeTask t) {
       code[q] = c;
       __syncthreads();
     }
-    if (row == 0) s_max = most;   // every thread counted the same totals
     transpose_codes(code);
-    // planes 4 .. 8 are compiled in the distance kernel
+    // every thread counted the same totals; planes 4 .. 8 are compiled in the
+    // distance kernel
     const int planes = max(kCodeMinPlanes, 32 - __clz(most));
     uint32_t *dst = t.words + code_stripe(t.layout, t.kb, t.layout.rb0 + rb, kb, 0) + row;
     // all planes: a pair of blocks reads as many as its larger dictionary has

@@ -552,7 +552,6 @@ constexpr TileConfig make_cfg(int id) {
                     TR,
                     kMaxKmers,
                     STAGES,
-                    TileShape<QT, RT, TQ, TR, STAGES, false>::kThreads,
                     TileShape<QT, RT, TQ, TR, STAGES, false>::kSmemBytes,
                     &launch_cfg<QT, RT, TQ, TR, STAGES, MINB>,
                     &occupancy_cfg<QT, RT, TQ, TR, STAGES, MINB>};

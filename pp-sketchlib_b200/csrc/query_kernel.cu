@@ -4,10 +4,12 @@
 // one query against 30,011 references (K = 10, 156 words) took 6.3 ms, most of
 // it padding; what the call cannot do without is one read of the references,
 // 0.8 ms.  Here a thread owns four references (one 128-bit load per bit plane,
-// straight from the packed stripes, all 14 planes of a block in flight) and
-// compares them with every query; the query words are broadcast from shared
-// memory.  HBM-bound up to about 12 queries (14 LOP3 per query and 32 bins
-// against 56 bytes), LOP3-bound above.
+// straight from the packed stripes) and compares them with every query; the query
+// words are broadcast from shared memory.  From 8 queries up a thread holds the 14
+// planes of a block; for fewer the compiler holds a few at a time (32 registers
+// for one query) and twice the warps keep as many loads in flight.  HBM-bound up
+// to about 12 queries (14 LOP3 per query and 32 bins against 56 bytes), LOP3-bound
+// above.
 //
 // The blocks of each k are cut into ranges so that a small reference set still
 // fills the device; a range's counts go to a uint16 array [k][range][query]

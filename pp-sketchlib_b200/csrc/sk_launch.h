@@ -16,7 +16,6 @@ struct TileConfig {
   int thread_rows, thread_cols;  // per-thread register block
   int max_kmers;                 // largest K the instance handles
   int stages;                    // pipeline depth
-  int threads;
   int smem_bytes;
   cudaError_t (*launch)(const LaunchParams &, int grid, cudaStream_t);
   int (*blocks_per_sm)();        // resident CTAs per SM at this shape's shared memory
