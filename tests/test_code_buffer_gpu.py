@@ -99,3 +99,32 @@ def test_codes_do_not_take_the_memory_of_needed_buffers():
             torch.cuda.empty_cache()
         np.testing.assert_array_equal(out.cpu().numpy(), want)
         db.close()
+
+
+def test_blocked_output_at_the_default_budget():
+    """13,000 samples to the host, 676 MB, with 1.2 GB of the device free: row
+    blocks in half of that."""
+    import torch
+    n, K, s64 = 13_000, 3, 4
+    kmers = [15, 17, 19]
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    words = torch.randint(0, 2**40, (n, K, s64 * 14), dtype=torch.int64, device="cuda", generator=gen)
+    out = torch.empty((n * (n - 1) // 2, 2), dtype=torch.float32, device="cuda")
+    torch.cuda.synchronize()
+    with capi.Context(0) as ctx:
+        db = capi.Database(ctx, words.data_ptr(), kmers, s64, n_samples=n)
+        capi.dists_dense(ctx, db, out=out.data_ptr())
+        ctx.synchronize()
+        db.close()
+    want = out.cpu().numpy()
+    del out
+    with capi.Context(0) as ctx:
+        db = capi.Database(ctx, words.data_ptr(), kmers, s64, n_samples=n)
+        hold = _fill(1200 << 20)
+        try:
+            got = capi.dists_dense(ctx, db)
+        finally:
+            del hold
+            torch.cuda.empty_cache()
+        db.close()
+    np.testing.assert_array_equal(got, want)

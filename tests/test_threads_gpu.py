@@ -59,3 +59,18 @@ def test_sketches_of_different_widths_on_threads():
         return make
 
     assert _at_once([job(s) for s in (64, 100, 156, 300)], 400) == []
+
+
+def test_coded_calls_on_threads():
+    """Jobs of different sizes, each coded in its own context's buffer."""
+    words, kmers = random_sketches(2300, 3, 8, seed=7)
+
+    def job(n, nq):
+        def make(ctx):
+            db = capi.Database(ctx, words[:n], kmers, 8)
+            qry = capi.Database(ctx, words[n:n + nq], kmers, 8) if nq else None
+            call = lambda: [capi.dists_dense(ctx, db, qry)]
+            return call, call()
+        return make
+
+    assert _at_once([job(1700, 0), job(2300, 0), job(1500, 300), job(1100, 140)], 25) == []
