@@ -5,6 +5,7 @@ import numpy as np
 import pytest
 
 from conftest import random_sketches
+from launched import names_during
 from sketchlib_b200 import capi
 from test_low_coverage_gpu import _offsets, _read_set
 
@@ -12,11 +13,8 @@ pytestmark = pytest.mark.gpu
 
 
 def _kernels(call):
-    from torch.profiler import ProfilerActivity, profile
     call()
-    with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA]) as prof:
-        call()
-    return " ".join(e.name for e in prof.events())
+    return " ".join(names_during(call))
 
 
 def _forms(ctx, ref, qry, few, w, kmers, s64):

@@ -4,6 +4,7 @@ import numpy as np
 import pytest
 
 from conftest import random_sketches
+from launched import names_during
 from sketchlib_b200 import capi
 
 pytestmark = pytest.mark.gpu
@@ -11,7 +12,6 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("small,group", [(10, 12), (3, 4), (20, 12)])
 def test_a_small_slice_takes_its_group_of_queries(small, group):
-    from torch.profiler import ProfilerActivity, profile
     n, nq, K, s64 = 4000, 1500, 4, 64
     w, kmers = random_sketches(n + 64, K, s64, seed=19)
     q = np.concatenate([w[n:]] * 24)[:nq]
@@ -20,12 +20,15 @@ def test_a_small_slice_takes_its_group_of_queries(small, group):
         server = capi.Server(ctx, ref, slots=1, slice_queries=128, kNN=2)
         first = server.submit(q)
         server.wait(first)                       # the kernels are loaded
-        with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA]) as prof:
-            large = server.submit(q)
-            ticket = server.submit(q[:small])
-            server.wait(ticket)
-            server.wait(large)
-        names = {e.name for e in prof.events() if "few_queries_kernel" in e.name}
+        tickets = []
+
+        def both():
+            tickets[:] = [server.submit(q), server.submit(q[:small])]
+            for t in tickets:
+                server.wait(t)
+
+        names = {x for x in names_during(both) if "few_queries_kernel" in x}
+        large, ticket = tickets
         got, whole = server.result(ticket)[:2], server.result(large)[:2]
         server.close()
         ref.close()

@@ -3,6 +3,7 @@ and all of it taken at the start."""
 import numpy as np
 import pytest
 
+from launched import names_during
 from sketchlib_b200 import capi
 
 pytestmark = pytest.mark.gpu
@@ -38,19 +39,18 @@ def test_slots_without_a_budget_leave_the_device_its_memory(references):
 
 @pytest.mark.parametrize("sizes", [(1024,), (129, 200, 1, 700, 1024)])
 def test_slices_allocate_nothing(references, sizes):
-    import torch
-    from torch.profiler import ProfilerActivity, profile
     ctx, ref, qwords = references
     server = capi.Server(ctx, ref, slots=1, slice_queries=1024, kNN=3)
     got = []
+
+    def slices():
+        for nq in sizes:
+            t = server.submit(qwords[:nq])
+            server.wait(t)
+            got.append((nq, *server.result(t)[:2]))
+
     try:
-        with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA]) as prof:
-            for nq in sizes:
-                t = server.submit(qwords[:nq])
-                server.wait(t)
-                idx, dist = server.result(t)[:2]
-                got.append((nq, idx, dist))
-        names = [e.name for e in prof.events()]
+        names = names_during(slices, repeats=1)
     finally:
         server.close()
     assert any("dist_items_kernel" in n for n in names)      # the profiler saw the calls

@@ -4,6 +4,7 @@ import numpy as np
 import pytest
 
 from conftest import random_sketches
+from launched import names_during
 from sketchlib_b200 import capi
 
 pytestmark = pytest.mark.gpu
@@ -12,11 +13,8 @@ K, S64 = 3, 4
 
 
 def _kernels(call):
-    from torch.profiler import ProfilerActivity, profile
     call()
-    with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA]) as prof:
-        call()
-    return " ".join(e.name for e in prof.events())
+    return " ".join(names_during(call))
 
 
 @pytest.mark.parametrize("how", ["autotuned", "loaded", "neither"])
